@@ -516,13 +516,17 @@ __device__ __forceinline__ int ld_err(const SweepCtl* ctl) {
   return (int)ld_relaxed(reinterpret_cast<const unsigned int*>(&ctl->err));
 }
 
-// v = *p once it is no longer pending
-template <typename T>
-__device__ __forceinline__ bool take(const T* p, T& v) {
-  using P = Pending<T>;
-  const typename P::U u = ld_relaxed(reinterpret_cast<const typename P::U*>(p));
-  v = P::from(u);
-  return u != P::bits;
+// *p into bits where on
+__device__ __forceinline__ void ld_relaxed_if(bool on, const unsigned long long* p,
+                                              unsigned long long& bits) {
+  asm volatile(
+      "{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.relaxed.gpu.global.b64 %0, [%1]; }"
+      : "+l"(bits) : "l"(p), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void ld_relaxed_if(bool on, const unsigned int* p, unsigned int& bits) {
+  asm volatile(
+      "{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.relaxed.gpu.global.b32 %0, [%1]; }"
+      : "+r"(bits) : "l"(p), "r"((unsigned)on) : "memory");
 }
 
 // x[0 .. n) = pending
@@ -533,18 +537,48 @@ __global__ void k_fill_pending(long long n, T* __restrict__ x) {
     x[e] = Pending<T>::value();
 }
 
-// Warp-level driver of one recurrence.  `step(i, k, first)` advances cell i
-// (this lane's) from slot k as far as its inputs allow and returns the next
-// slot (w when the cell is done and stored).  Slices are taken in the order
-// that makes every dependency point to an earlier (or the same) slice.  A
-// warp whose lanes wait spins for kSweepSpin polls, then sleeps briefly
-// between polls.
+// Warp-level driver of one recurrence: each lane takes one cell of the
+// warp's slice.  A cell's slots are taken C at a time (one chunk for rows of
+// up to C slots), their indices and coefficients (`coef(e)`, read-only data)
+// in registers, so that a poll is one batch of loads of the neighbour values
+// and nothing else.  In an order of many levels (GATE) the dependencies are
+// first packed to the front, while the warp waits anyway, so that the sum
+// runs over them alone (0.93 -> 0.74 us a level); in an order of a few
+// levels, where bandwidth counts, the packing would only delay the
+// coefficients.
+// Once the values are all there they are folded in in slot order (`use`),
+// the sequential loop's arithmetic; `finish` stores the cell.  A lane stores
+// as soon as its own inputs are there, because a slice that spans two levels
+// holds cells that wait for cells of the same slice.
+//
+// What bounds a level-by-level order is the step from one level's store to
+// the next level's load, through L2 (0.24-0.45 us one way between two SMs,
+// within a die and across).  Two things had made that step 1.65 us: a
+// second, serial round trip for slots past the fourth, and the polls of all
+// the resident warps -- dozens of levels ahead of the front, each re-reading
+// every neighbour value -- which kept L2 busy.  So, where the order has
+// levels to wait for (GATE), a warp first waits on ONE value, with one
+// sector per poll: the last dependency of the last cell its slice depends
+// on, an ancestor two steps back (one step back was 4% slower).  Only the
+// slices next to the front then poll their own inputs.
 constexpr int kSweepSpin = 64;
 constexpr int kSweepSleep = 64;  // ns
+constexpr int kGateSleep = 32;   // ns
 
-template <bool UP, typename Step>
-__device__ __forceinline__ void sweep_slices(int n, const uint8_t* __restrict__ slice_w,
-                                             SweepCtl* ctl, Step&& step) {
+template <bool UP>
+__device__ __forceinline__ bool sweep_dep(int j, int i) {
+  return j >= 0 && (UP ? j > i : j < i);
+}
+
+template <bool UP, bool GATE, int C, int V, typename A, typename T, typename Start, typename Coef,
+          typename Use, typename Finish>
+__device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const T* vals, SweepCtl* ctl,
+                                           Start&& start, Coef&& coef, Use&& use,
+                                           Finish&& finish) {
+  using P = Pending<T>;
+  using U = typename P::U;
+  constexpr unsigned full = 0xffffffffu;
+  const U* bits_of = reinterpret_cast<const U*>(vals);
   const int lane = threadIdx.x & 31;
   const int ns = (n + 31) >> 5;
   const int W = gridDim.x * (blockDim.x >> 5);
@@ -552,98 +586,154 @@ __device__ __forceinline__ void sweep_slices(int n, const uint8_t* __restrict__ 
   for (int r = gw; r < ns; r += W) {
     const int s = UP ? ns - 1 - r : r;
     const int i = s * 32 + lane;
-    const int w = __ldg(&slice_w[s]);
-    int k = step(i, i < n ? 0 : w, true);
+    const int w = __ldg(&R.slice_w[s]);
+    const int base = __ldg(&R.slice_ptr[s]) + lane;
+    int dj[C];  // the chunk's dependencies in slot order: the first nd (GATE), or
+    A a[C];     // those of the slots in mask
+    U bits[C][V];
+    int nd = 0, k0 = 0;
+    unsigned mask = 0;
+    bool done = i >= n;
+    auto on = [&](int q) { return GATE ? q < nd : ((mask >> q) & 1u) != 0; };
+    auto load = [&]() {
+      int j[C], du[C];
+#pragma unroll
+      for (int u = 0; u < C; ++u) {
+        j[u] = -1;
+        if (k0 + u < w) j[u] = __ldg(&R.col[base + (k0 + u) * kWarp]);
+      }
+      if constexpr (GATE) {
+        nd = 0;
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          dj[u] = du[u] = 0;
+          const bool dep = sweep_dep<UP>(j[u], i);
+#pragma unroll
+          for (int q = 0; q <= u; ++q)
+            if (dep && nd == q) {
+              dj[q] = j[u];
+              du[q] = u;
+            }
+          nd += dep;
+        }
+      } else {
+        mask = 0;
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          dj[u] = j[u];
+          du[u] = u;
+          if (sweep_dep<UP>(j[u], i)) mask |= 1u << u;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+        if (on(q)) a[q] = coef(base + (k0 + du[q]) * kWarp);
+#pragma unroll
+        for (int v = 0; v < V; ++v) bits[q][v] = 0;
+      }
+    };
+    if (!done) {
+      start(i);
+      load();
+    }
+    if constexpr (GATE) {
+      // the last cell of an earlier slice that this chunk depends on, then
+      // the last dependency of that cell (indices offset so that 0 is none;
+      // backward, counted from the top)
+      unsigned last = 0;
+#pragma unroll
+      for (int q = 0; q < C; ++q)
+        if (q < nd && (UP ? (dj[q] >> 5) > s : (dj[q] >> 5) < s))
+          last = max(last, (unsigned)(UP ? n - dj[q] : dj[q] + 1));
+      last = __reduce_max_sync(full, last);
+      if (last) {
+        const int jl = UP ? n - (int)last : (int)last - 1;
+        const int wl = __ldg(&R.slice_w[jl >> 5]);
+        const int bl = __ldg(&R.slice_ptr[jl >> 5]) + (jl & 31);
+        const int c = lane < wl ? __ldg(&R.col[bl + lane * kWarp]) : -1;
+        unsigned far = sweep_dep<UP>(c, jl) ? (unsigned)(UP ? n - c : c + 1) : 0u;
+        far = __reduce_max_sync(full, far);
+        if (far) {
+          const U* g = &bits_of[(size_t)(UP ? n - (int)far : (int)far - 1) * V];
+          for (int poll = 0; ld_relaxed(g) == P::bits; ++poll) {
+            if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
+              if (lane == 0) atomicExch(&ctl->err, 1);
+              break;
+            }
+            __nanosleep(kGateSleep);
+          }
+          __syncwarp();
+        }
+      }
+    }
     for (int poll = 0;; ++poll) {
-      __syncwarp();
-      if (__all_sync(0xffffffffu, k >= w)) break;
+      if (!done) {
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+#pragma unroll
+          for (int v = 0; v < V; ++v)
+            ld_relaxed_if(on(q), &bits_of[(size_t)dj[q] * V + v], bits[q][v]);
+        bool ready = true;
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+#pragma unroll
+          for (int v = 0; v < V; ++v) ready &= bits[q][v] != P::bits;
+        if (ready) {
+#pragma unroll
+          for (int q = 0; q < C; ++q) {
+            if (GATE && q >= nd) break;
+            if (!GATE && !on(q)) continue;
+            T xv[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) xv[v] = P::from(bits[q][v]);
+            use(a[q], xv);
+          }
+          k0 += C;
+          if (k0 < w) {
+            load();
+          } else {
+            finish(i);
+            done = true;
+          }
+        }
+      }
+      if (__all_sync(full, done)) break;
       if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
         if (lane == 0) atomicExch(&ctl->err, 1);
         break;
       }
       if (poll >= kSweepSpin) __nanosleep(kSweepSleep);
-      if (k < w) k = step(i, k, false);
     }
   }
-}
-
-// One advance of a recurrence row: from slot k, the slots of the dependency
-// side (`dep(j)`) are taken in chunks of C -- their neighbour values and
-// their coefficients (`coef(e)`, read-only data) loaded at once, so that a
-// coefficient never waits behind a value that has just arrived -- then
-// added in slot order up to the first one still pending.  `use(a, xv)`
-// folds a ready value in.  Returns the slot to resume from (w when the row
-// is complete).
-template <int C, int V, typename T, typename Dep, typename Coef, typename Use>
-__device__ __forceinline__ int advance(const Rows<T>& R, int base, int w, int k, const T* vals,
-                                       Dep&& dep, Coef&& coef, Use&& use) {
-  using A = decltype(coef(0));
-  while (k < w) {
-    int j[C];
-    A a[C];
-    T xv[C][V];
-    bool rdy[C];
-#pragma unroll
-    for (int u = 0; u < C; ++u) {
-      const int e = base + (k + u) * kWarp;
-      j[u] = k + u < w ? __ldg(&R.col[e]) : -1;
-      rdy[u] = true;
-      if (j[u] >= 0 && dep(j[u])) {
-        a[u] = coef(e);
-#pragma unroll
-        for (int v = 0; v < V; ++v) rdy[u] &= take(&vals[(size_t)j[u] * V + v], xv[u][v]);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < C; ++u) {
-      if (k >= w) return w;
-      if (j[u] >= 0 && dep(j[u])) {
-        if (!rdy[u]) return k;
-        use(a[u], xv[u]);
-      }
-      ++k;
-    }
-  }
-  return k;
 }
 
 // solv_precond.f90:10-29: d_i = pl_i - sum_{j<i} n^2 c_j (DIC, imat 1) or
 // - (p c_j) n (DILU, imat 2) in face order; c_r = d; c = 1/(d + small).
 // imat <= 0 is Jacobi (no recurrence; k_precond_jacobi), imat >= 3 keeps
-// d = pl (the reference's fall-through).  c must start out pending.
-__global__ void __launch_bounds__(kSweepThreads) k_precond_sf(
-    int n, int imat, Rows<double> R, const int* __restrict__ slot_src,
-    const double* __restrict__ fp, const double* __restrict__ fn, double* c,
-    double* __restrict__ c_r, SweepCtl* ctl) {
-  const int lane = threadIdx.x & 31;
+// d = pl (the reference's fall-through).  c must start out pending.  A lower
+// neighbour's ng%n is the slot's sweep coefficient; DILU also takes ng%p,
+// from its face.
+template <int IMAT, bool GATE>
+__global__ void __launch_bounds__(kSweepThreads, 1) k_precond_sf(
+    int n, Rows<double> R, const int* __restrict__ slot_src,
+    const double* __restrict__ fp, double* c, double* __restrict__ c_r, SweepCtl* ctl) {
   double d = 0.0;
-  int base = 0;
-  sweep_slices<false>(n, R.slice_w, ctl, [&](int i, int k, bool first) -> int {
-    const int w = __ldg(&R.slice_w[i >> 5]);
-    if (first) {
-      if (i >= n) return w;
-      base = __ldg(&R.slice_ptr[i >> 5]) + lane;
-      d = R.diag[i];
-    }
-    if (imat == 1 || imat == 2) {
-      k = advance<4, 1>(
-          R, base, w, k, c, [&](int j) { return j < i; },
-          [&](int e) {
-            const int f = __ldg(&slot_src[e]) >> 1;
-            return make_double2(__ldg(imat == 1 ? &fn[f] : &fp[f]), __ldg(&fn[f]));
-          },
-          [&](const double2& a, const double (&cj)[1]) {
-            if (imat == 1)
-              d = sub(d, mul(mul(a.y, a.y), cj[0]));
-            else
-              d = sub(d, mul(mul(a.x, cj[0]), a.y));
-          });
-      if (k < w) return k;
-    }
-    c_r[i] = d;
-    st_relaxed(&c[i], 1.0 / add(d, kSmall));
-    return w;
-  });
+  sweep_rows<false, GATE, 8, 1, double2>(
+      n, R, c, ctl, [&](int i) { d = R.diag[i]; },
+      [&](int e) {
+        return make_double2(IMAT == 2 ? __ldg(&fp[__ldg(&slot_src[e]) >> 1]) : 0.0,
+                            __ldg(&R.sval[e]));
+      },
+      [&](const double2& a, const double (&cj)[1]) {
+        if (IMAT == 1)
+          d = sub(d, mul(mul(a.y, a.y), cj[0]));
+        else
+          d = sub(d, mul(mul(a.x, cj[0]), a.y));
+      },
+      [&](int i) {
+        c_r[i] = d;
+        st_relaxed(&c[i], 1.0 / add(d, kSmall));
+      });
 }
 
 // Jacobi diagonal (solv_precond.f90:13 with imat <= 0): c_r = pl, c = 1/(pl+small)
@@ -656,84 +746,75 @@ __global__ void k_precond_jacobi(int n, const double* __restrict__ diag, double*
   }
 }
 
-// slots per chunk: fewer for wide FP64 rows, which would spill
-template <typename T, int V> struct SweepChunk {
-  static constexpr int value = V == 1 ? 4 : (V >= 4 && sizeof(T) == 8 ? 1 : 2);
+// slots per chunk: fewer for several components, which would spill
+template <int V> struct SweepChunk {
+  static constexpr int value = V <= 2 ? 8 : 6;
+};
+// Blocks per SM the sweeps' registers are held to: none where the levels'
+// latency counts, enough warps for bandwidth in an order of a few levels.
+template <int V, bool GATE> struct SweepBlocks {
+  static constexpr int value = GATE ? 1 : (V <= 2 ? 4 : 3);
 };
 
 // solv_direct.f90:12-24 forward sweep, x_i = (b_i - sum_{j<i} n x_j) c_i, into
 // t (which starts out pending); the backward sweep's output x is reset to
 // pending on the way.
-template <typename T, int V>
-__global__ void __launch_bounds__(kSweepThreads, 4) k_fwd_sf(
+template <typename T, int V, bool GATE>
+__global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_fwd_sf(
     int n, Rows<T> R, const T* __restrict__ c, const T* __restrict__ bvec, T* t, T* x,
     SweepCtl* ctl, const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;
-  const int lane = threadIdx.x & 31;
   T acc[V], ci = T(0);
-  int base = 0;
-  sweep_slices<false>(n, R.slice_w, ctl, [&](int i, int k, bool first) -> int {
-    const int w = __ldg(&R.slice_w[i >> 5]);
-    if (first) {
-      if (i >= n) return w;
-      base = __ldg(&R.slice_ptr[i >> 5]) + lane;
-      ci = __ldg(&c[i]);
+  sweep_rows<false, GATE, SweepChunk<V>::value, V, T>(
+      n, R, t, ctl,
+      [&](int i) {
+        ci = __ldg(&c[i]);
 #pragma unroll
-      for (int v = 0; v < V; ++v) acc[v] = bvec[(size_t)i * V + v];
-    }
-    k = advance<SweepChunk<T, V>::value, V>(
-        R, base, w, k, t, [&](int j) { return j < i; },
-        [&](int e) { return __ldg(&R.sval[e]); },
-        [&](const T a, const T (&xv)[V]) {
+        for (int v = 0; v < V; ++v) acc[v] = bvec[(size_t)i * V + v];
+      },
+      [&](int e) { return __ldg(&R.sval[e]); },
+      [&](const T a, const T (&xv)[V]) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], mul(a, xv[v]));
-        });
-    if (k < w) return k;
+        for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], mul(a, xv[v]));
+      },
+      [&](int i) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      st_relaxed(&t[(size_t)i * V + v], mul(acc[v], ci));
-      x[(size_t)i * V + v] = Pending<T>::value();
-    }
-    return w;
-  });
+        for (int v = 0; v < V; ++v) {
+          st_relaxed(&t[(size_t)i * V + v], mul(acc[v], ci));
+          x[(size_t)i * V + v] = Pending<T>::value();
+        }
+      });
 }
 
 // solv_direct.f90:26-38 backward sweep with the x = x c_r scaling of :26:
 // x_i = (t_i c_r_i - sum_{j>i} p x_j) c_i; x starts out pending, and each
 // t_i is reset to pending once read, ready for the next forward sweep.
-template <typename T, int V>
-__global__ void __launch_bounds__(kSweepThreads, 4) k_bwd_sf(
+template <typename T, int V, bool GATE>
+__global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_bwd_sf(
     int n, Rows<T> R, const T* __restrict__ c, const T* __restrict__ c_r, T* t, T* x,
     SweepCtl* ctl, const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;
-  const int lane = threadIdx.x & 31;
   T acc[V], ci = T(0);
-  int base = 0;
-  sweep_slices<true>(n, R.slice_w, ctl, [&](int i, int k, bool first) -> int {
-    const int w = __ldg(&R.slice_w[i >> 5]);
-    if (first) {
-      if (i >= n) return w;
-      base = __ldg(&R.slice_ptr[i >> 5]) + lane;
-      ci = __ldg(&c[i]);
-      const T cr = c_r[i];
+  sweep_rows<true, GATE, SweepChunk<V>::value, V, T>(
+      n, R, x, ctl,
+      [&](int i) {
+        ci = __ldg(&c[i]);
+        const T cr = c_r[i];
 #pragma unroll
-      for (int v = 0; v < V; ++v) acc[v] = mul(t[(size_t)i * V + v], cr);
-    }
-    k = advance<SweepChunk<T, V>::value, V>(
-        R, base, w, k, x, [&](int j) { return j > i; },
-        [&](int e) { return __ldg(&R.sval[e]); },
-        [&](const T a, const T (&xv)[V]) {
+        for (int v = 0; v < V; ++v) acc[v] = mul(t[(size_t)i * V + v], cr);
+      },
+      [&](int e) { return __ldg(&R.sval[e]); },
+      [&](const T a, const T (&xv)[V]) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], mul(a, xv[v]));
-        });
-    if (k < w) return k;
+        for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], mul(a, xv[v]));
+      },
+      [&](int i) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      st_relaxed(&x[(size_t)i * V + v], mul(acc[v], ci));
-      t[(size_t)i * V + v] = Pending<T>::value();
-    }
-    return w;
-  });
+        for (int v = 0; v < V; ++v) {
+          st_relaxed(&x[(size_t)i * V + v], mul(acc[v], ci));
+          t[(size_t)i * V + v] = Pending<T>::value();
+        }
+      });
 }
 
 // Jacobi: x = b*c (solv_direct.f90:41)
@@ -1775,16 +1856,15 @@ __global__ void k_loop_ctl(cudaGraphConditionalHandle h, const int* __restrict__
   }
 }
 
-// Self-test of the recurrences' bounded wait: one slice whose only cell
-// waits on a value nothing ever writes, through the same driver
-// (sweep_slices) as the sweeps, so the wait runs out after kSweepPolls
-// polls and sets ctl->err.  slice_w holds {1}; never is pending.
-__global__ void k_sweep_selftest(const uint8_t* __restrict__ slice_w, const double* never,
-                                 SweepCtl* ctl) {
-  sweep_slices<false>(1, slice_w, ctl, [&](int i, int k, bool first) -> int {
-    double v;
-    return i == 0 && take(never, v) ? 1 : (i == 0 ? 0 : 1);
-  });
+// Self-test of the recurrences' bounded wait: a two-cell slice whose second
+// cell depends on the first one's value, which nothing ever writes, through
+// the same driver (sweep_rows) as the sweeps, so the wait runs out after
+// kSweepPolls polls and sets ctl->err.  R holds slice_ptr {0}, slice_w {1}
+// and col {-1, 0}; never holds two pending values.
+__global__ void k_sweep_selftest(Rows<double> R, const double* never, SweepCtl* ctl) {
+  sweep_rows<false, false, 1, 1, int>(
+      2, R, never, ctl, [](int) {}, [](int) { return 0; },
+      [](int, const double (&)[1]) {}, [](int) {});
 }
 
 }  // namespace sg

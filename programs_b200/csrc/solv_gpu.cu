@@ -36,6 +36,7 @@ using sg::SegMap;
 namespace {
 
 constexpr int kMaxV = 4;
+constexpr int kGateLevels = 8;
 
 struct DevBuf {
   void* p = nullptr;
@@ -1202,10 +1203,15 @@ int sweep_check(solv_gpu_ctx* c) {
   return set_err(c, SOLV_GPU_TIMEOUT, "triangular sweep: a wait for a neighbour ran out");
 }
 
+// Whether the recurrences' warps wait at the gate (sweep_rows): an order of a
+// few levels has no front to stay behind.
+bool sweep_gate(const solv_gpu_ctx* c) { return (int)c->lvl_ptr.size() - 1 >= kGateLevels; }
+
 // solv_precond: c, c_r in internal order (FP64).  DIC / DILU is one
-// sync-free recurrence over the cells (c starts out pending).
+// sync-free recurrence over the cells (c starts out pending); imat >= 3 is
+// the reference's fall-through, the unmodified diagonal.
 int launch_precond(solv_gpu_ctx* c, int imat, double* cc, double* cr) {
-  if (imat <= 0) {
+  if (imat <= 0 || imat >= 3) {
     sg::k_precond_jacobi<<<grid_for(c, c->N), c->block, 0, c->stream>>>(c->N, c->diag.as<double>(),
                                                                          cc, cr);
     c->launches++;
@@ -1214,9 +1220,10 @@ int launch_precond(solv_gpu_ctx* c, int imat, double* cc, double* cr) {
   }
   sg::k_fill_pending<double><<<grid_for(c, c->N), c->block, 0, c->stream>>>(c->N, cc);
   c->launches++;
-  return coop_launch(c, sg::k_precond_sf, c->N, imat, rows<double>(c), (const int*)c->slot_src.as<int>(),
-                     (const double*)c->fp.as<double>(), (const double*)c->fn.as<double>(), cc, cr,
-                     sweep_ctl(c));
+  auto kern = sweep_gate(c) ? (imat == 1 ? sg::k_precond_sf<1, true> : sg::k_precond_sf<2, true>)
+                            : (imat == 1 ? sg::k_precond_sf<1, false> : sg::k_precond_sf<2, false>);
+  return coop_launch(c, kern, c->N, rows<double>(c), (const int*)c->slot_src.as<int>(),
+                     (const double*)c->fp.as<double>(), cc, cr, sweep_ctl(c));
 }
 
 // x = M^-1 b  (solv_direct), internal order, V components: the forward
@@ -1238,9 +1245,12 @@ int launch_direct(solv_gpu_ctx* c, int imat, const T* cc, const T* cr, T* x, con
   }
   Rows<T> R = rows<T>(c);
   T* t = sweep_t<T>(c);
-  int rc = coop_launch(c, sg::k_fwd_sf<T, V>, c->N, R, cc, b, t, x, sweep_ctl(c), n_active);
+  const bool gate = sweep_gate(c);
+  int rc = coop_launch(c, gate ? sg::k_fwd_sf<T, V, true> : sg::k_fwd_sf<T, V, false>, c->N, R, cc, b,
+                       t, x, sweep_ctl(c), n_active);
   if (rc) return rc;
-  return coop_launch(c, sg::k_bwd_sf<T, V>, c->N, R, cc, cr, t, x, sweep_ctl(c), n_active);
+  return coop_launch(c, gate ? sg::k_bwd_sf<T, V, true> : sg::k_bwd_sf<T, V, false>, c->N, R, cc, cr,
+                     t, x, sweep_ctl(c), n_active);
 }
 
 // Workspace for V components in precision T.
@@ -2711,16 +2721,18 @@ int solv_gpu_selftest_sweep_wait(solv_gpu_ctx* c) {
   if (!c) return SOLV_GPU_BAD_INPUT;
   CUDA_TRY(c, cudaSetDevice(c->dev));
   DevBuf w, v;
-  CUDA_TRY(c, w.ensure(16));
-  CUDA_TRY(c, v.ensure(sizeof(double)));
+  CUDA_TRY(c, w.ensure(4 * sizeof(int)));  // col[2], slice_ptr[1], slice_w[1]
+  CUDA_TRY(c, v.ensure(2 * sizeof(double)));
   if (!c->sweep_ctl.p) {
     CUDA_TRY(c, c->sweep_ctl.ensure(sizeof(sg::SweepCtl)));
     CUDA_TRY(c, cudaMemsetAsync(c->sweep_ctl.p, 0, sizeof(sg::SweepCtl), c->stream));
   }
-  const uint8_t one = 1;
-  CUDA_TRY(c, cudaMemcpyAsync(w.p, &one, 1, cudaMemcpyHostToDevice, c->stream));
-  sg::k_fill_pending<double><<<1, 32, 0, c->stream>>>(1, v.as<double>());
-  sg::k_sweep_selftest<<<1, 32, 0, c->stream>>>(w.as<uint8_t>(), v.as<double>(), sweep_ctl(c));
+  const int rows2[4] = {-1, 0, 0, 1};
+  CUDA_TRY(c, cudaMemcpyAsync(w.p, rows2, sizeof(rows2), cudaMemcpyHostToDevice, c->stream));
+  sg::k_fill_pending<double><<<1, 32, 0, c->stream>>>(2, v.as<double>());
+  Rows<double> R{w.as<int>() + 2, w.as<uint8_t>() + 3 * sizeof(int), w.as<int>(), nullptr, nullptr,
+                 nullptr};
+  sg::k_sweep_selftest<<<1, 32, 0, c->stream>>>(R, v.as<double>(), sweep_ctl(c));
   CUDA_TRY(c, cudaGetLastError());
   return sweep_check(c);  // synchronises; SOLV_GPU_TIMEOUT when the wait ran out
 }

@@ -1,0 +1,86 @@
+"""The DIC/DILU recurrences (kernels.cuh: sweep_rows) on the structures where
+their chunks, their gate and their slices end: rows wider than one chunk of
+slots, slices that hold many levels (cells that wait for cells of the same
+warp), orders of few levels, several components.  Bit-exact against the
+oracle for the factorisation and the sweeps; capped solves, whose only other
+difference is the reductions' summation order (a few 1e-16 per step), to
+1e-11."""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+from programs_b200.mesh import FaceMatrix, Mesh, uniform
+
+pytestmark = pytest.mark.gpu
+
+
+def _from_pairs(n, pairs, seed):
+    """A diagonally dominant face matrix with the given couplings (1-based)."""
+    rng = np.random.default_rng(seed)
+    ip, inb = (np.array(c, np.int32) for c in zip(*pairs))
+    p, q = -rng.uniform(0.2, 1.0, (2, len(ip)))
+    pl = 1.0 - np.bincount(ip - 1, p, n) - np.bincount(inb - 1, q, n)
+    return FaceMatrix(n, ip, inb, p, q, pl)
+
+
+def _chain(n):
+    return _from_pairs(n, [(k, k + 1) for k in range(1, n)], 1)
+
+
+def _random(n, per, seed, swap=False):
+    rng = np.random.default_rng(seed)
+    pairs = {(int(a), k) for k in range(2, n + 1) for a in rng.integers(1, k, per)}
+    pairs = sorted(pairs)
+    if swap:  # owner above neighbour: the sweep coefficients differ from the product's
+        pairs = [(b, a) if (a + b) % 3 == 0 else (a, b) for a, b in pairs]
+    return _from_pairs(n, pairs, seed)
+
+
+def _hex(nx, ny, nz, order):
+    m = Mesh.hex(nx, ny, nz, jitter=0.15, seed=3, permute=True)
+    m.renumber(order)
+    return m.momentum()[0]
+
+
+CASES = {
+    "chain_70": lambda: _chain(70),
+    "chain_9": lambda: _chain(9),
+    "narrow_2x2x50": lambda: _hex(2, 2, 50, Mesh.RCM),
+    "star_41": lambda: _from_pairs(41, [(1, k) for k in range(2, 42)], 2),
+    "random_5": lambda: _random(333, 5, 4),
+    "random_13_swapped": lambda: _random(500, 13, 5, swap=True),
+    "hex_rcm": lambda: _hex(11, 13, 12, Mesh.RCM),
+    "hex_color": lambda: _hex(11, 13, 12, Mesh.COLOR),
+    "one_deep": lambda: _hex(37, 21, 1, Mesh.RCM),
+}
+
+
+@pytest.fixture(scope="module", params=sorted(CASES))
+def case(request, gpu):
+    A = CASES[request.param]()
+    gpu.matrix_set(A)
+    return A, Oracle.from_matrix(A)
+
+
+@pytest.mark.parametrize("imat", [1, 2])
+def test_factorisation_and_sweeps(gpu, case, imat):
+    A, o = case
+    c_ref, cr_ref = o.solv_precond(imat)
+    c, cr = np.empty(A.n_cell), np.empty(A.n_cell)
+    gpu.solv_precond(imat, c, cr)
+    assert np.array_equal(cr, cr_ref) and np.array_equal(c, c_ref)
+    for seed in (9, 10):  # the second finds the buffers as the first left them
+        b = uniform(seed, A.n_cell)
+        x = np.zeros(A.n_cell)
+        gpu.solv_direct(imat, c, cr, x, b)
+        assert np.array_equal(x, o.solv_direct(imat, c_ref, cr_ref, b))
+
+
+@pytest.mark.parametrize("V", [1, 2, 3, 4])
+def test_capped_bicg(gpu, case, V):
+    A, o = case
+    phi = uniform(5, A.n_cell * V).reshape(A.n_cell, V).copy()
+    b = uniform(6, A.n_cell * V).reshape(V, A.n_cell).T.copy(order="F")
+    ref = o.solv_bicg(2, 1e-30, 2, phi.copy(), b.copy(order="F"))
+    gpu.solv_bicg(2, 1e-30, 2, phi, b, np.zeros(V))
+    assert np.linalg.norm(phi - ref[0]) <= 1e-11 * np.linalg.norm(ref[0])
