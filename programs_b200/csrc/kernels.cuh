@@ -561,9 +561,20 @@ __global__ void k_fill_pending(long long n, T* __restrict__ x) {
 // sector per poll: the last dependency of the last cell its slice depends
 // on, an ancestor two steps back (one step back was 4% slower).  Only the
 // slices next to the front then poll their own inputs.
+// A batch's systems are recurrences of their own, one after the other in the
+// internal order; in index order the front would pass through them one by
+// one, so with GATE the blocks are dealt out to the systems (SweepMap), and
+// a slice that holds the end of one system and the start of the next is
+// visited for each.
 constexpr int kSweepSpin = 64;
 constexpr int kSweepSleep = 64;  // ns
 constexpr int kGateSleep = 32;   // ns
+
+struct SweepMap {
+  const int* __restrict__ c0;  // the systems' cell ranges
+  const int* __restrict__ c1;
+  int n_sys;
+};
 
 template <bool UP>
 __device__ __forceinline__ bool sweep_dep(int j, int i) {
@@ -572,19 +583,49 @@ __device__ __forceinline__ bool sweep_dep(int j, int i) {
 
 template <bool UP, bool GATE, int C, int V, typename A, typename T, typename Start, typename Coef,
           typename Use, typename Finish>
-__device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const T* vals, SweepCtl* ctl,
-                                           Start&& start, Coef&& coef, Use&& use,
-                                           Finish&& finish) {
+__device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const SweepMap& sm,
+                                           const T* vals, SweepCtl* ctl, Start&& start,
+                                           Coef&& coef, Use&& use, Finish&& finish) {
   using P = Pending<T>;
   using U = typename P::U;
   constexpr unsigned full = 0xffffffffu;
   const U* bits_of = reinterpret_cast<const U*>(vals);
   const int lane = threadIdx.x & 31;
-  const int ns = (n + 31) >> 5;
-  const int W = gridDim.x * (blockDim.x >> 5);
-  const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  for (int r = gw; r < ns; r += W) {
-    const int s = UP ? ns - 1 - r : r;
+  // this block's systems (sys, sys + step, ...), its rank among theirs
+  int sys = 0, step = 1, rank = blockIdx.x, nblk = gridDim.x;
+  const bool by_sys = GATE && sm.n_sys > 1;
+  if (by_sys && sm.n_sys >= (int)gridDim.x) {
+    sys = blockIdx.x;
+    step = gridDim.x;
+    rank = 0;
+    nblk = 1;
+  } else if (by_sys) {
+    step = sm.n_sys;
+    const int per = gridDim.x / sm.n_sys, more = gridDim.x % sm.n_sys;
+    const int cut = more * (per + 1), b = blockIdx.x;
+    nblk = b < cut ? per + 1 : per;
+    sys = b < cut ? b / nblk : more + (b - cut) / nblk;
+    rank = (b < cut ? b : b - cut) % nblk;
+  }
+  const int warps = blockDim.x >> 5;
+  int c0 = 0, c1 = n;
+  int r = rank * warps + (threadIdx.x >> 5);
+  const int r0 = r, W = nblk * warps;
+  if (by_sys) {
+    c0 = sm.c0[sys];
+    c1 = sm.c1[sys];
+  }
+  for (;; r += W) {
+    const int s_lo = c0 >> 5, ns = ((c1 + 31) >> 5) - s_lo;
+    if (r >= ns) {  // this system is done: the block's next
+      sys += step;
+      if (!by_sys || sys >= sm.n_sys) break;
+      c0 = sm.c0[sys];
+      c1 = sm.c1[sys];
+      r = r0 - W;
+      continue;
+    }
+    const int s = s_lo + (UP ? ns - 1 - r : r);
     const int i = s * 32 + lane;
     const int w = __ldg(&R.slice_w[s]);
     const int base = __ldg(&R.slice_ptr[s]) + lane;
@@ -593,7 +634,7 @@ __device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const T* val
     U bits[C][V];
     int nd = 0, k0 = 0;
     unsigned mask = 0;
-    bool done = i >= n;
+    bool done = i < c0 || i >= c1;
     auto on = [&](int q) { return GATE ? q < nd : ((mask >> q) & 1u) != 0; };
     auto load = [&]() {
       int j[C], du[C];
@@ -715,11 +756,11 @@ __device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const T* val
 // from its face.
 template <int IMAT, bool GATE>
 __global__ void __launch_bounds__(kSweepThreads, 1) k_precond_sf(
-    int n, Rows<double> R, const int* __restrict__ slot_src,
+    int n, Rows<double> R, SweepMap sm, const int* __restrict__ slot_src,
     const double* __restrict__ fp, double* c, double* __restrict__ c_r, SweepCtl* ctl) {
   double d = 0.0;
   sweep_rows<false, GATE, 8, 1, double2>(
-      n, R, c, ctl, [&](int i) { d = R.diag[i]; },
+      n, R, sm, c, ctl, [&](int i) { d = R.diag[i]; },
       [&](int e) {
         return make_double2(IMAT == 2 ? __ldg(&fp[__ldg(&slot_src[e]) >> 1]) : 0.0,
                             __ldg(&R.sval[e]));
@@ -761,12 +802,12 @@ template <int V, bool GATE> struct SweepBlocks {
 // pending on the way.
 template <typename T, int V, bool GATE>
 __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_fwd_sf(
-    int n, Rows<T> R, const T* __restrict__ c, const T* __restrict__ bvec, T* t, T* x,
+    int n, Rows<T> R, SweepMap sm, const T* __restrict__ c, const T* __restrict__ bvec, T* t, T* x,
     SweepCtl* ctl, const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;
   T acc[V], ci = T(0);
   sweep_rows<false, GATE, SweepChunk<V>::value, V, T>(
-      n, R, t, ctl,
+      n, R, sm, t, ctl,
       [&](int i) {
         ci = __ldg(&c[i]);
 #pragma unroll
@@ -791,12 +832,12 @@ __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_
 // t_i is reset to pending once read, ready for the next forward sweep.
 template <typename T, int V, bool GATE>
 __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_bwd_sf(
-    int n, Rows<T> R, const T* __restrict__ c, const T* __restrict__ c_r, T* t, T* x,
+    int n, Rows<T> R, SweepMap sm, const T* __restrict__ c, const T* __restrict__ c_r, T* t, T* x,
     SweepCtl* ctl, const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;
   T acc[V], ci = T(0);
   sweep_rows<true, GATE, SweepChunk<V>::value, V, T>(
-      n, R, x, ctl,
+      n, R, sm, x, ctl,
       [&](int i) {
         ci = __ldg(&c[i]);
         const T cr = c_r[i];
@@ -1863,7 +1904,7 @@ __global__ void k_loop_ctl(cudaGraphConditionalHandle h, const int* __restrict__
 // and col {-1, 0}; never holds two pending values.
 __global__ void k_sweep_selftest(Rows<double> R, const double* never, SweepCtl* ctl) {
   sweep_rows<false, false, 1, 1, int>(
-      2, R, never, ctl, [](int) {}, [](int) { return 0; },
+      2, R, SweepMap{nullptr, nullptr, 1}, never, ctl, [](int) {}, [](int) { return 0; },
       [](int, const double (&)[1]) {}, [](int) {});
 }
 

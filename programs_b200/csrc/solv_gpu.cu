@@ -1173,7 +1173,9 @@ int coop_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), Args... args) {
     c->coop_blocks[(const void*)kern] = per_sm;
   }
   const long long warps = ((long long)c->N + 31) / 32;
-  const long long want = (warps + sg::kSweepThreads / 32 - 1) / (sg::kSweepThreads / 32);
+  // (a block per system of a batch at least)
+  const long long want = std::max<long long>((warps + sg::kSweepThreads / 32 - 1) / (sg::kSweepThreads / 32),
+                                             c->n_seg);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)std::max(1LL, std::min<long long>(want, (long long)per_sm * c->n_sm)));
   cfg.blockDim = dim3(sg::kSweepThreads);
@@ -1207,6 +1209,11 @@ int sweep_check(solv_gpu_ctx* c) {
 // few levels has no front to stay behind.
 bool sweep_gate(const solv_gpu_ctx* c) { return (int)c->lvl_ptr.size() - 1 >= kGateLevels; }
 
+sg::SweepMap sweep_map(solv_gpu_ctx* c) {
+  const SegMap m = segmap(c);
+  return {m.seg_c0, m.seg_c1, c->n_seg};
+}
+
 // solv_precond: c, c_r in internal order (FP64).  DIC / DILU is one
 // sync-free recurrence over the cells (c starts out pending); imat >= 3 is
 // the reference's fall-through, the unmodified diagonal.
@@ -1222,7 +1229,7 @@ int launch_precond(solv_gpu_ctx* c, int imat, double* cc, double* cr) {
   c->launches++;
   auto kern = sweep_gate(c) ? (imat == 1 ? sg::k_precond_sf<1, true> : sg::k_precond_sf<2, true>)
                             : (imat == 1 ? sg::k_precond_sf<1, false> : sg::k_precond_sf<2, false>);
-  return coop_launch(c, kern, c->N, rows<double>(c), (const int*)c->slot_src.as<int>(),
+  return coop_launch(c, kern, c->N, rows<double>(c), sweep_map(c), (const int*)c->slot_src.as<int>(),
                      (const double*)c->fp.as<double>(), cc, cr, sweep_ctl(c));
 }
 
@@ -1246,11 +1253,11 @@ int launch_direct(solv_gpu_ctx* c, int imat, const T* cc, const T* cr, T* x, con
   Rows<T> R = rows<T>(c);
   T* t = sweep_t<T>(c);
   const bool gate = sweep_gate(c);
-  int rc = coop_launch(c, gate ? sg::k_fwd_sf<T, V, true> : sg::k_fwd_sf<T, V, false>, c->N, R, cc, b,
-                       t, x, sweep_ctl(c), n_active);
+  int rc = coop_launch(c, gate ? sg::k_fwd_sf<T, V, true> : sg::k_fwd_sf<T, V, false>, c->N, R,
+                       sweep_map(c), cc, b, t, x, sweep_ctl(c), n_active);
   if (rc) return rc;
-  return coop_launch(c, gate ? sg::k_bwd_sf<T, V, true> : sg::k_bwd_sf<T, V, false>, c->N, R, cc, cr,
-                     t, x, sweep_ctl(c), n_active);
+  return coop_launch(c, gate ? sg::k_bwd_sf<T, V, true> : sg::k_bwd_sf<T, V, false>, c->N, R,
+                     sweep_map(c), cc, cr, t, x, sweep_ctl(c), n_active);
 }
 
 // Workspace for V components in precision T.

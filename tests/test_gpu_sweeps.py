@@ -84,3 +84,19 @@ def test_capped_bicg(gpu, case, V):
     ref = o.solv_bicg(2, 1e-30, 2, phi.copy(), b.copy(order="F"))
     gpu.solv_bicg(2, 1e-30, 2, phi, b, np.zeros(V))
     assert np.linalg.norm(phi - ref[0]) <= 1e-11 * np.linalg.norm(ref[0])
+
+
+@pytest.mark.parametrize("n_sys", [2, 13, 900])  # fewer systems than blocks, and more
+def test_batch_of_systems_that_share_slices(gpu, n_sys):
+    """Systems end inside slices; each must come out as by itself."""
+    mats = [_hex(2 + k % 3, 3, 2 + k % 5, Mesh.RCM) if k % 4 else _chain(3 + k % 37)
+            for k in range(n_sys - 1)] + [_hex(9, 10, 11, Mesh.RCM)]
+    cp = gpu.matrix_set_batch(mats)
+    b = uniform(4, cp[-1])
+    phi = np.zeros((cp[-1], 1))
+    gpu.solv_bicg_batch(2, 1e-30, 2, phi, np.asfortranarray(b.reshape(-1, 1).copy()))
+    for k in sorted({0, 1, n_sys // 2, n_sys - 2, n_sys - 1}):
+        sl = slice(cp[k], cp[k + 1])
+        ref = Oracle.from_matrix(mats[k]).solv_bicg(2, 1e-30, 2, np.zeros((mats[k].n_cell, 1)),
+                                                    b[sl].reshape(-1, 1))
+        assert np.linalg.norm(phi[sl] - ref[0]) <= 1e-11 * np.linalg.norm(ref[0])
