@@ -1425,6 +1425,302 @@ __global__ void SG_BOUNDS(1) k_fcg_update(SegMap sm, T* __restrict__ phi, T* __r
   }
 }
 
+// ============ resident Jacobi PCG: the whole GPU on one loop, matrix in shared memory ============
+// The Krylov loop of solv_cg.f90:37-84 with imat = 0 as one cooperative
+// launch, for systems (one, or a batch of at most one per SM) whose matrix
+// fits the SMs' shared memory: as a graph of step kernels an iteration of a
+// small system is three launches and three reduction tails (14-16 us at
+// 32^3), none of it bandwidth.  Each block owns a run of consecutive cells
+// of one system, one block per SM: their slots in shared memory (slot-major,
+// so the reads are free of bank conflicts; slots past the capacity stay in
+// global memory), their r, c, phi, p and q in registers.  Two block-to-block
+// exchanges an iteration are left: p.q, and |r|_1 with r.z.  The p kernel's
+// exchange goes because a block forms its neighbours' p itself: every cell
+// publishes the pair {z, p} once r is updated, one 16-byte gather per slot,
+// and p_j = z_j + beta p_j is the owner's own operation, bit for bit.
+// In an exchange a block pushes its partials into every block's inbox, and
+// the value is the flag (an entry holds the pending pattern until it is
+// written): no counter, no atomic, one trip through L2, and nobody polls a
+// line that others poll (148 blocks polling one shared array took 3 000 -
+// 4 000 cycles a time, an inbox each about 1 000).  Every block sums its
+// inbox in the same fixed tree, so all hold the same scalars and stop
+// together, and the sums are deterministic.  The second exchange also
+// publishes the pairs: release before the push, acquire after the poll.
+// Before that release each block puts its inbox of the other parity back to
+// pending: it has read it already, and the next to write there has to pass
+// this exchange first.  The acquire also drops the L1's old pairs, so the
+// gathers of one iteration may share lines there.
+// Measured: see kGridShapes (solv_gpu.cu).
+constexpr int kGridMaxCells = 6144;  // cells a block owns
+constexpr int kGridMaxBlocks = 160;  // inbox entries: five a lane
+
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void st_bits(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Fixed-order warp sum, the result in every lane.
+__device__ __forceinline__ double warp_sum_all(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// One warp: push this block's NV partials t into the inboxes of the system's
+// nb blocks (entry `rank` of each; `stride` words from one block's inbox to
+// the next) and return all the blocks' sums in t.  False when the wait ran
+// out.
+template <int NV>
+__device__ __forceinline__ bool push_and_total(unsigned long long* inbox0, size_t stride, int rank,
+                                               int nb, double (&t)[NV], SweepCtl* ctl) {
+  using P = Pending<double>;
+  constexpr int Q = kGridMaxBlocks / 32;
+  const int l = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (l + 32 * q < nb)
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        st_bits(inbox0 + (l + 32 * q) * stride + (size_t)v * kGridMaxBlocks + rank,
+                (unsigned long long)__double_as_longlong(t[v]));
+  const unsigned long long* mine = inbox0 + rank * stride;
+  unsigned long long bits[Q][NV];
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) bits[q][v] = 0;
+  for (int poll = 0;; ++poll) {
+    bool ready = true;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        ld_relaxed_if(l + 32 * q < nb, mine + (size_t)v * kGridMaxBlocks + l + 32 * q, bits[q][v]);
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) ready &= bits[q][v] != P::bits;
+    if (__all_sync(0xffffffffu, ready)) break;
+    if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
+      if (l == 0) atomicExch(&ctl->err, 1);
+      return false;
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    t[v] = 0.0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) t[v] += P::from(bits[q][v]);  // 0 past the last block
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) t[v] = warp_sum_all(t[v]);
+  return true;
+}
+
+// inbox: per block, per parity, three rows of kGridMaxBlocks words (p.q;
+// |r|_1; r.z), all pending.
+constexpr int kInboxWords = 3 * kGridMaxBlocks;
+
+template <int B, int RPT, bool BIG>
+__global__ void __launch_bounds__(B, 1) k_pcg_grid(
+    Rows<double> R, SegMap sm, int W, int resident, const double* __restrict__ c,
+    double* __restrict__ phi, const double* __restrict__ r_in, double2* zp,
+    unsigned long long* inbox, Lane* __restrict__ lanes, SweepCtl* ctl) {
+  constexpr int NW = B / 32;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  double* val_s = reinterpret_cast<double*>(dyn);
+  int* col_s = reinterpret_cast<int*>(val_s + (size_t)resident * W * B);
+  __shared__ double red[2][32];
+  __shared__ double tot_s[2];
+  __shared__ int fail_s;
+  const int b = blockIdx.x, sys = sm.blk_seg[b], nb = sm.seg_nblk[sys], b0 = sm.seg_blk0[sys];
+  const int rank = sm.blk_rank[b];
+  const int c0 = sm.seg_c0[sys], c1 = sm.seg_c1[sys];
+  const int chunk = (((c1 - c0) + nb - 1) / nb + 31) & ~31;
+  const int lo = c0 + rank * chunk, hi = min(lo + chunk, c1);
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  const Lane L0 = lanes[sys];
+  if (!L0.active) return;  // uniform over the system's blocks
+  if (tid == 0) fail_s = 0;
+  constexpr int NR = BIG ? 1 : RPT;  // BIG: c and phi stay in global memory
+  double rr[RPT], pp[RPT], qq[RPT], cc[NR], ph[NR];
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    const int i = lo + k * B + tid;
+    const bool h = i < hi;
+    rr[k] = h ? r_in[i] : 0.0;
+    if constexpr (!BIG) {
+      cc[k] = h ? c[i] : 0.0;
+      ph[k] = h ? phi[i] : 0.0;
+    }
+    pp[k] = qq[k] = 0.0;
+    if (k < resident) {
+      int base = 0, wi = 0;
+      if (h) {
+        RowIt<double> it(R, i);
+        base = it.base;
+        wi = it.w;
+      }
+      for (int u = 0; u < W; ++u) {
+        const int e = base + u * kWarp;
+        val_s[(k * W + u) * B + tid] = u < wi ? R.val[e] : 0.0;
+        col_s[(k * W + u) * B + tid] = u < wi ? R.col[e] : -1;
+      }
+    }
+  }
+  auto c_of = [&](int k, int i) { return BIG ? __ldg(&c[i]) : cc[BIG ? 0 : k]; };
+  // The sums over the system's blocks of every thread's t[], in parity par's
+  // inbox; two values: the exchange that also publishes the pairs.
+  auto exchange = [&](auto& t, int par) -> bool {
+    constexpr int NV = sizeof(t) / sizeof(double);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) t[v] = warp_sum(t[v]);
+    if (l == 0)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) red[v][w] = t[v];
+    if (NV == 2 && nb > 1 && w == NW - 1) {  // this block's other inbox back to pending
+      unsigned long long* o = inbox + ((size_t)b * 2 + (par ^ 1)) * kInboxWords;
+      for (int q = l; q < nb; q += 32)
+#pragma unroll
+        for (int v = 0; v < 3; ++v) st_bits(o + v * kGridMaxBlocks + q, Pending<double>::bits);
+    }
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) t[v] = l < NW ? red[v][l] : 0.0;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) t[v] = warp_sum_all(t[v]);
+      bool ok = true;
+      if (nb > 1) {
+        if (NV == 2) fence_gpu();
+        ok = push_and_total<NV>(inbox + ((size_t)b0 * 2 + par) * kInboxWords +
+                                    (NV == 2 ? kGridMaxBlocks : 0),
+                                2 * (size_t)kInboxWords, rank, nb, t, ctl);
+        if (NV == 2) fence_gpu();
+      }
+      if (l == 0) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) tot_s[v] = t[v];
+        if (!ok) fail_s = 1;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) t[v] = tot_s[v];
+    return fail_s == 0;
+  };
+  const double res0_n = L0.res0_n, reduc = L0.reduc;
+  const int n_iter = L0.n_iter;
+  double s_cur = L0.s, s_prev = L0.s_prev, beta = 0.0, alpha = L0.alpha, pq = L0.pq;
+  double l1v = L0.l1, ratio = L0.ratio;
+  int iter = L0.iter, status = kLaneRunning, par = 1;
+  {  // s = r.(c r), beta = (1/s_old) s (k_cg_rz with JAC); the first pairs, p = 0
+    double t[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int i = lo + k * B + tid;
+      if (i < hi) {
+        const double z = mul(rr[k], c_of(k, i));
+        t[1] += prod(rr[k], z);
+        __stcg(&zp[i], make_double2(z, 0.0));
+      }
+    }
+    if (!exchange(t, par)) return;
+    const double b0s = 1.0 / s_cur;
+    s_prev = s_cur;
+    s_cur = t[1];
+    beta = b0s * s_cur;
+  }
+  while (true) {
+    par ^= 1;
+    // p = z + beta p here and at the neighbours; q = A p, p.q
+    double a[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int i = lo + k * B + tid;
+      if (i >= hi) continue;
+      pp[k] = add(mul(rr[k], c_of(k, i)), mul(beta, pp[k]));
+      double y = mul(__ldg(&R.diag[i]), pp[k]);
+      const bool here = k < resident;
+      const RowIt<double> it(R, i);
+      const int wi = here ? W : it.w;
+      for (int u0 = 0; u0 < wi; u0 += 6) {
+        int j[6];
+        double av[6];
+        double2 x[6];
+#pragma unroll
+        for (int u = 0; u < 6; ++u) {
+          j[u] = -1;
+          av[u] = 0.0;
+          if (u0 + u < wi) {
+            const int at = (k * W + u0 + u) * B + tid, e = it.base + (u0 + u) * kWarp;
+            j[u] = here ? col_s[at] : __ldg(&R.col[e]);
+            av[u] = here ? val_s[at] : __ldg(&R.val[e]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 6; ++u) x[u] = j[u] >= 0 ? zp[j[u]] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 6; ++u)
+          if (j[u] >= 0) y = add(y, mul(av[u], add(x[u].x, mul(beta, x[u].y))));
+      }
+      qq[k] = y;
+      a[0] += prod(pp[k], y);
+    }
+    if (!exchange(a, par)) return;
+    pq = a[0];
+    alpha = s_cur / (pq + kSmall);  // solv_cg.f90:67-68
+    // phi += alpha p; r -= alpha q; |r|_1; r.(c r) (k_cg_update with JAC)
+    double t[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int i = lo + k * B + tid;
+      if (i >= hi) continue;
+      if constexpr (BIG) phi[i] = add(phi[i], mul(alpha, pp[k]));
+      else ph[k] = add(ph[k], mul(alpha, pp[k]));
+      const double rn = sub(rr[k], mul(alpha, qq[k]));
+      const double z = mul(rn, c_of(k, i));
+      rr[k] = rn;
+      t[0] += fabs(rn);
+      t[1] += prod(rn, z);
+      __stcg(&zp[i], make_double2(z, pp[k]));
+    }
+    if (!exchange(t, par)) return;
+    iter += 1;
+    l1v = t[0];
+    ratio = l1v / (res0_n + kSmall);  // solv_cg.f90:81
+    if (!(ratio == ratio) || isinf(ratio)) status = kLaneNaN;
+    else if (ratio < reduc) status = kLaneConverged;  // :82
+    else if (iter >= n_iter) status = kLaneMaxIter;
+    if (status != kLaneRunning) break;
+    const double b1 = 1.0 / s_cur;
+    s_prev = s_cur;
+    s_cur = t[1];
+    beta = b1 * s_cur;
+  }
+  if constexpr (!BIG) {
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const int i = lo + k * B + tid;
+      if (i < hi) phi[i] = ph[k];
+    }
+  }
+  if (rank == 0 && tid == 0) {
+    Lane L = L0;
+    L.s = s_cur;
+    L.s_prev = s_prev;
+    L.beta = beta;
+    L.alpha = alpha;
+    L.pq = pq;
+    L.iter = iter;
+    L.l1 = l1v;
+    L.ratio = ratio;
+    L.active = 0;
+    L.status = status;
+    lanes[sys] = L;
+    atomicSub(sm.n_active, 1);
+  }
+}
+
 // ============ persistent fused Jacobi PCG: one thread-block cluster per system ============
 // The whole Krylov loop of solv_cg.f90:37-84 with imat = 0 in one launch:
 // each cluster of CTAs (kPcgCluster, or kPcgClusterMax where the GPU holds
@@ -1883,6 +2179,31 @@ __global__ void k_block_locality(int n, Rows<double> R, const int* __restrict__ 
   if ((threadIdx.x & 31) == 0 && tot) {
     atomicAdd(&cnt[0], tot);
     atomicAdd(&cnt[1], loc);
+  }
+}
+
+// How well a warp's gathers share lines: over all pairs of neighbouring cells
+// of a slice and each slot, how many read columns at most two apart (cnt[0]
+// pairs, cnt[1] near ones).
+__global__ void k_near_slots(int n, Rows<double> R, unsigned long long* __restrict__ cnt) {
+  const int lane = threadIdx.x & 31, ns = (n + 31) >> 5;
+  const int W = gridDim.x * (blockDim.x >> 5);
+  unsigned tot = 0, near = 0;
+  for (int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < ns; s += W) {
+    const int w = R.slice_w[s], base = R.slice_ptr[s] + lane;
+    for (int k = 0; k < w; ++k) {
+      const int j = s * 32 + lane < n ? R.col[base + k * kWarp] : -1;
+      const int before = __shfl_up_sync(0xffffffffu, j, 1);
+      if (lane == 0 || j < 0 || before < 0) continue;
+      ++tot;
+      near += abs(j - before) <= 2;
+    }
+  }
+  tot = __reduce_add_sync(0xffffffffu, tot);
+  near = __reduce_add_sync(0xffffffffu, near);
+  if (lane == 0) {
+    atomicAdd(&cnt[0], (unsigned long long)tot);
+    atomicAdd(&cnt[1], (unsigned long long)near);
   }
 }
 

@@ -185,6 +185,13 @@ struct solv_gpu_ctx {
   int persistent = 0;                  // FP64 Jacobi PCG as one cluster-persistent launch
   std::map<const void*, int> pcg_max16;  // clusters of 16 resident at once, per kernel
   std::map<int, double> pcg_local;       // share of slots within their own block of 2^k cells
+  // the resident PCG's block map of the current structure (resident_plan)
+  int max_w = 0;                         // widest slice
+  bool grid_planned = false;
+  int grid_shape = -1;                   // of kGridShapes; -1: the systems do not fit
+  int grid_res = 0;                      // a thread's cells with their slots in shared memory
+  int grid_blk = 0, grid_smem = 0;
+  DevBuf grid_map, grid_inbox, grid_zp;
   int gnn_layer_blocks = 0;              // resident blocks per SM of k_gnn_layer_tc
   int fcg_stall_iters = 1000;
   double fcg_stall_drop = 0.9;
@@ -443,6 +450,9 @@ int matrix_structure(solv_gpu_ctx* c, int N, int F, const int* ip, const int* in
   c->mg_valid = false;
   c->mg.clear();
   c->pcg_local.clear();
+  c->grid_planned = false;
+  c->max_w = 0;
+  for (uint8_t w : sw) c->max_w = std::max(c->max_w, (int)w);
   cudaStream_t st = c->stream;
   CUDA_TRY(c, c->old_of_new.ensure(N * sizeof(int)));
   CUDA_TRY(c, c->slice_ptr.ensure((ns + 1) * sizeof(int)));
@@ -1592,6 +1602,141 @@ int iterate(solv_gpu_ctx* c, int solver, int imat, int n_iter, WS<T>& w, int& gr
   return SOLV_GPU_OK;
 }
 
+// ---- resident PCG (k_pcg_grid) --------------------------------------------------
+using GridKernel = void (*)(Rows<double>, SegMap, int, int, const double*, double*, const double*,
+                            double2*, unsigned long long*, Lane*, sg::SweepCtl*);
+struct GridShape {
+  int threads, rpt;  // threads a block, cells a thread
+  GridKernel kern;
+};
+const GridShape kGridShapes[] = {{256, 1, sg::k_pcg_grid<256, 1, false>},
+                                 {512, 1, sg::k_pcg_grid<512, 1, false>},
+                                 {1024, 1, sg::k_pcg_grid<1024, 1, false>},
+                                 {1024, 2, sg::k_pcg_grid<1024, 2, false>},
+                                 {1024, 3, sg::k_pcg_grid<1024, 3, false>},
+                                 {1024, 4, sg::k_pcg_grid<1024, 4, true>},
+                                 {1024, 6, sg::k_pcg_grid<1024, 6, true>}};
+constexpr int kGridShapeCount = sizeof(kGridShapes) / sizeof(kGridShapes[0]);
+
+// Blocks of the resident PCG for the current structure, once per structure:
+// one block each to begin with, the rest of the SMs, one by one, to whichever
+// system will run longest -- iterations, which grow with the edge of the
+// mesh, times an iteration's fixed part (worth kGridFixed cells) and its
+// cells -- as long as that leaves kGridMinCells a block (32^3: 2.46 ms with
+// 128 cells a block on all SMs, 2.08 with 512 on 64).  It fits when no block
+// owns more than kGridMaxCells cells and there are no more systems than SMs.
+// Beyond kGridAnyOrder cells a block the gathers of the pairs fill L1 and
+// decide: in RCM order the loop stays ahead of the step kernels to the end
+// (ms to 1e-10, step kernels against this: 64^3 12.9 / 6.5, 76^3 18.3 / 10.5,
+// 80^3 20.5 / 13.9, 96^3 38.3 / 31.0), in a random order only up to there
+// (64^3 15.7 / 9.5, 72^3 20.8 / 21.7, 90^3 37.4 / 51.1); k_near_slots tells.
+constexpr int kGridMinCells = 512;
+constexpr int kGridFixed = 2500;
+constexpr int kGridAnyOrder = 2048;
+
+int resident_plan(solv_gpu_ctx* c) {
+  if (c->grid_planned) return SOLV_GPU_OK;
+  c->grid_planned = true;
+  c->grid_shape = -1;
+  const int ns = c->n_seg, cap = std::min(c->n_sm, sg::kGridMaxBlocks);
+  if (ns > cap || c->N > (long long)cap * sg::kGridMaxCells) return SOLV_GPU_OK;
+  std::vector<int> n(ns), nb(ns, 1);
+  for (int k = 0; k < ns; ++k) n[k] = c->seg_c1_caller[k] - c->seg_c0_caller[k];
+  auto run_time = [&](int k) {
+    const double cells = (double)n[k] / nb[k];
+    if (cells > sg::kGridMaxCells) return 1e30 * cells;  // must be split
+    return cells <= kGridMinCells ? 0.0 : std::cbrt((double)n[k]) * (kGridFixed + cells);
+  };
+  for (int used = ns; used < cap; ++used) {
+    int most = 0;
+    for (int k = 1; k < ns; ++k)
+      if (run_time(k) > run_time(most)) most = k;
+    if (run_time(most) == 0.0) break;
+    nb[most]++;
+  }
+  int chunk = 0, total = 0;
+  for (int k = 0; k < ns; ++k) {
+    chunk = std::max(chunk, ((n[k] + nb[k] - 1) / nb[k] + 31) & ~31);
+    total += nb[k];
+  }
+  int shape = 0;
+  while (shape < kGridShapeCount && kGridShapes[shape].threads * kGridShapes[shape].rpt < chunk)
+    ++shape;
+  if (shape == kGridShapeCount) return SOLV_GPU_OK;
+  if (chunk > kGridAnyOrder) {
+    unsigned long long h[2] = {0, 0};
+    DevBuf cnt;
+    CUDA_TRY(c, cnt.ensure(sizeof(h)));
+    CUDA_TRY(c, cudaMemsetAsync(cnt.p, 0, sizeof(h), c->stream));
+    sg::k_near_slots<<<grid_for(c, c->N), c->block, 0, c->stream>>>(c->N, rows<double>(c),
+                                                                    cnt.as<unsigned long long>());
+    CUDA_TRY(c, cudaMemcpyAsync(h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (2 * h[1] < h[0]) return SOLV_GPU_OK;
+  }
+  const GridShape& G = kGridShapes[shape];
+  cudaFuncAttributes fa;
+  int optin = 0;
+  CUDA_TRY(c, cudaFuncGetAttributes(&fa, G.kern));
+  CUDA_TRY(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
+  const int row = std::max(c->max_w, 1) * G.threads * 12;  // one cell a thread
+  const int res = std::min(G.rpt, (optin - (int)fa.sharedSizeBytes) / row);
+  CUDA_TRY(c, cudaFuncSetAttribute(G.kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   optin - (int)fa.sharedSizeBytes));
+  std::vector<int> m;  // blk_seg, blk_rank, seg_nblk, seg_blk0, seg_c0, seg_c1
+  for (int k = 0; k < ns; ++k) m.insert(m.end(), nb[k], k);
+  for (int k = 0; k < ns; ++k)
+    for (int r = 0; r < nb[k]; ++r) m.push_back(r);
+  m.insert(m.end(), nb.begin(), nb.end());
+  for (int k = 0, b0 = 0; k < ns; b0 += nb[k++]) m.push_back(b0);
+  m.insert(m.end(), c->seg_c0_caller.begin(), c->seg_c0_caller.end());
+  m.insert(m.end(), c->seg_c1_caller.begin(), c->seg_c1_caller.end());
+  CUDA_TRY(c, upload(c->grid_map, m, c->stream));
+  CUDA_TRY(c, c->grid_inbox.ensure((size_t)2 * sg::kInboxWords * total * sizeof(double)));
+  CUDA_TRY(c, c->grid_zp.ensure((size_t)c->N * sizeof(double2)));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // m dies here
+  c->grid_blk = total;
+  c->grid_smem = res * row;
+  c->grid_res = res;
+  c->grid_shape = shape;
+  return SOLV_GPU_OK;
+}
+
+// The whole loop from r0 (the initial residual) and the Jacobi c into phi.
+int resident_pcg(solv_gpu_ctx* c, const double* cc, double* phi, const double* r0) {
+  const int nb = c->grid_blk, ns = c->n_seg;
+  const GridShape& G = kGridShapes[c->grid_shape];
+  int* m = c->grid_map.as<int>();
+  SegMap sm;
+  sm.blk_seg = m;
+  sm.blk_rank = m + nb;
+  sm.seg_nblk = m + 2 * nb;
+  sm.seg_blk0 = m + 2 * nb + ns;
+  sm.seg_c0 = m + 2 * nb + 2 * ns;
+  sm.seg_c1 = m + 2 * nb + 3 * ns;
+  sm.ticket = nullptr;
+  sm.n_active = c->n_active.as<int>();
+  const long long words = 2LL * sg::kInboxWords * nb;
+  sg::k_fill_pending<double><<<grid_for(c, words), c->block, 0, c->stream>>>(
+      words, c->grid_inbox.as<double>());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nb);
+  cfg.blockDim = dim3((unsigned)G.threads);
+  cfg.dynamicSmemBytes = (size_t)c->grid_smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(c, cudaLaunchKernelEx(&cfg, G.kern, rows<double>(c), sm, std::max(c->max_w, 1),
+                                 c->grid_res, cc, phi, r0, c->grid_zp.as<double2>(),
+                                 c->grid_inbox.as<unsigned long long>(), c->lanes.as<Lane>(),
+                                 sweep_ctl(c)));
+  c->launches += 2;
+  return SOLV_GPU_OK;
+}
+
 // Full FP64 solve (solver 0 = CG, 1 = BiCGSTAB) on device buffers in the
 // caller layouts.
 template <int V>
@@ -1627,11 +1772,22 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
     return SOLV_GPU_OK;
   }
   if ((rc = launch_precond(c, imat, w.c, w.cr))) return rc;  // solv_precond
-  CUDA_TRY(c, cudaMemcpyAsync(w.r, w.r0, (size_t)N * V * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  CUDA_TRY(c, cudaMemsetAsync(w.p, 0, (size_t)N * V * sizeof(double), s));
-  CUDA_TRY(c, cudaMemsetAsync(w.q, 0, (size_t)N * V * sizeof(double), s));
-  CUDA_TRY(c, cudaMemsetAsync(w.v, 0, (size_t)N * V * sizeof(double), s));
-  CUDA_TRY(c, cudaMemsetAsync(w.z, 0, (size_t)N * V * sizeof(double), s));
+  // Jacobi-PCG of systems that fit: one launch with the matrix in shared
+  // memory (resident_plan), unless the caller asked for a graph form; with
+  // SOLV_OPT_PERSISTENT the systems that do not fit keep a cluster each
+  const bool jac_cg = solver == 0 && imat <= 0 && V == 1;
+  bool grid = jac_cg && n_iter > 0 && (c->persistent || (c->graph_loop == 2 && c->graph_iters > 0));
+  if (grid) {
+    if ((rc = resident_plan(c))) return rc;
+    grid = c->grid_shape >= 0;
+  }
+  if (!grid) {
+    CUDA_TRY(c, cudaMemcpyAsync(w.r, w.r0, (size_t)N * V * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    CUDA_TRY(c, cudaMemsetAsync(w.p, 0, (size_t)N * V * sizeof(double), s));
+    CUDA_TRY(c, cudaMemsetAsync(w.q, 0, (size_t)N * V * sizeof(double), s));
+    CUDA_TRY(c, cudaMemsetAsync(w.v, 0, (size_t)N * V * sizeof(double), s));
+    CUDA_TRY(c, cudaMemsetAsync(w.z, 0, (size_t)N * V * sizeof(double), s));
+  }
   {
     int na = nl;
     if (n_iter <= 0) na = 0;
@@ -1640,9 +1796,9 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
   sg::k_lane_init<<<(nl + 255) / 256, 256, 0, s>>>(c->lanes.as<Lane>(), nl, n_iter, reduc,
                                                    c->n_active.as<int>());
   SegMap sm = segmap(c);
-  const bool fused = c->persistent && solver == 0 && imat <= 0 && V == 1;
+  const bool fused = c->persistent && jac_cg && !grid;
   if (solver == 0) {
-    if (imat <= 0 && !fused) {
+    if (imat <= 0 && !fused && !grid) {
       sg::k_cg_rz<double, V, true><<<c->seg.total_blk, c->block, 0, s>>>(
           sm, w.c, w.r, w.z, c->part.as<double>(), c->lanes.as<Lane>());
       c->launches++;
@@ -1655,7 +1811,9 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
   c->launches += 2;
   CUDA_TRY(c, cudaGetLastError());
   int gl = 0;
-  if (fused) {  // the whole loop in one launch: one cluster per system
+  if (grid) {
+    if ((rc = resident_pcg(c, w.c, w.phi, w.r0)) || (rc = sweep_check(c))) return rc;
+  } else if (fused) {  // the whole loop in one launch: one cluster per system
     // systems of at most 16 x 2048 cells run with their vectors in the
     // cluster's registers and shared memory (k_pcg_cluster_res), larger
     // ones from global memory (k_pcg_cluster); 16 blocks per cluster where
