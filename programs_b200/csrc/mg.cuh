@@ -47,7 +47,6 @@ namespace mg {
 
 constexpr int kCoarsest = 256;   // dense inverse at or below this many cells
 constexpr int kMaxLevels = 12;   // coarse levels at most
-constexpr int kCoarseBlock = 256;
 
 // ---- host: graphs and aggregation ---------------------------------------------
 // Undirected graph in CSR with positive coupling strengths (|a_ij|).
@@ -379,10 +378,9 @@ __global__ void k_mg_dinv(int n, sg::Rows<float> R, float* __restrict__ dinv) {
   }
 }
 
-// Dense FP64 copy of the coarsest matrix (row-major n x n).
+// Dense FP64 copy of the coarsest matrix (row-major n x n, zeroed before).
 __global__ void k_mg_dense(int n, sg::Rows<float> R, double* __restrict__ A) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    for (int j = 0; j < n; ++j) A[(size_t)i * n + j] = 0.0;
     sg::RowIt<float> it(R, i);
     double d = R.diag[i];
     for (int k = 0; k < it.w; ++k) {
@@ -397,47 +395,81 @@ __global__ void k_mg_dense(int n, sg::Rows<float> R, double* __restrict__ A) {
   }
 }
 
-// In-place Gauss-Jordan inverse of the symmetric positive definite coarsest
-// matrix (no pivoting needed), one block; a pivot below 1e-13 of the largest
-// diagonal (a singular, all-Neumann system) drops that row and column,
-// which leaves a generalised inverse.  Result rounded to FP32.
-__global__ void __launch_bounds__(1024)
-k_mg_invert(int n, double* __restrict__ A, float* __restrict__ Ainv) {
-  __shared__ double f[kCoarsest];
-  __shared__ double dmax;
-  __shared__ bool skip;
-  const int t = threadIdx.x, nt = blockDim.x;
-  if (t == 0) {
+// Gauss-Jordan inverse of the symmetric positive definite coarsest matrix
+// (no pivoting needed); a pivot below 1e-13 of the largest diagonal (a
+// singular, all-Neumann system) drops that row and column, which leaves a
+// generalised inverse.  Result rounded to FP32.
+// The n steps are a serial chain, so what counts is the step: the matrix
+// stays in registers of CS blocks (one, or a cluster of 8 above 128 cells) --
+// a thread owns one column of kInvRows consecutive rows -- and a step is the
+// pivot row, shared by its owner, the pivot column, shared by each block for
+// its own rows, one barrier, and kInvRows updates.  Through global memory in
+// one block the step swept n^2 entries through L2 (252 us at n = 67, 3.77 ms
+// at n = 242, a tenth of a 160^3 solve).
+constexpr int kInvRows = 16;
+template <int COLS, int CS>
+__global__ void __launch_bounds__(CS == 1 ? 1024 : 512)
+k_mg_invert(int n, const double* __restrict__ A, float* __restrict__ Ainv) {
+  namespace cg = cooperative_groups;
+  constexpr int NT = CS == 1 ? 1024 : 512, GRP = NT / COLS;  // row groups in this block
+  static_assert(CS * GRP * kInvRows >= COLS, "every row has an owner");
+  __shared__ double row_s[2][COLS + 1];                // the pivot row and 1 / pivot, in its owner's block
+  __shared__ double col_s[2][GRP][kInvRows];           // the pivot column of this block's rows
+  __shared__ double dmax_s;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = CS == 1 ? 0 : (int)cl.block_rank();
+  const int j = threadIdx.x % COLS, g = threadIdx.x / COLS;
+  const int i0 = (rank * GRP + g) * kInvRows;  // this thread's rows i0 .. i0 + kInvRows
+  double a[kInvRows];
+#pragma unroll
+  for (int r = 0; r < kInvRows; ++r)
+    a[r] = i0 + r < n && j < n ? A[(size_t)(i0 + r) * n + j] : 0.0;
+  if (threadIdx.x < 32) {
     double m = 0.0;
-    for (int i = 0; i < n; ++i) m = fmax(m, fabs(A[(size_t)i * n + i]));
-    dmax = m;
+    for (int i = threadIdx.x; i < n; i += 32) m = fmax(m, fabs(A[(size_t)i * n + i]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) dmax_s = m;
   }
   __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    if (t == 0) skip = !(fabs(A[(size_t)k * n + k]) > 1e-13 * dmax);
-    __syncthreads();
-    if (skip) {
-      for (int j = t; j < n; j += nt) {
-        A[(size_t)k * n + j] = 0.0;
-        A[(size_t)j * n + k] = 0.0;
+  const double dmax = dmax_s;
+  for (int k0 = 0; k0 < n; k0 += kInvRows) {
+    const int owner = k0 / kInvRows / GRP;
+    const bool mine = i0 == k0;  // the pivot rows of this round are this group's
+#pragma unroll
+    for (int kk = 0; kk < kInvRows; ++kk) {
+      const int k = k0 + kk, par = kk & 1;  // buffers alternate: kInvRows is even
+      if (k < n) {
+        if (mine) row_s[par][j] = a[kk];
+        if (mine && j == k) row_s[par][COLS] = 1.0 / a[kk];
+        if (j == k) {
+#pragma unroll
+          for (int r = 0; r < kInvRows; ++r) col_s[par][g][r] = a[r];
+        }
+        if (CS == 1) __syncthreads();
+        else cl.sync();
+        const double* rs = CS == 1 ? row_s[par] : cl.map_shared_rank(&row_s[par][0], owner);
+        const double piv = rs[k], rj = rs[j], ip = rs[COLS];
+        if (!(fabs(piv) > 1e-13 * dmax)) {
+#pragma unroll
+          for (int r = 0; r < kInvRows; ++r)
+            if (j == k || i0 + r == k) a[r] = 0.0;
+        } else {
+          const double pr = j == k ? ip : rj * ip;
+#pragma unroll
+          for (int r = 0; r < kInvRows; ++r) {
+            const double f = col_s[par][g][r];
+            const double v = (j == k ? 0.0 : a[r]) - f * pr;
+            a[r] = i0 + r == k ? pr : v;
+          }
+        }
       }
-      __syncthreads();
-      continue;
     }
-    const double ip = 1.0 / A[(size_t)k * n + k];
-    __syncthreads();
-    for (int j = t; j < n; j += nt) A[(size_t)k * n + j] = (j == k) ? ip : A[(size_t)k * n + j] * ip;
-    for (int i = t; i < n; i += nt) f[i] = (i == k) ? 0.0 : A[(size_t)i * n + k];
-    __syncthreads();
-    for (int q = t; q < n * n; q += nt) {
-      const int i = q / n, j = q % n;
-      if (i == k) continue;
-      const double a = (j == k) ? 0.0 : A[q];
-      A[q] = a - f[i] * A[(size_t)k * n + j];
-    }
-    __syncthreads();
   }
-  for (int q = t; q < n * n; q += nt) Ainv[q] = (float)A[q];
+#pragma unroll
+  for (int r = 0; r < kInvRows; ++r)
+    if (i0 + r < n && j < n) Ainv[(size_t)(i0 + r) * n + j] = (float)a[r];
+  if (CS > 1) cl.sync();  // no block leaves while others may still read its pivot row
 }
 
 // ---- device: the V-cycle ---------------------------------------------------------
@@ -474,6 +506,186 @@ __global__ void k_mg_pre(int n, sg::Rows<float> R, const float* __restrict__ din
     }
     x[i] = xi;
     t[i] = bi - y;
+  }
+}
+
+// The coarse levels' rows hold 17-27 slots, and from the second level on
+// there are too few rows to fill the SMs with one thread each, so G lanes
+// share a row: lane = part * (32/G) + row, so a load still reads 32/G
+// consecutive words per slot.  Returns sum_j a_ij (x(j) - xi) in every lane.
+template <int G, typename X>
+__device__ __forceinline__ float row_diff(const sg::Rows<float>& R, int i, int part, float xi,
+                                          X&& x) {
+  constexpr int CH = 4;
+  sg::RowIt<float> it(R, i);
+  float y = 0.0f;
+  for (int k0 = part; k0 < it.w; k0 += CH * G) {
+    int j[CH];
+    float a[CH], xj[CH];
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      j[u] = -1;
+      a[u] = 0.0f;
+      if (k0 + u * G < it.w) {
+        const int e = it.base + (k0 + u * G) * sg::kWarp;
+        j[u] = __ldg(&R.col[e]);
+        a[u] = __ldg(&R.val[e]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < CH; ++u) xj[u] = j[u] >= 0 ? x(j[u]) : xi;
+#pragma unroll
+    for (int u = 0; u < CH; ++u)
+      if (j[u] >= 0) y = fmaf(a[u], xj[u] - xi, y);
+  }
+#pragma unroll
+  for (int o = 16; o >= 32 / G; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+  return y;
+}
+
+// Calls f(row, part, store) for every row of n, G lanes a row (whole warps at
+// a time; rows past n repeat the last one with store off).
+template <int G, typename F>
+__device__ __forceinline__ void rows_by_group(int n, int thread, int n_threads, F&& f) {
+  constexpr int RW = 32 / G;  // rows a warp
+  const int lane = thread & 31, part = lane / RW, rl = lane % RW;
+  for (int i0 = (thread >> 5) * RW; i0 < n; i0 += (n_threads >> 5) * RW)
+    f(min(i0 + rl, n - 1), part, part == 0 && i0 + rl < n);
+}
+
+// pre- and post-smoothing (k_mg_pre, k_mg_post) of a coarse level of at most
+// kCoarseCells rows, 4 lanes a row.
+constexpr int kCoarseLanes = 4;
+constexpr int kCoarseCells = 100000;
+__global__ void k_mg_pre_coarse(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
+                                const float* __restrict__ b, float* __restrict__ x,
+                                float* __restrict__ t, const int* __restrict__ n_active) {
+  if (n_active && *n_active == 0) return;
+  rows_by_group<kCoarseLanes>(
+      n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
+      [&](int i, int part, bool store) {
+        const float bi = b[i], xi = w * dinv[i] * bi;
+        const float y = R.diag[i] * xi + row_diff<kCoarseLanes>(R, i, part, xi, [&](int j) {
+                          return w * dinv[j] * b[j];
+                        });
+        if (store) {
+          x[i] = xi;
+          t[i] = bi - y;
+        }
+      });
+}
+__global__ void k_mg_post_coarse(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
+                                 const float* __restrict__ b, const float* __restrict__ x,
+                                 float* __restrict__ y, const int* __restrict__ n_active) {
+  if (n_active && *n_active == 0) return;
+  rows_by_group<kCoarseLanes>(
+      n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
+      [&](int i, int part, bool store) {
+        const float xi = x[i];
+        const float ax = R.diag[i] * xi +
+                         row_diff<kCoarseLanes>(R, i, part, xi, [&](int j) { return x[j]; });
+        if (store) y[i] = xi + w * dinv[i] * (b[i] - ax);
+      });
+}
+
+// The V-cycle's bottom in one launch: from the finer level's residual t to
+// the correction y of level 0 here (the first of at most kFuseCells cells),
+// one thread-block cluster over all the levels below.  As a kernel per step
+// these levels are four dependent launches each on a few hundred to a few
+// thousand rows, 5-12 us apiece; here a step ends with a cluster barrier
+// (0.4-0.7 us with its stores).  More lanes share a row the fewer rows there
+// are.  The vectors pass between the blocks through L2 (loads that skip L1).
+// A whole V-cycle, before / after, us: 32^3 67 / 53, 64^3 99 / 86, 100^3
+// 182 / 153, 160^3 413 / 386, 200^3 666 / 634; with levels of up to 16k cells
+// in here, more than 16 SMs are good for, 160^3 took 420.
+struct FuseLevel {
+  int n;
+  sg::Rows<float> R;
+  const float* dinv;
+  const int *agg_ptr, *agg_cells, *agg_of;  // members on the finer level; finer cell -> cell
+  float *x, *b, *t, *y;
+};
+struct FuseArgs {
+  int n_level;
+  FuseLevel lv[kMaxLevels];
+  const float* t_fine;  // residual of the level above lv[0]
+  const float* ainv;    // dense inverse of the last level
+};
+constexpr int kFuseCells = 6000;
+constexpr int kFuseThreads = 1024;
+constexpr int kFuseCluster = 16;
+
+template <int G>
+__device__ __forceinline__ void fuse_pre(const FuseLevel& L, float w, int t, int nt) {
+  rows_by_group<G>(L.n, t, nt, [&](int i, int part, bool store) {
+    const float bi = __ldcg(&L.b[i]), xi = w * __ldg(&L.dinv[i]) * bi;
+    const float y = __ldg(&L.R.diag[i]) * xi + row_diff<G>(L.R, i, part, xi, [&](int j) {
+                      return w * __ldg(&L.dinv[j]) * __ldcg(&L.b[j]);
+                    });
+    if (store) {
+      __stcg(&L.x[i], xi);
+      __stcg(&L.t[i], bi - y);
+    }
+  });
+}
+template <int G>
+__device__ __forceinline__ void fuse_post(const FuseLevel& L, float w, int t, int nt) {
+  rows_by_group<G>(L.n, t, nt, [&](int i, int part, bool store) {
+    const float xi = __ldcg(&L.x[i]);
+    const float ax = __ldg(&L.R.diag[i]) * xi +
+                     row_diff<G>(L.R, i, part, xi, [&](int j) { return __ldcg(&L.x[j]); });
+    if (store) __stcg(&L.y[i], xi + w * __ldg(&L.dinv[i]) * (__ldcg(&L.b[i]) - ax));
+  });
+}
+
+__global__ void __launch_bounds__(kFuseThreads) k_mg_bottom(FuseArgs A, float w, float alpha,
+                                                            const int* __restrict__ n_active) {
+  if (n_active && *n_active == 0) return;  // the same for every block
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ float sb[kCoarsest];
+  const int nt = (int)cl.num_blocks() * kFuseThreads;
+  const int t = (int)cl.block_rank() * kFuseThreads + threadIdx.x;
+  const int last = A.n_level - 1;
+  for (int l = 0; l <= last; ++l) {
+    const FuseLevel& L = A.lv[l];
+    const float* tf = l == 0 ? A.t_fine : A.lv[l - 1].t;
+    for (int I = t; I < L.n; I += nt) {  // restriction, members in list order
+      float s = 0.0f;
+      for (int m = __ldg(&L.agg_ptr[I]); m < __ldg(&L.agg_ptr[I + 1]); ++m)
+        s += __ldcg(&tf[__ldg(&L.agg_cells[m])]);
+      __stcg(&L.b[I], s);
+    }
+    cl.sync();
+    if (l == last) break;
+    if (L.n * 2 > nt) fuse_pre<2>(L, w, t, nt);
+    else if (L.n * 8 > nt) fuse_pre<8>(L, w, t, nt);
+    else fuse_pre<16>(L, w, t, nt);
+    cl.sync();
+  }
+  {  // x = Ainv b, a warp a row
+    const FuseLevel& L = A.lv[last];
+    for (int i = threadIdx.x; i < L.n; i += kFuseThreads) sb[i] = __ldcg(&L.b[i]);
+    __syncthreads();
+    for (int i = t >> 5; i < L.n; i += nt >> 5) {
+      float s = 0.0f;
+      for (int j = threadIdx.x & 31; j < L.n; j += 32)
+        s = fmaf(__ldg(&A.ainv[(size_t)i * L.n + j]), sb[j], s);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((threadIdx.x & 31) == 0) __stcg(&L.y[i], s);
+    }
+  }
+  for (int l = last - 1; l >= 0; --l) {
+    const FuseLevel& L = A.lv[l];
+    const FuseLevel& C = A.lv[l + 1];
+    cl.sync();
+    for (int i = t; i < L.n; i += nt)
+      __stcg(&L.x[i], __ldcg(&L.x[i]) + alpha * __ldcg(&C.y[__ldg(&C.agg_of[i])]));
+    cl.sync();
+    if (L.n * 2 > nt) fuse_post<2>(L, w, t, nt);
+    else if (L.n * 8 > nt) fuse_post<8>(L, w, t, nt);
+    else fuse_post<16>(L, w, t, nt);
   }
 }
 
@@ -613,21 +825,6 @@ __global__ void k_mg_prolong(int n, const int* __restrict__ agg_of, float a,
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     x[i] += a * xc[agg_of[i]];
-}
-
-// x = Ainv b on the coarsest level (one block)
-__global__ void __launch_bounds__(kCoarseBlock)
-k_mg_coarse_solve(int n, const float* __restrict__ Ainv, const float* __restrict__ b,
-                  float* __restrict__ x, const int* __restrict__ n_active) {
-  if (n_active && *n_active == 0) return;
-  __shared__ float sb[kCoarsest];
-  for (int j = threadIdx.x; j < n; j += blockDim.x) sb[j] = b[j];
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    float s = 0.0f;
-    for (int j = 0; j < n; ++j) s = fmaf(Ainv[(size_t)i * n + j], sb[j], s);
-    x[i] = s;
-  }
 }
 
 // ---- device: training the network through the V-cycle ----------------------------

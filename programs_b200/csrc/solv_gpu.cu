@@ -175,6 +175,7 @@ struct solv_gpu_ctx {
   DevBuf mg_train;                     // training through the V-cycle: 8 vectors
   DevBuf mg_dq;                        // smoother 2: the network's per-cell weights q^2
   DevBuf g_zero;                       // smoother 2 training: face weights held at zero
+  int mg_bottom_cs = 0;                // blocks in k_mg_bottom's cluster
   double mg_setup_s = 0.0;
   double mg_smooth_scale = 1.0;        // factor the last solve applied to K (see mg_bound_smoother)
   float mg_scale_min = 0.5f;           // floor on the network's per-cell scales
@@ -957,6 +958,24 @@ int mg_setup(solv_gpu_ctx* c) {
   return SOLV_GPU_OK;
 }
 
+// One thread-block cluster of cs blocks.
+template <typename... KArgs, typename... Args>
+int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), int cs, int threads, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cs);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, args...));
+  return SOLV_GPU_OK;
+}
+
 // Coefficients of every coarse level for the current values (each solve):
 // Galerkin sums level by level, inverse diagonals, the coarsest inverse.
 int mg_values(solv_gpu_ctx* c) {
@@ -977,53 +996,102 @@ int mg_values(solv_gpu_ctx* c) {
     rsprev = L->rs.as<float>();
   }
   MgLevel& C = *c->mg.back();
-  mg::k_mg_dense<<<grid_for(c, C.n), B, 0, s>>>(C.n, C.rows(), c->mg_dense.as<double>());
-  mg::k_mg_invert<<<1, 1024, 0, s>>>(C.n, c->mg_dense.as<double>(), c->mg_ainv.as<float>());
+  CUDA_TRY(c, cudaMemsetAsync(c->mg_dense.p, 0, (size_t)C.n * C.n * sizeof(double), s));
+  mg::k_mg_dense<<<(C.n + 31) / 32, 32, 0, s>>>(C.n, C.rows(), c->mg_dense.as<double>());
+  if (C.n <= 128)
+    mg::k_mg_invert<128, 1><<<1, 1024, 0, s>>>(C.n, c->mg_dense.as<double>(), c->mg_ainv.as<float>());
+  else if ((rc = cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, 8, 512, C.n,
+                                (const double*)c->mg_dense.as<double>(), c->mg_ainv.as<float>())))
+    return rc;
   c->launches += 2 + 3 * (int)c->mg.size() + 2;
   CUDA_TRY(c, cudaGetLastError());
   return SOLV_GPU_OK;
 }
 
-// The V-cycle below level 0: level 1's right-hand side mg[0]->b in, its
-// correction mg[0]->y out.  Returns the number of kernels launched.
-int mg_coarse_cycle(solv_gpu_ctx* c, const int* na) {
+// The first level the V-cycle's bottom kernel takes (k_mg_bottom): the levels
+// of at most kFuseCells cells, the last one always.
+int mg_fuse_from(const solv_gpu_ctx* c) {
+  int l = 0;
+  while (l + 1 < (int)c->mg.size() && c->mg[l]->n > mg::kFuseCells) ++l;
+  return l;
+}
+
+// Blocks in the bottom kernel's cluster: 16 where the GPU holds such a
+// cluster, else the portable 8.
+int mg_bottom_blocks(solv_gpu_ctx* c) {
+  if (c->mg_bottom_cs) return c->mg_bottom_cs;
+  int n16 = 0;
+  if (cudaFuncSetAttribute(mg::k_mg_bottom, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+      cudaSuccess) {
+    cudaLaunchConfig_t qc = {};
+    qc.gridDim = dim3(mg::kFuseCluster);
+    qc.blockDim = dim3(mg::kFuseThreads);
+    cudaLaunchAttribute qa[1];
+    qa[0].id = cudaLaunchAttributeClusterDimension;
+    qa[0].val.clusterDim.x = mg::kFuseCluster;
+    qa[0].val.clusterDim.y = 1;
+    qa[0].val.clusterDim.z = 1;
+    qc.attrs = qa;
+    qc.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n16, mg::k_mg_bottom, &qc) != cudaSuccess) n16 = 0;
+  }
+  cudaGetLastError();  // a refused query leaves the portable size
+  c->mg_bottom_cs = n16 > 0 ? mg::kFuseCluster : 8;
+  return c->mg_bottom_cs;
+}
+
+// The V-cycle below level 0: level 0's residual t0 in, level 1's correction
+// mg[0]->y out.  Returns the number of kernels launched.
+int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na) {
   cudaStream_t s = c->stream;
   const int B = c->block;
   const float w = (float)c->mg_omega, a = (float)c->mg_alpha;
-  const int L = (int)c->mg.size();
-  int k = 0;
-  for (int l = 0; l + 1 < L; ++l) {
+  const int L = (int)c->mg.size(), lf = mg_fuse_from(c);
+  const float* t = t0;
+  for (int l = 0; l < lf; ++l) {
     MgLevel& F = *c->mg[l];
-    MgLevel& C = *c->mg[l + 1];
-    with_chunk(c->row_chunk, [&](auto ch) {
-      mg::k_mg_pre<decltype(ch)::value><<<grid_for(c, F.n), B, 0, s>>>(
+    mg::k_mg_restrict<<<grid_for(c, F.n), B, 0, s>>>(F.n, F.agg_ptr.as<int>(),
+                                                     F.agg_cells.as<int>(), t, F.b.as<float>(), na);
+    if (F.n <= mg::kCoarseCells)
+      mg::k_mg_pre_coarse<<<grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
           F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.t.as<float>(),
           na);
-    });
-    mg::k_mg_restrict<<<grid_for(c, C.n), B, 0, s>>>(C.n, C.agg_ptr.as<int>(),
-                                                     C.agg_cells.as<int>(), F.t.as<float>(),
-                                                     C.b.as<float>(), na);
-    k += 2;
+    else
+      with_chunk(c->row_chunk, [&](auto ch) {
+        mg::k_mg_pre<decltype(ch)::value><<<grid_for(c, F.n), B, 0, s>>>(
+            F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(),
+            F.t.as<float>(), na);
+      });
+    t = F.t.as<float>();
   }
-  {
-    MgLevel& C = *c->mg[L - 1];
-    mg::k_mg_coarse_solve<<<1, mg::kCoarseBlock, 0, s>>>(C.n, c->mg_ainv.as<float>(),
-                                                         C.b.as<float>(), C.y.as<float>(), na);
-    k += 1;
+  mg::FuseArgs A = {};
+  A.n_level = L - lf;
+  A.t_fine = t;
+  A.ainv = c->mg_ainv.as<float>();
+  for (int l = lf; l < L; ++l) {
+    MgLevel& F = *c->mg[l];
+    A.lv[l - lf] = {F.n, F.rows(), F.dinv.as<float>(), F.agg_ptr.as<int>(), F.agg_cells.as<int>(),
+                    F.agg_of.as<int>(), F.x.as<float>(), F.b.as<float>(), F.t.as<float>(),
+                    F.y.as<float>()};
   }
-  for (int l = L - 2; l >= 0; --l) {
+  cluster_launch(c, mg::k_mg_bottom, mg_bottom_blocks(c), mg::kFuseThreads, A, w, a, na);
+  for (int l = lf - 1; l >= 0; --l) {
     MgLevel& F = *c->mg[l];
     MgLevel& C = *c->mg[l + 1];
     mg::k_mg_prolong<<<grid_for(c, F.n), B, 0, s>>>(F.n, C.agg_of.as<int>(), a, C.y.as<float>(),
                                                     F.x.as<float>(), na);
-    with_chunk(c->row_chunk, [&](auto ch) {
-      mg::k_mg_post<float, decltype(ch)::value><<<grid_for(c, F.n), B, 0, s>>>(
+    if (F.n <= mg::kCoarseCells)
+      mg::k_mg_post_coarse<<<grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
           F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.y.as<float>(),
           na);
-    });
-    k += 2;
+    else
+      with_chunk(c->row_chunk, [&](auto ch) {
+        mg::k_mg_post<float, decltype(ch)::value><<<grid_for(c, F.n), B, 0, s>>>(
+            F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(),
+            F.y.as<float>(), na);
+      });
   }
-  return k;
+  return 4 * lf + 1;
 }
 
 // z = one symmetric V-cycle applied to r (FP32, level 0 = the context's
@@ -1058,10 +1126,7 @@ int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, 
     });
     k += 1;
   }
-  mg::k_mg_restrict<<<grid_for(c, L1.n), B, 0, s>>>(L1.n, L1.agg_ptr.as<int>(),
-                                                    L1.agg_cells.as<int>(), t0, L1.b.as<float>(),
-                                                    na);
-  k += 1 + mg_coarse_cycle(c, na);
+  k += mg_coarse_cycle(c, t0, na);
   mg::k_mg_prolong<<<grid_resident(c, N), B, 0, s>>>(N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0,
                                                 na);
   k += 1;
@@ -1144,9 +1209,8 @@ int mg_bound_smoother(solv_gpu_ctx* c, double* applied) {
 
 // Kernels in one V-cycle (launch statistics of graph replays).
 int mg_kernels(const solv_gpu_ctx* c) {
-  const int L = (int)c->mg.size();
   const int fine = c->mg_smoother == 1 ? 5 : 3;  // smoothing, residual, prolongation
-  return fine + 1 + 2 * (L - 1) + 1 + 2 * (L - 1);
+  return fine + 4 * mg_fuse_from(c) + 1;
 }
 
 // ---- building blocks -----------------------------------------------------------
@@ -3429,10 +3493,7 @@ static int mg_train_sample(solv_gpu_ctx* c, float** B) {
   mg::k_mg_net<false, float><<<G, Bk, 0, s>>>(N, R0, ge, q, w, gz, nullptr, tmp, nullptr);
   mg::k_mg_resid<<<G, Bk, 0, s>>>(N, R0, gz, tmp, gx, nullptr);
   // through the coarse correction x += a P C P^T (b - A x): gx -= A (a P C P^T gx)
-  mg::k_mg_restrict<<<grid_for(c, L1.n), Bk, 0, s>>>(L1.n, L1.agg_ptr.as<int>(),
-                                                     L1.agg_cells.as<int>(), gx, L1.b.as<float>(),
-                                                     nullptr);
-  mg_coarse_cycle(c, nullptr);
+  mg_coarse_cycle(c, gx, nullptr);
   CUDA_TRY(c, cudaMemsetAsync(tmp, 0, (size_t)N * sizeof(float), s));
   mg::k_mg_prolong<<<G, Bk, 0, s>>>(N, L1.agg_of.as<int>(), a, L1.y.as<float>(), tmp, nullptr);
   mg::k_mg_resid<<<G, Bk, 0, s>>>(N, R0, gx, tmp, az, nullptr);  // az = adjoint at x = w K b
