@@ -19,6 +19,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+#include <type_traits>
+
 namespace sg {
 
 constexpr double kSmall = 1e-20;  // spray-simulation/precision.f90:8
@@ -529,6 +532,37 @@ __device__ __forceinline__ void ld_relaxed_if(bool on, const unsigned int* p, un
       : "+r"(bits) : "l"(p), "r"((unsigned)on) : "memory");
 }
 
+// Where a recurrence's values are: global memory (relaxed, at the GPU's
+// scope) or this block's shared memory (one system a block, cells from base).
+template <typename T>
+struct GlobalVals {
+  using U = typename Pending<T>::U;
+  const U* p;
+  __device__ __forceinline__ void get(bool on, int j, int V, int v, U& bits) const {
+    ld_relaxed_if(on, &p[(size_t)j * V + v], bits);
+  }
+  __device__ __forceinline__ U peek(int j, int V) const { return ld_relaxed(&p[(size_t)j * V]); }
+};
+struct SharedVals {
+  using U = unsigned long long;
+  unsigned at;  // shared-memory address of cell base's first value
+  int base;
+  __device__ __forceinline__ void get(bool on, int j, int V, int v, U& bits) const {
+    asm volatile(
+        "{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.relaxed.cta.shared.b64 %0, [%1]; }"
+        : "+l"(bits) : "r"(at + (unsigned)((j - base) * V + v) * 8u), "r"((unsigned)on) : "memory");
+  }
+  __device__ __forceinline__ U peek(int j, int V) const {
+    U bits = 0;
+    get(true, j, V, 0, bits);
+    return bits;
+  }
+  __device__ __forceinline__ void put(int j, int V, int v, double x) const {
+    asm volatile("st.relaxed.cta.shared.b64 [%0], %1;" ::"r"(at + (unsigned)((j - base) * V + v) * 8u),
+                 "l"(__double_as_longlong(x)) : "memory");
+  }
+};
+
 // x[0 .. n) = pending
 template <typename T>
 __global__ void k_fill_pending(long long n, T* __restrict__ x) {
@@ -546,8 +580,9 @@ __global__ void k_fill_pending(long long n, T* __restrict__ x) {
 // runs over them alone (0.93 -> 0.74 us a level); in an order of a few
 // levels, where bandwidth counts, the packing would only delay the
 // coefficients.
-// Once the values are all there they are folded in in slot order (`use`),
-// the sequential loop's arithmetic; `finish` stores the cell.  A lane stores
+// Once the values are all there, the products (`term`, side by side) are
+// folded in in slot order (`fold`), the sequential loop's arithmetic;
+// `finish` stores the cell.  A lane stores
 // as soon as its own inputs are there, because a slice that spans two levels
 // holds cells that wait for cells of the same slice.
 //
@@ -581,16 +616,151 @@ __device__ __forceinline__ bool sweep_dep(int j, int i) {
   return j >= 0 && (UP ? j > i : j < i);
 }
 
-template <bool UP, bool GATE, int C, int V, typename A, typename T, typename Start, typename Coef,
-          typename Use, typename Finish>
-__device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const SweepMap& sm,
-                                           const T* vals, SweepCtl* ctl, Start&& start,
-                                           Coef&& coef, Use&& use, Finish&& finish) {
+// One slice of a recurrence over the cells c0 .. c1 (n: those of the matrix).
+template <bool UP, bool GATE, int C, int V, typename A, typename T, typename Vals, typename Start,
+          typename Coef, typename Term, typename Fold, typename Finish>
+__device__ __forceinline__ void sweep_slice(int n, const Rows<T>& R, int s, int c0, int c1,
+                                            const Vals& vals, SweepCtl* ctl, Start&& start,
+                                            Coef&& coef, Term&& term, Fold&& fold,
+                                            Finish&& finish) {
   using P = Pending<T>;
   using U = typename P::U;
   constexpr unsigned full = 0xffffffffu;
-  const U* bits_of = reinterpret_cast<const U*>(vals);
   const int lane = threadIdx.x & 31;
+  const int i = s * 32 + lane;
+  const int w = __ldg(&R.slice_w[s]);
+  const int base = __ldg(&R.slice_ptr[s]) + lane;
+  int dj[C];  // the chunk's dependencies in slot order: the first nd (GATE), or
+  A a[C];     // those of the slots in mask
+  U bits[C][V];
+  int nd = 0, k0 = 0;
+  unsigned mask = 0;
+  bool done = i < c0 || i >= c1;
+  auto on = [&](int q) { return GATE ? q < nd : ((mask >> q) & 1u) != 0; };
+  auto load = [&]() {
+    int j[C], du[C];
+#pragma unroll
+    for (int u = 0; u < C; ++u) {
+      j[u] = -1;
+      if (k0 + u < w) j[u] = __ldg(&R.col[base + (k0 + u) * kWarp]);
+    }
+    if constexpr (GATE) {
+      nd = 0;
+#pragma unroll
+      for (int u = 0; u < C; ++u) {
+        dj[u] = du[u] = 0;
+        const bool dep = sweep_dep<UP>(j[u], i);
+#pragma unroll
+        for (int q = 0; q <= u; ++q)
+          if (dep && nd == q) {
+            dj[q] = j[u];
+            du[q] = u;
+          }
+        nd += dep;
+      }
+    } else {
+      mask = 0;
+#pragma unroll
+      for (int u = 0; u < C; ++u) {
+        dj[u] = j[u];
+        du[u] = u;
+        if (sweep_dep<UP>(j[u], i)) mask |= 1u << u;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < C; ++q) {
+      if (on(q)) a[q] = coef(base + (k0 + du[q]) * kWarp);
+#pragma unroll
+      for (int v = 0; v < V; ++v) bits[q][v] = 0;
+    }
+  };
+  if (!done) {
+    start(i);
+    load();
+  }
+  if constexpr (GATE) {
+    // the last cell of an earlier slice that this chunk depends on, then
+    // the last dependency of that cell (indices offset so that 0 is none;
+    // backward, counted from the top)
+    unsigned last = 0;
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+      if (q < nd && (UP ? (dj[q] >> 5) > s : (dj[q] >> 5) < s))
+        last = max(last, (unsigned)(UP ? n - dj[q] : dj[q] + 1));
+    last = __reduce_max_sync(full, last);
+    if (last) {
+      const int jl = UP ? n - (int)last : (int)last - 1;
+      const int wl = __ldg(&R.slice_w[jl >> 5]);
+      const int bl = __ldg(&R.slice_ptr[jl >> 5]) + (jl & 31);
+      const int c = lane < wl ? __ldg(&R.col[bl + lane * kWarp]) : -1;
+      unsigned far = sweep_dep<UP>(c, jl) ? (unsigned)(UP ? n - c : c + 1) : 0u;
+      far = __reduce_max_sync(full, far);
+      if (far) {
+        const int g = UP ? n - (int)far : (int)far - 1;
+        for (int poll = 0; vals.peek(g, V) == P::bits; ++poll) {
+          if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
+            if (lane == 0) atomicExch(&ctl->err, 1);
+            break;
+          }
+          __nanosleep(kGateSleep);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  for (int poll = 0;; ++poll) {
+    if (!done) {
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) vals.get(on(q), dj[q], V, v, bits[q][v]);
+      }
+      bool ready = true;
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) ready &= bits[q][v] != P::bits;
+      }
+      if (ready) {
+        T m[C][V];
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            T xv[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) xv[v] = P::from(bits[q][v]);
+          term(a[q], xv, m[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            if (GATE && q >= nd) break;
+          if (on(q)) fold(m[q]);
+        }
+        k0 += C;
+        if (k0 < w) {
+          load();
+        } else {
+          finish(i);
+          done = true;
+        }
+      }
+    }
+    if (__all_sync(full, done)) break;
+    if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
+      if (lane == 0) atomicExch(&ctl->err, 1);
+      break;
+    }
+    if (poll >= kSweepSpin) __nanosleep(kSweepSleep);
+  }
+}
+
+// The slices of all the systems, a block's warps taking turns.
+template <bool UP, bool GATE, int C, int V, typename A, typename T, typename Start, typename Coef,
+          typename Term, typename Fold, typename Finish>
+__device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const SweepMap& sm,
+                                           const T* values, SweepCtl* ctl, Start&& start,
+                                           Coef&& coef, Term&& term, Fold&& fold,
+                                           Finish&& finish) {
+  const GlobalVals<T> vals{reinterpret_cast<const typename Pending<T>::U*>(values)};
   // this block's systems (sys, sys + step, ...), its rank among theirs
   int sys = 0, step = 1, rank = blockIdx.x, nblk = gridDim.x;
   const bool by_sys = GATE && sm.n_sys > 1;
@@ -626,125 +796,7 @@ __device__ __forceinline__ void sweep_rows(int n, const Rows<T>& R, const SweepM
       continue;
     }
     const int s = s_lo + (UP ? ns - 1 - r : r);
-    const int i = s * 32 + lane;
-    const int w = __ldg(&R.slice_w[s]);
-    const int base = __ldg(&R.slice_ptr[s]) + lane;
-    int dj[C];  // the chunk's dependencies in slot order: the first nd (GATE), or
-    A a[C];     // those of the slots in mask
-    U bits[C][V];
-    int nd = 0, k0 = 0;
-    unsigned mask = 0;
-    bool done = i < c0 || i >= c1;
-    auto on = [&](int q) { return GATE ? q < nd : ((mask >> q) & 1u) != 0; };
-    auto load = [&]() {
-      int j[C], du[C];
-#pragma unroll
-      for (int u = 0; u < C; ++u) {
-        j[u] = -1;
-        if (k0 + u < w) j[u] = __ldg(&R.col[base + (k0 + u) * kWarp]);
-      }
-      if constexpr (GATE) {
-        nd = 0;
-#pragma unroll
-        for (int u = 0; u < C; ++u) {
-          dj[u] = du[u] = 0;
-          const bool dep = sweep_dep<UP>(j[u], i);
-#pragma unroll
-          for (int q = 0; q <= u; ++q)
-            if (dep && nd == q) {
-              dj[q] = j[u];
-              du[q] = u;
-            }
-          nd += dep;
-        }
-      } else {
-        mask = 0;
-#pragma unroll
-        for (int u = 0; u < C; ++u) {
-          dj[u] = j[u];
-          du[u] = u;
-          if (sweep_dep<UP>(j[u], i)) mask |= 1u << u;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < C; ++q) {
-        if (on(q)) a[q] = coef(base + (k0 + du[q]) * kWarp);
-#pragma unroll
-        for (int v = 0; v < V; ++v) bits[q][v] = 0;
-      }
-    };
-    if (!done) {
-      start(i);
-      load();
-    }
-    if constexpr (GATE) {
-      // the last cell of an earlier slice that this chunk depends on, then
-      // the last dependency of that cell (indices offset so that 0 is none;
-      // backward, counted from the top)
-      unsigned last = 0;
-#pragma unroll
-      for (int q = 0; q < C; ++q)
-        if (q < nd && (UP ? (dj[q] >> 5) > s : (dj[q] >> 5) < s))
-          last = max(last, (unsigned)(UP ? n - dj[q] : dj[q] + 1));
-      last = __reduce_max_sync(full, last);
-      if (last) {
-        const int jl = UP ? n - (int)last : (int)last - 1;
-        const int wl = __ldg(&R.slice_w[jl >> 5]);
-        const int bl = __ldg(&R.slice_ptr[jl >> 5]) + (jl & 31);
-        const int c = lane < wl ? __ldg(&R.col[bl + lane * kWarp]) : -1;
-        unsigned far = sweep_dep<UP>(c, jl) ? (unsigned)(UP ? n - c : c + 1) : 0u;
-        far = __reduce_max_sync(full, far);
-        if (far) {
-          const U* g = &bits_of[(size_t)(UP ? n - (int)far : (int)far - 1) * V];
-          for (int poll = 0; ld_relaxed(g) == P::bits; ++poll) {
-            if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
-              if (lane == 0) atomicExch(&ctl->err, 1);
-              break;
-            }
-            __nanosleep(kGateSleep);
-          }
-          __syncwarp();
-        }
-      }
-    }
-    for (int poll = 0;; ++poll) {
-      if (!done) {
-#pragma unroll
-        for (int q = 0; q < C; ++q)
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-            ld_relaxed_if(on(q), &bits_of[(size_t)dj[q] * V + v], bits[q][v]);
-        bool ready = true;
-#pragma unroll
-        for (int q = 0; q < C; ++q)
-#pragma unroll
-          for (int v = 0; v < V; ++v) ready &= bits[q][v] != P::bits;
-        if (ready) {
-#pragma unroll
-          for (int q = 0; q < C; ++q) {
-            if (GATE && q >= nd) break;
-            if (!GATE && !on(q)) continue;
-            T xv[V];
-#pragma unroll
-            for (int v = 0; v < V; ++v) xv[v] = P::from(bits[q][v]);
-            use(a[q], xv);
-          }
-          k0 += C;
-          if (k0 < w) {
-            load();
-          } else {
-            finish(i);
-            done = true;
-          }
-        }
-      }
-      if (__all_sync(full, done)) break;
-      if (poll >= kSweepPolls || ((poll & 63) == 63 && ld_err(ctl))) {
-        if (lane == 0) atomicExch(&ctl->err, 1);
-        break;
-      }
-      if (poll >= kSweepSpin) __nanosleep(kSweepSleep);
-    }
+    sweep_slice<UP, GATE, C, V, A>(n, R, s, c0, c1, vals, ctl, start, coef, term, fold, finish);
   }
 }
 
@@ -765,12 +817,10 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_precond_sf(
         return make_double2(IMAT == 2 ? __ldg(&fp[__ldg(&slot_src[e]) >> 1]) : 0.0,
                             __ldg(&R.sval[e]));
       },
-      [&](const double2& a, const double (&cj)[1]) {
-        if (IMAT == 1)
-          d = sub(d, mul(mul(a.y, a.y), cj[0]));
-        else
-          d = sub(d, mul(mul(a.x, cj[0]), a.y));
+      [&](const double2& a, const double (&cj)[1], double (&m)[1]) {
+        m[0] = IMAT == 1 ? mul(mul(a.y, a.y), cj[0]) : mul(mul(a.x, cj[0]), a.y);
       },
+      [&](const double (&m)[1]) { d = sub(d, m[0]); },
       [&](int i) {
         c_r[i] = d;
         st_relaxed(&c[i], 1.0 / add(d, kSmall));
@@ -814,9 +864,13 @@ __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_
         for (int v = 0; v < V; ++v) acc[v] = bvec[(size_t)i * V + v];
       },
       [&](int e) { return __ldg(&R.sval[e]); },
-      [&](const T a, const T (&xv)[V]) {
+      [&](const T a, const T (&xv)[V], T (&m)[V]) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], mul(a, xv[v]));
+        for (int v = 0; v < V; ++v) m[v] = mul(a, xv[v]);
+      },
+      [&](const T (&m)[V]) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], m[v]);
       },
       [&](int i) {
 #pragma unroll
@@ -845,9 +899,13 @@ __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_
         for (int v = 0; v < V; ++v) acc[v] = mul(t[(size_t)i * V + v], cr);
       },
       [&](int e) { return __ldg(&R.sval[e]); },
-      [&](const T a, const T (&xv)[V]) {
+      [&](const T a, const T (&xv)[V], T (&m)[V]) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], mul(a, xv[v]));
+        for (int v = 0; v < V; ++v) m[v] = mul(a, xv[v]);
+      },
+      [&](const T (&m)[V]) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], m[v]);
       },
       [&](int i) {
 #pragma unroll
@@ -1721,6 +1779,472 @@ __global__ void __launch_bounds__(B, 1) k_pcg_grid(
   }
 }
 
+// ============ small systems: the whole call in one launch, a block per system ============
+// solv_res, solv_precond and the loop of solv_cg.f90:26-84 (SOLVER 0) or
+// solv_bicg.f90:27-118 (SOLVER 1), FP64, with the layout conversions, for
+// systems whose gathered vectors fit one block's shared memory.  A call on a
+// few hundred or thousand cells spent its time in 20 launches before the loop,
+// 5-9 per iteration (1.5-3 us each, and the graph's remaining iterations as
+// early exits) and the host's round trips; here it is one launch.  What
+// neighbours read (p, or z, and the sweeps' t) is in shared memory, so a step
+// of a DIC/DILU recurrence is a store and a poll on the SM (SharedVals; 0.74
+// us through L2); a cell's own values stay in global memory (L1, L2), its
+// thread the only one to touch them.  Per-cell arithmetic and the order of
+// the updates are the step kernels'; the sums run in this block's fixed tree.
+// A system's slices go to the warps in turn: cell i always to warp
+// (i / 32 - first slice) % warps.
+struct SmallArgs {
+  Rows<double> R;
+  const int *seg_c0, *seg_c1, *old_of_new, *slot_src;
+  const double* fp;
+  double *phi_dev, *res_dev;                       // caller layouts
+  double *phi, *r, *r0, *p, *q, *v, *c, *cr;       // internal order
+  Lane* lanes;
+  double* l1;
+  SweepCtl* ctl;
+  int N, not_r0, imat, n_iter;
+  double reduc;
+};
+constexpr int kSmallThreads = 512;
+enum : int { kSmallResidual = 1, kSmallLoop = 2 };  // the parts of a launch
+
+// gathered vectors in shared memory: t and z of the sweeps, p of CG
+template <int SOLVER, bool SW>
+constexpr int kSmallVectors = (SW ? 2 : 0) + (SOLVER == 0 || !SW ? 1 : 0);
+
+// z = M^-1 b: the two sweeps of solv_direct.f90 over the cells c0 .. c1, one
+// block (ends with a barrier).  Not inlined: BiCGSTAB's two calls would
+// otherwise spill each other's addresses around every wait.
+template <int V>
+__device__ __noinline__ void small_direct(const SmallArgs& A, int c0, int c1, const double* b,
+                                          double* t_s, double* z_s) {
+  constexpr int NW = kSmallThreads / 32, C = V <= 2 ? 8 : 6;
+  const Rows<double>& R = A.R;
+  const int s_lo = c0 >> 5, ns = ((c1 + 31) >> 5) - s_lo, first = s_lo * 32;
+  const int wid = threadIdx.x >> 5;
+  const SharedVals tv{(unsigned)__cvta_generic_to_shared(t_s), first};
+  const SharedVals zv{(unsigned)__cvta_generic_to_shared(z_s), first};
+  double acc[V], ci = 0.0;
+  auto coef = [&](int e) { return __ldg(&R.sval[e]); };
+  auto term = [](const double a, const double (&xv)[V], double (&m)[V]) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) m[v] = mul(a, xv[v]);
+  };
+  auto fold = [&](const double (&m)[V]) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = sub(acc[v], m[v]);
+  };
+  for (int r = wid; r < ns; r += NW)
+    sweep_slice<false, true, C, V, double>(
+        A.N, R, s_lo + r, c0, c1, tv, A.ctl,
+        [&](int i) {
+          ci = A.c[i];
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[v] = b[(size_t)i * V + v];
+        },
+        coef, term, fold,
+        [&](int i) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            tv.put(i, V, v, mul(acc[v], ci));
+            zv.put(i, V, v, Pending<double>::value());
+          }
+        });
+  __syncthreads();
+  for (int r = wid; r < ns; r += NW)
+    sweep_slice<true, true, C, V, double>(
+        A.N, R, s_lo + ns - 1 - r, c0, c1, zv, A.ctl,
+        [&](int i) {
+          ci = A.c[i];
+          const double cr = A.cr[i];
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[v] = mul(t_s[(i - first) * V + v], cr);
+        },
+        coef, term, fold,
+        [&](int i) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            zv.put(i, V, v, mul(acc[v], ci));
+            t_s[(i - first) * V + v] = Pending<double>::value();
+          }
+        });
+  __syncthreads();
+}
+
+template <int SOLVER, int V, bool SW>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_constant__ SmallArgs A, int parts) {
+  constexpr int NW = kSmallThreads / 32;
+  extern __shared__ __align__(16) double dyn_s[];
+  __shared__ double red[2][2 * V][NW];
+  __shared__ Lane L_s[V];     // the lanes as reported
+  __shared__ double rn_s[V];  // their |r0|_1
+  const Rows<double>& R = A.R;
+  const int sys = blockIdx.x, c0 = A.seg_c0[sys], c1 = A.seg_c1[sys];
+  const int s_lo = c0 >> 5, ns = ((c1 + 31) >> 5) - s_lo, first = s_lo * 32;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* t_s = dyn_s;                             // SW: forward sweeps
+  double* z_s = dyn_s + (SW ? ns * 32 * V : 0);    // SW: backward sweeps; BiCGSTAB: z
+  double* p_s = SOLVER == 0 && SW ? z_s + ns * 32 * V : z_s;  // CG: p
+  double* x_s = SOLVER == 0 ? p_s : z_s;           // what the matrix product gathers
+  auto vals_of = [&](double* a) {
+    return SharedVals{(unsigned)__cvta_generic_to_shared(a), first};
+  };
+  auto each = [&](auto&& f) {  // f(i) for this thread's cells
+    for (int r = wid; r < ns; r += NW) {
+      const int i = first + r * 32 + lane;
+      if (i >= c0 && i < c1) f(i);
+    }
+  };
+  auto li = [&](int i, int v) { return (i - first) * V + v; };
+  int buf = 0;
+  auto sums = [&](auto& t) {  // block sums of t[], in every thread (and a barrier)
+    constexpr int NR = sizeof(t) / sizeof(double);
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const double x = warp_sum(t[k]);
+      if (lane == 0) red[buf][k][wid] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NR; ++k) t[k] = warp_sum_all(lane < NW ? red[buf][k][lane] : 0.0);
+    buf ^= 1;
+  };
+  // y = b - A x (RES) or y = A x for row i, x gathered from x_s
+  auto row = [&](int i, const double* x, auto res, double (&y)[V]) {
+    constexpr bool RES = decltype(res)::value;
+    RowIt<double> it(R, i);
+    const double d = __ldg(&R.diag[i]);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const double m = mul(d, x[li(i, v)]);
+      y[v] = RES ? sub(y[v], m) : m;
+    }
+    for (int u0 = 0; u0 < it.w; u0 += 6) {
+      int j[6];
+      double a[6];
+#pragma unroll
+      for (int u = 0; u < 6; ++u) {
+        j[u] = -1;
+        if (u0 + u < it.w) {
+          const int e = it.base + (u0 + u) * kWarp;
+          j[u] = __ldg(&R.col[e]);
+          a[u] = __ldg(&R.val[e]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 6; ++u)
+        if (j[u] >= 0) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const double m = mul(a[u], x[li(j[u], v)]);
+            y[v] = RES ? sub(y[v], m) : add(y[v], m);
+          }
+        }
+    }
+  };
+  using True = std::true_type;
+  using False = std::false_type;
+
+  if (parts & kSmallResidual) {  // solv_res.f90:12-29
+    each([&](int i) {
+      const int o = A.old_of_new[i];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const double f = A.phi_dev[(size_t)o * V + v];
+        A.phi[(size_t)i * V + v] = f;
+        x_s[li(i, v)] = f;
+      }
+    });
+    __syncthreads();
+    double l1[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) l1[v] = 0.0;
+    each([&](int i) {
+      const int o = A.old_of_new[i];
+      double y[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) y[v] = A.res_dev[(size_t)v * A.N + o];
+      if (!A.not_r0) row(i, x_s, True(), y);
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        A.res_dev[(size_t)v * A.N + o] = y[v];
+        A.r0[(size_t)i * V + v] = y[v];
+        l1[v] += fabs(y[v]);
+      }
+    });
+    sums(l1);
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int v = 0; v < V; ++v) A.l1[sys * V + v] = l1[v];
+    if (gridDim.x == 1) {  // solv_cg.f90:21 (a batch: the host looks at all its systems)
+      double mx = -HUGE_VAL;
+#pragma unroll
+      for (int v = 0; v < V; ++v) mx = mx < l1[v] ? l1[v] : mx;
+      if (mx < kSmall) return;
+    }
+    __syncthreads();
+  }
+  if (!(parts & kSmallLoop)) return;
+
+  // the lanes' scalars (every thread's own copy), bit v of act: still running
+  struct Scalars {
+    double s, alpha, beta, beta0, gam;  // BiCGSTAB: s is rho, beta is omeg
+  };
+  Scalars L[V];
+  unsigned act = 0;
+  int iter = 0;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {  // as k_lane_init
+    L[v] = {SOLVER == 0 ? kLarge : 0.0, 1.0, 0.0, 1.0, 1.0};
+    if (A.n_iter > 0) act |= 1u << v;
+    if (threadIdx.x == 0) {
+      L_s[v] = Lane{};
+      L_s[v].status = A.n_iter > 0 ? kLaneRunning : kLaneMaxIter;
+      rn_s[v] = A.l1[sys * V + v];  // this block's own, or the launch's before
+    }
+  }
+  auto on = [&](int v) { return ((act >> v) & 1u) != 0; };
+  auto pending = [&](double* a, int per) {  // whole slices
+    for (int k = threadIdx.x; k < ns * 32 * per; k += kSmallThreads) a[k] = Pending<double>::value();
+  };
+  // solv_precond
+  if constexpr (SW) {
+    pending(t_s, 1);
+    __syncthreads();
+    const SharedVals cv = vals_of(t_s);
+    double d = 0.0;
+    const bool dilu = A.imat == 2;
+    for (int r = wid; r < ns; r += NW)
+      sweep_slice<false, true, 8, 1, double2>(
+          A.N, R, s_lo + r, c0, c1, cv, A.ctl, [&](int i) { d = __ldg(&R.diag[i]); },
+          [&](int e) {
+            return make_double2(dilu ? __ldg(&A.fp[__ldg(&A.slot_src[e]) >> 1]) : 0.0,
+                                __ldg(&R.sval[e]));
+          },
+          [&](const double2& a, const double (&cj)[1], double (&m)[1]) {
+            m[0] = dilu ? mul(mul(a.x, cj[0]), a.y) : mul(mul(a.y, a.y), cj[0]);
+          },
+          [&](const double (&m)[1]) { d = sub(d, m[0]); },
+          [&](int i) {
+            const double ci = 1.0 / add(d, kSmall);
+            A.cr[i] = d;
+            A.c[i] = ci;
+            cv.put(i, 1, 0, ci);
+          });
+    __syncthreads();
+    pending(t_s, V);
+  }
+  each([&](int i) {
+    if constexpr (!SW) A.c[i] = 1.0 / add(__ldg(&R.diag[i]), kSmall);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const size_t k = (size_t)i * V + v;
+      A.r[k] = A.r0[k];
+      if (SOLVER == 0) p_s[li(i, v)] = 0.0;
+      else A.p[k] = A.q[k] = 0.0;
+    }
+  });
+  __syncthreads();
+  auto direct = [&](const double* b) {
+    if constexpr (SW) small_direct<V>(A, c0, c1, b, t_s, z_s);
+  };
+  // the stopping test of a lane whose |r|_1 is l1 (solv_cg.f90:78-82)
+  auto stop = [&](int v, double l1) {
+    const double ratio = l1 / (rn_s[v] + kSmall);
+    int status = kLaneRunning;
+    if (!(ratio == ratio) || isinf(ratio)) status = kLaneNaN;
+    else if (ratio < A.reduc) status = kLaneConverged;
+    else if (iter >= A.n_iter) status = kLaneMaxIter;
+    if (status == kLaneRunning) return;
+    act &= ~(1u << v);
+    if (threadIdx.x == 0) {
+      L_s[v].iter = iter;
+      L_s[v].l1 = l1;
+      L_s[v].ratio = ratio;
+      L_s[v].status = status;
+    }
+  };
+  if constexpr (SOLVER == 0) {
+    while (act) {
+      ++iter;
+      direct(A.r);
+      double rz[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) rz[v] = 0.0;
+      auto z_of = [&](int i, int v, double ri) {
+        return SW ? z_s[li(i, v)] : mul(ri, A.c[i]);
+      };
+      each([&](int i) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const double ri = A.r[(size_t)i * V + v];
+          rz[v] += prod(ri, z_of(i, v, ri));
+        }
+      });
+      sums(rz);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (on(v)) {
+          const double b = 1.0 / L[v].s;
+          L[v].s = rz[v];
+          L[v].beta = b * L[v].s;
+        }
+      each([&](int i) {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (on(v))
+            p_s[li(i, v)] = add(z_of(i, v, A.r[(size_t)i * V + v]), mul(L[v].beta, p_s[li(i, v)]));
+      });
+      __syncthreads();
+      double pq[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) pq[v] = 0.0;
+      each([&](int i) {
+        double y[V];
+        row(i, p_s, False(), y);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          A.q[(size_t)i * V + v] = y[v];
+          pq[v] += prod(p_s[li(i, v)], y[v]);
+        }
+      });
+      sums(pq);
+      double l1[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        if (on(v)) L[v].alpha = L[v].s / (pq[v] + kSmall);
+        l1[v] = 0.0;
+      }
+      each([&](int i) {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (on(v)) {
+            const size_t k = (size_t)i * V + v;
+            A.phi[k] = add(A.phi[k], mul(L[v].alpha, p_s[li(i, v)]));
+            const double rn = sub(A.r[k], mul(L[v].alpha, A.q[k]));
+            A.r[k] = rn;
+            l1[v] += fabs(rn);
+          }
+      });
+      sums(l1);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (on(v)) stop(v, l1[v]);
+    }
+  } else {
+    auto head = [&](Scalars& X, double rho) {  // solv_bicg.f90:48-50
+      X.s = rho;
+      X.beta = X.s * X.gam / (X.alpha * X.beta0 + kSmall);
+      X.beta0 = X.s;
+    };
+    double rho[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) rho[v] = 0.0;
+    each([&](int i) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const size_t k = (size_t)i * V + v;
+        rho[v] += prod(A.r[k], A.r0[k]);
+      }
+    });
+    sums(rho);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      if (on(v)) head(L[v], rho[v]);
+    while (act) {
+      ++iter;
+      each([&](int i) {  // p = r + omeg (p - alpha u)
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const size_t k = (size_t)i * V + v;
+          if (on(v))
+            A.p[k] = add(A.r[k], mul(L[v].beta, sub(A.p[k], mul(L[v].alpha, A.q[k]))));
+          if (!SW) z_s[li(i, v)] = mul(A.p[k], A.c[i]);
+        }
+      });
+      if (SW) direct(A.p);
+      else __syncthreads();
+      double g[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) g[v] = 0.0;
+      each([&](int i) {  // u = A z, u.r0
+        double y[V];
+        row(i, z_s, False(), y);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const size_t k = (size_t)i * V + v;
+          A.q[k] = y[v];
+          g[v] += prod(y[v], A.r0[k]);
+        }
+      });
+      sums(g);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (on(v)) L[v].gam = L[v].s / (g[v] + kSmall);
+      each([&](int i) {  // phi += gam z; r -= gam u
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const size_t k = (size_t)i * V + v;
+          if (on(v)) {
+            A.phi[k] = add(A.phi[k], mul(L[v].gam, z_s[li(i, v)]));
+            A.r[k] = sub(A.r[k], mul(L[v].gam, A.q[k]));
+          }
+          if (!SW) z_s[li(i, v)] = mul(A.r[k], A.c[i]);
+        }
+      });
+      __syncthreads();
+      if (SW) direct(A.r);
+      double d[2 * V];
+#pragma unroll
+      for (int k = 0; k < 2 * V; ++k) d[k] = 0.0;
+      each([&](int i) {  // v = A z, v.r, v.v
+        double y[V];
+        row(i, z_s, False(), y);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const size_t k = (size_t)i * V + v;
+          A.v[k] = y[v];
+          d[v] += prod(y[v], A.r[k]);
+          d[V + v] += prod(y[v], y[v]);
+        }
+      });
+      sums(d);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (on(v)) L[v].alpha = d[v] / (d[V + v] + kSmall);
+#pragma unroll
+      for (int k = 0; k < 2 * V; ++k) d[k] = 0.0;
+      each([&](int i) {  // phi += alpha z; r -= alpha v; |r|_1, r.r0
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (on(v)) {
+            const size_t k = (size_t)i * V + v;
+            A.phi[k] = add(A.phi[k], mul(L[v].alpha, z_s[li(i, v)]));
+            const double rn = sub(A.r[k], mul(L[v].alpha, A.v[k]));
+            A.r[k] = rn;
+            d[v] += fabs(rn);
+            d[V + v] += prod(rn, A.r0[k]);
+          }
+      });
+      sums(d);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (on(v)) {
+          stop(v, d[v]);
+          if (on(v)) head(L[v], d[V + v]);
+        }
+    }
+  }
+  each([&](int i) {
+    const int o = A.old_of_new[i];
+#pragma unroll
+    for (int v = 0; v < V; ++v) A.phi_dev[(size_t)o * V + v] = A.phi[(size_t)i * V + v];
+  });
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int v = 0; v < V; ++v) A.lanes[sys * V + v] = L_s[v];
+}
+
 // ============ persistent fused Jacobi PCG: one thread-block cluster per system ============
 // The whole Krylov loop of solv_cg.f90:37-84 with imat = 0 in one launch:
 // each cluster of CTAs (kPcgCluster, or kPcgClusterMax where the GPU holds
@@ -2226,7 +2750,7 @@ __global__ void k_loop_ctl(cudaGraphConditionalHandle h, const int* __restrict__
 __global__ void k_sweep_selftest(Rows<double> R, const double* never, SweepCtl* ctl) {
   sweep_rows<false, false, 1, 1, int>(
       2, R, SweepMap{nullptr, nullptr, 1}, never, ctl, [](int) {}, [](int) { return 0; },
-      [](int, const double (&)[1]) {}, [](int) {});
+      [](int, const double (&)[1], double (&)[1]) {}, [](const double (&)[1]) {}, [](int) {});
 }
 
 }  // namespace sg

@@ -139,6 +139,8 @@ struct solv_gpu_ctx {
   DevBuf w_t, wf_t;
   bool t_ready = false, tf_ready = false;  // t / tf hold only the pending pattern
   DevBuf sweep_ctl;
+  bool sweeps_checked = false;             // this solve has read the flag itself
+  std::map<const void*, bool> small_ready;  // small-system kernels with their shared memory set
   std::map<const void*, int> coop_blocks;  // resident blocks per SM, per sweep kernel
 
   // captured iteration graphs, keyed by (solver, imat, V, fp32)
@@ -1801,6 +1803,102 @@ int resident_pcg(solv_gpu_ctx* c, const double* cc, double* phi, const double* r
   return SOLV_GPU_OK;
 }
 
+// ---- small systems (k_small_solve) ---------------------------------------------
+using SmallKernel = void (*)(const sg::SmallArgs, int);
+template <int V>
+SmallKernel small_kernel(int solver, bool sweeps, int& vectors) {
+  vectors = solver == 0 ? (sweeps ? sg::kSmallVectors<0, true> : sg::kSmallVectors<0, false>)
+                        : (sweeps ? sg::kSmallVectors<1, true> : sg::kSmallVectors<1, false>);
+  if (solver == 0) return sweeps ? sg::k_small_solve<0, V, true> : sg::k_small_solve<0, V, false>;
+  return sweeps ? sg::k_small_solve<1, V, true> : sg::k_small_solve<1, V, false>;
+}
+
+// Whether a call runs as k_small_solve (unless the caller asked for a graph
+// form or a persistent cluster): every system small, no more of them than SMs.
+// A DIC/DILU iteration costs one block about 0.65 us a level and 0.008 us a
+// value (cell x component), the step kernels 1.5 us a level and 20 us (20^3
+// RCM, 58 levels, 8000 cells: 104 against 106 us; one-deep 37x42, 78 levels:
+// 63 against 140; 14^3 multicolour, 2 levels: 32 against 27), hence the line;
+// 8192 values also fill the shared memory.  Without a recurrence 4096 (14^3
+// BiCGSTAB 17 against 27 us an iteration), and Jacobi-PCG of one component,
+// which k_pcg_grid spreads over several SMs, 1024.
+constexpr int kSmallValues = 8192;
+constexpr int kSmallValuesNone = 4096;
+constexpr int kSmallValuesJacobi = 1024;
+bool small_fits(const solv_gpu_ctx* c, int solver, int imat, int V, int n_iter) {
+  if (c->graph_loop != 2 || c->graph_iters <= 0 || c->persistent || c->n_seg > c->n_sm || n_iter < 0)
+    return false;
+  int most = 0;
+  for (size_t k = 0; k < c->seg_c0_caller.size(); ++k)
+    most = std::max(most, c->seg_c1_caller[k] - c->seg_c0_caller[k]);
+  const int levels = (int)c->lvl_ptr.size() - 1;
+  const int cap = imat > 0                ? std::min(kSmallValues, 100 * std::min(levels, 1000) + 2000)
+                  : solver == 0 && V == 1 ? kSmallValuesJacobi
+                                          : kSmallValuesNone;
+  return (long long)most * V <= cap;
+}
+
+template <int V>
+int solve_small(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter, WS<double>& w,
+                double* phi_dev, double* res0_dev, double* res0_n, int not_r0,
+                std::vector<Lane>& hl, bool& zero) {
+  cudaStream_t s = c->stream;
+  const SegMap m = segmap(c);
+  const int nl = c->n_seg * V;
+  int slices = 0, vectors = 0;
+  for (size_t k = 0; k < c->seg_c0_caller.size(); ++k)
+    slices = std::max(slices, ((c->seg_c1_caller[k] + 31) >> 5) - (c->seg_c0_caller[k] >> 5));
+  SmallKernel kern = small_kernel<V>(solver, imat > 0, vectors);
+  const size_t smem = (size_t)vectors * slices * 32 * V * sizeof(double);
+  if (!c->small_ready[(const void*)kern]) {
+    CUDA_TRY(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     3 * (kSmallValues + 64 * V) * (int)sizeof(double)));
+    c->small_ready[(const void*)kern] = true;
+  }
+  sg::SmallArgs A;
+  A.R = rows<double>(c);
+  A.seg_c0 = m.seg_c0;
+  A.seg_c1 = m.seg_c1;
+  A.old_of_new = c->old_of_new.as<int>();
+  A.slot_src = c->slot_src.as<int>();
+  A.fp = c->fp.as<double>();
+  A.phi_dev = phi_dev;
+  A.res_dev = res0_dev;
+  A.phi = w.phi; A.r = w.r; A.r0 = w.r0; A.p = w.p; A.q = w.q; A.v = w.v; A.c = w.c; A.cr = w.cr;
+  A.lanes = c->lanes.as<Lane>();
+  A.l1 = c->l1.as<double>();
+  A.ctl = sweep_ctl(c);
+  A.N = c->N;
+  A.not_r0 = not_r0;
+  A.imat = imat;
+  A.n_iter = n_iter;
+  A.reduc = reduc;
+  sg::SweepCtl ctl{};
+  // solv_cg.f90:21 looks at all the systems of a batch before any iterates
+  const int both = sg::kSmallResidual | sg::kSmallLoop;
+  zero = false;
+  for (int parts = c->n_seg > 1 ? sg::kSmallResidual : both;; parts = sg::kSmallLoop) {
+    kern<<<c->n_seg, sg::kSmallThreads, smem, s>>>(A, parts);
+    c->launches++;
+    CUDA_TRY(c, cudaGetLastError());
+    if (parts & sg::kSmallResidual)
+      CUDA_TRY(c, cudaMemcpyAsync(res0_n, c->l1.p, nl * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (parts & sg::kSmallLoop) {
+      CUDA_TRY(c, cudaMemcpyAsync(hl.data(), c->lanes.p, nl * sizeof(Lane), cudaMemcpyDeviceToHost, s));
+      CUDA_TRY(c, cudaMemcpyAsync(&ctl, c->sweep_ctl.p, sizeof(ctl), cudaMemcpyDeviceToHost, s));
+    }
+    CUDA_TRY(c, cudaStreamSynchronize(s));
+    if (parts & sg::kSmallResidual) {
+      double mx = -HUGE_VAL;
+      for (int l = 0; l < nl; ++l) mx = std::max(mx, res0_n[l]);
+      if ((zero = mx < sg::kSmall)) return SOLV_GPU_OK;
+    }
+    if (parts & sg::kSmallLoop) break;
+  }
+  c->sweeps_checked = true;
+  return ctl.err ? sweep_check(c) : SOLV_GPU_OK;
+}
+
 // Full FP64 solve (solver 0 = CG, 1 = BiCGSTAB) on device buffers in the
 // caller layouts.
 template <int V>
@@ -1813,28 +1911,54 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
   const int N = c->N;
   cudaStream_t s = c->stream;
   const int* o2n = c->old_of_new.as<int>();
+  const int nl = c->n_seg * V;
+  std::vector<Lane> hl(nl);
+  auto zero_rhs = [&]() {  // solv_cg.f90:21 early return
+    if (st) st->status = SOLV_GPU_ZERO_RHS;
+    if (out_iters) std::fill(out_iters, out_iters + nl, 0);
+    if (out_ratio) std::fill(out_ratio, out_ratio + nl, 0.0);
+    return SOLV_GPU_OK;
+  };
+  auto report = [&](int graph_launches) {
+    int status = SOLV_GPU_OK;
+    for (int l = 0; l < nl; ++l) {
+      if (hl[l].status == sg::kLaneNaN) status = SOLV_GPU_NAN;
+      else if (hl[l].status != sg::kLaneConverged && status == SOLV_GPU_OK) status = SOLV_GPU_MAXITER;
+      if (out_iters) out_iters[l] = hl[l].iter;
+      if (out_ratio) out_ratio[l] = hl[l].ratio;
+    }
+    if (st) {
+      for (int v = 0; v < V && v < nl; ++v) {
+        st->iters[v] = hl[v].iter;
+        st->ratio[v] = hl[v].ratio;
+      }
+      st->status = status;
+      st->graph_launches += graph_launches;
+    }
+    return status;
+  };
+  if (small_fits(c, solver, imat, V, n_iter)) {
+    bool zero = false;
+    if (st) st->n_vc = V;
+    rc = solve_small<V>(c, solver, imat, reduc, n_iter, w, phi_dev, res0_dev, res0_n, not_r0, hl,
+                        zero);
+    return rc ? rc : zero ? zero_rhs() : report(0);
+  }
   sg::k_phi_in<double><<<grid_for(c, N), c->block, 0, s>>>(N, V, o2n, phi_dev, w.phi);
   sg::k_col_in<<<grid_for(c, N), c->block, 0, s>>>(N, V, o2n, res0_dev, w.r0);
   c->launches += 2;
-  const int nl = c->n_seg * V;
   rc = run_res(c, V, w.phi, w.r0, not_r0);  // solv_res: r0 = b - A phi, res0_n
   if (rc) return rc;
   sg::k_set_res0n<<<1, 256, 0, s>>>(c->lanes.as<Lane>(), nl, c->l1.as<double>());
   // res0 out = initial residual (solv_cg.f90:20)
   sg::k_col_out<<<grid_for(c, N), c->block, 0, s>>>(N, V, o2n, w.r0, res0_dev);
   c->launches++;
-  std::vector<Lane> hl(nl);
   CUDA_TRY(c, cudaMemcpyAsync(res0_n, c->l1.p, nl * sizeof(double), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaStreamSynchronize(s));
   double mx = -HUGE_VAL;
   for (int l = 0; l < nl; ++l) mx = std::max(mx, res0_n[l]);
   if (st) st->n_vc = V;
-  if (mx < sg::kSmall) {  // solv_cg.f90:21 early return
-    if (st) st->status = SOLV_GPU_ZERO_RHS;
-    if (out_iters) std::fill(out_iters, out_iters + nl, 0);
-    if (out_ratio) std::fill(out_ratio, out_ratio + nl, 0.0);
-    return SOLV_GPU_OK;
-  }
+  if (mx < sg::kSmall) return zero_rhs();
   if ((rc = launch_precond(c, imat, w.c, w.cr))) return rc;  // solv_precond
   // Jacobi-PCG of systems that fit: one launch with the matrix in shared
   // memory (resident_plan), unless the caller asked for a graph form; with
@@ -1968,22 +2092,7 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
   c->launches++;
   CUDA_TRY(c, cudaMemcpyAsync(hl.data(), c->lanes.p, nl * sizeof(Lane), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaStreamSynchronize(s));
-  int status = SOLV_GPU_OK;
-  for (int l = 0; l < nl; ++l) {
-    if (hl[l].status == sg::kLaneNaN) status = SOLV_GPU_NAN;
-    else if (hl[l].status != sg::kLaneConverged && status == SOLV_GPU_OK) status = SOLV_GPU_MAXITER;
-    if (out_iters) out_iters[l] = hl[l].iter;
-    if (out_ratio) out_ratio[l] = hl[l].ratio;
-  }
-  if (st) {
-    for (int v = 0; v < V && v < nl; ++v) {
-      st->iters[v] = hl[v].iter;
-      st->ratio[v] = hl[v].ratio;
-    }
-    st->status = status;
-    st->graph_launches += gl;
-  }
-  return status;
+  return report(gl);
 }
 
 // Mixed precision: FP32 inner Krylov solves of A d = r inside an FP64
@@ -3064,10 +3173,11 @@ static int solve_common(solv_gpu_ctx* c, int solver, int imat, double reduc, int
   }
   CUDA_TRY(c, cudaSetDevice(c->dev));
   c->launches = 0;
+  c->sweeps_checked = false;
   CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
   int rc = solve_dispatch(c, solver, imat, reduc, n_iter, n_vc, phi_dev, res0_dev, res0_n, not_r0,
                           st, out_iters, out_ratio);
-  if (imat > 0 && c->sweep_ctl.p && (rc == SOLV_GPU_OK || rc == SOLV_GPU_MAXITER || rc == SOLV_GPU_NAN)) {
+  if (imat > 0 && !c->sweeps_checked && c->sweep_ctl.p && (rc == SOLV_GPU_OK || rc == SOLV_GPU_MAXITER || rc == SOLV_GPU_NAN)) {
     const int rs = sweep_check(c);
     if (rs) rc = rs;
   }
