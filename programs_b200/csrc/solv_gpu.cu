@@ -3692,10 +3692,13 @@ int solv_gpu_gnn_grad_dev(solv_gpu_ctx* c, const double* r0_dev, const double* s
   const float gsc = 1.0f / ((float)N * (float)n_samples);
   if (c->gnn_loss == 2 && c->mg_smoother == 2)  // the face weights are not used
     CUDA_TRY(c, cudaMemsetAsync(B[TB_ES], 0, N * sizeof(float), c->stream));
-  gnn::k_gnn_heads_back<<<gw, 256, 0, c->stream>>>(N, B[TB_H0 + 3], B[TB_PA], B[TB_S], B[TB_DS],
+  // blocks of the kernels that end in parameter gradients: enough to fill the
+  // SMs, few enough that the atomics at their ends do not count
+  const int gb = std::min(gw, c->n_sm * 4);
+  gnn::k_gnn_heads_back<<<gb, 32 * gnn::kBackWarps, 0, c->stream>>>(N, B[TB_H0 + 3], B[TB_PA], B[TB_S], B[TB_DS],
                                                    B[TB_ES], gsc, P, B[TB_DHA], G);
   float* dcur = B[TB_DHA];
-  const int lb = std::max(1, std::min((N + 7) / 8, c->n_sm * 8));
+  const int lb = std::max(1, std::min((N + 7) / 8, c->n_sm * 4));
   for (int l = gnn::NL - 1; l >= 0; --l) {
     const float* L = P + gnn::P_LAYER + l * gnn::LAYER_SZ;
     gnn::k_gnn_layer_back1<<<lb, 256, 0, c->stream>>>(
@@ -3706,7 +3709,7 @@ int solv_gpu_gnn_grad_dev(solv_gpu_ctx* c, const double* r0_dev, const double* s
                                                       dnext);
     dcur = dnext;
   }
-  gnn::k_gnn_enc_back<<<gw, 256, 0, c->stream>>>(N, F, B[TB_U0], B[TB_PRE0], dcur, G);
+  gnn::k_gnn_enc_back<<<gb, 32 * gnn::kBackWarps, 0, c->stream>>>(N, F, B[TB_U0], B[TB_PRE0], dcur, G);
   CUDA_TRY(c, cudaGetLastError());
   double j = 0;
   CUDA_TRY(c, cudaMemcpyAsync(&j, c->g_jsum.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
