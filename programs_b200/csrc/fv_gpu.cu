@@ -30,13 +30,62 @@ __device__ __forceinline__ double lerp(double w, double an, double ap) {
   return da(dm(w, an), dm(ds(1.0, w), ap));
 }
 
+// What bounds the cell kernels is the number of gather requests L1 can take
+// (60-77% of its throughput at 80^3, DRAM at 30%), so everything gathered
+// stands in aligned 32-byte records and moves in 256-bit loads: two per face
+// (unit normal and area; centre and weight), one per cell (centre and volume),
+// one per gradient carried from sweep to sweep.  As arrays of single values
+// the same visit took 18 requests.  The face kernels that need a few of these
+// values, in face order, read them as plain arrays (sw, vol).  A cell's faces stand in a sliced
+// ELL (32 cells a slice, slot-major, faces ascending) with the cell on the
+// face's other side beside them, so a warp reads consecutive words and the
+// neighbour's values need no trip through the face.
+struct alignas(32) D4 {
+  double x, y, z, w;
+};
+__device__ __forceinline__ D4 ld4(const D4* p) {  // read-only data
+  D4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+
 struct Geo {
   int n_cell, n_face;
-  const int *ip, *in;          // 0-based, in = -1 on boundary faces
-  const double *s, *nrm, *xf, *l, *w;
-  const double *xc, *vol;
-  const int *cf_ptr, *cf;      // faces of each cell, ascending
+  const int2* ab;              // owner and neighbour cell, 0-based (-1 on boundary faces)
+  const D4 *fn, *fc;           // per face {unit normal, area}; {centre, w_fp}
+  const D4* cr;                // per cell {centre, volume}
+  const double2* sw;           // per face {area, w_fp}
+  const double *l, *vol;       // l_pn; cell volumes
+  const int* cs_ptr;           // first slot of each slice of 32 cells
+  const int2* cs;              // slots: {2 face + (1 for the neighbour's side), other cell};
+                               // {-1, -1} padding, other cell -1 on boundary faces
 };
+
+struct Face {
+  double nx, ny, nz, s, x, y, z, w;
+};
+__device__ __forceinline__ Face face_of(const Geo& g, int f) {
+  const D4 a = ld4(g.fn + f), b = ld4(g.fc + f);
+  return {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+}
+struct Cell {
+  double x, y, z, vol;
+};
+__device__ __forceinline__ Cell cell_of(const Geo& g, int c) {
+  const D4 a = ld4(g.cr + c);
+  return {a.x, a.y, a.z, a.w};
+}
+// f(face, owner side, other cell) for the faces of cell c, ascending
+template <typename F>
+__device__ __forceinline__ void faces_of(const Geo& g, int c, F&& f) {
+  const int b = g.cs_ptr[c >> 5], e = g.cs_ptr[(c >> 5) + 1];
+  for (int q = b + (c & 31); q < e; q += 32) {
+    const int2 t = g.cs[q];
+    if (t.x < 0) break;  // padding only follows a cell's faces
+    f(t.x >> 1, (t.x & 1) == 0, t.y);
+  }
+}
 
 // std::min / std::max as the host evaluates them (ties and NaN included)
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
@@ -51,15 +100,11 @@ __device__ __forceinline__ double dot3(double ax, double ay, double az, double b
                                        double bz) {
   return da(da(dm(ax, bx), dm(ay, by)), dm(az, bz));
 }
-__device__ __forceinline__ Dx aux_dx(const Geo& g, int f, int c) {
-  const double* xf = g.xf + 3 * f;
-  const double* nn = g.nrm + 3 * f;
-  const double* xc = g.xc + 3 * c;
-  const double t = dot3(ds(xf[0], xc[0]), ds(xf[1], xc[1]), ds(xf[2], xc[2]), nn[0], nn[1], nn[2]);
-  return {ds(ds(xf[0], dm(nn[0], t)), xc[0]), ds(ds(xf[1], dm(nn[1], t)), xc[1]),
-          ds(ds(xf[2], dm(nn[2], t)), xc[2])};
+__device__ __forceinline__ Dx aux_dx(const Face& F, const Cell& C) {
+  const double t = dot3(ds(F.x, C.x), ds(F.y, C.y), ds(F.z, C.z), F.nx, F.ny, F.nz);
+  return {ds(ds(F.x, dm(F.nx, t)), C.x), ds(ds(F.y, dm(F.ny, t)), C.y),
+          ds(ds(F.z, dm(F.nz, t)), C.z)};
 }
-
 
 constexpr int kBlock = 256;
 constexpr int kRedBlocks = 1024;
@@ -67,12 +112,11 @@ constexpr int kRedBlocks = 1024;
 int grid(long long n) { return (int)std::max(1LL, std::min((n + kBlock - 1) / kBlock, 148LL * 16)); }
 
 // d = rho (1/a_P)_f area V_f / l_pn (cfd_setup.f90:604-634)
-__device__ __forceinline__ double pc_coef(const Geo& g, int f, int a, int b, const double* ap,
-                                          double rho) {
-  const double w = g.w[f];
-  const double p_r = da(dd(w, da(ap[b], 1e-20)), dd(ds(1.0, w), da(ap[a], 1e-20)));
-  const double v = lerp(w, g.vol[b], g.vol[a]);
-  return dd(dm(dm(dm(rho, p_r), g.s[f]), v), g.l[f]);
+__device__ __forceinline__ double pc_coef(double w, double s, double l, double vb, double va,
+                                          double apb, double apa, double rho) {
+  const double p_r = da(dd(w, da(apb, 1e-20)), dd(ds(1.0, w), da(apa, 1e-20)));
+  const double v = lerp(w, vb, va);
+  return dd(dm(dm(dm(rho, p_r), s), v), l);
 }
 
 // ---- momentum ---------------------------------------------------------------------
@@ -80,20 +124,21 @@ __global__ void k_fv_mom_faces(Geo g, const double* __restrict__ u, const double
                                double rho, double mu, double* __restrict__ p, double* __restrict__ n,
                                double* __restrict__ flux_out) {
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
-    const int a = g.ip[f], b = g.in[f];
-    const double d = dd(dm(mu, g.s[f]), g.l[f]);
+    const int2 ab = g.ab[f];
+    const int a = ab.x, b = ab.y;
+    const double2 sw = g.sw[f];
+    const double d = dd(dm(mu, sw.x), g.l[f]);
     if (b >= 0) {
       double c;
       if (flux) {
         c = flux[f];
       } else {
-        const double w = g.w[f];
-        const double uf = lerp(w, u[3 * b], u[3 * a]);
-        const double vf = lerp(w, u[3 * b + 1], u[3 * a + 1]);
-        const double wf = lerp(w, u[3 * b + 2], u[3 * a + 2]);
-        const double un = da(da(dm(uf, g.nrm[3 * f]), dm(vf, g.nrm[3 * f + 1])),
-                             dm(wf, g.nrm[3 * f + 2]));
-        c = dm(dm(rho, g.s[f]), un);
+        const D4 F = ld4(g.fn + f);
+        const double uf = lerp(sw.y, u[3 * b], u[3 * a]);
+        const double vf = lerp(sw.y, u[3 * b + 1], u[3 * a + 1]);
+        const double wf = lerp(sw.y, u[3 * b + 2], u[3 * a + 2]);
+        const double un = da(da(dm(uf, F.x), dm(vf, F.y)), dm(wf, F.z));
+        c = dm(dm(rho, sw.x), un);
       }
       if (flux_out) flux_out[f] = c;
       const double mn = (0.0 < c) ? 0.0 : c;  // std::min(c, 0.0)
@@ -113,19 +158,17 @@ __global__ void k_fv_mom_cells(Geo g, const double* __restrict__ u, const double
                                double* __restrict__ pl, double* __restrict__ rhs) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
     double s = 0.0, rx = 0.0;
-    for (int q = g.cf_ptr[c]; q < g.cf_ptr[c + 1]; ++q) {
-      const int f = g.cf[q];
-      if (g.in[f] < 0) {
+    faces_of(g, c, [&](int f, bool own, int other) {
+      if (other < 0) {
         const double d = -p[f];
         s = da(s, d);
         // the moving lid: the y = 1 wall (outward normal +y)
-        if (g.nrm[3 * f + 1] > 0.9 && g.xf[3 * f + 1] > 1.0 - 1e-9) rx = da(rx, dm(d, u_lid));
-      } else if (g.ip[f] == c) {
-        s = ds(s, p[f]);
+        const Face F = face_of(g, f);
+        if (F.ny > 0.9 && F.y > 1.0 - 1e-9) rx = da(rx, dm(d, u_lid));
       } else {
-        s = ds(s, n[f]);
+        s = ds(s, own ? p[f] : n[f]);
       }
-    }
+    });
     s = dd(s, urf);
     pl[c] = s;
     if (rhs) {
@@ -142,10 +185,12 @@ __global__ void k_fv_pc_faces(Geo g, const double* __restrict__ ap, double rho, 
                               double* __restrict__ dface, double* __restrict__ p,
                               double* __restrict__ n) {
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
-    const int a = g.ip[f], b = g.in[f];
+    const int2 ab = g.ab[f];
+    const int a = ab.x, b = ab.y;
     double d = 0.0, off = 0.0;
     if (b >= 0) {
-      d = pc_coef(g, f, a, b, ap, rho);
+      const double2 sw = g.sw[f];
+      d = pc_coef(sw.y, sw.x, g.l[f], g.vol[b], g.vol[a], ap[b], ap[a], rho);
       if (a != pc && b != pc) off = -d;
     }
     dface[f] = d;
@@ -157,41 +202,52 @@ __global__ void k_fv_pc_faces(Geo g, const double* __restrict__ ap, double rho, 
 __global__ void k_fv_pc_cells(Geo g, const double* __restrict__ dface, double* __restrict__ pl) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int q = g.cf_ptr[c]; q < g.cf_ptr[c + 1]; ++q) {
-      const int f = g.cf[q];
-      if (g.in[f] >= 0) s = da(s, dface[f]);
-    }
+    faces_of(g, c, [&](int f, bool, int other) {
+      if (other >= 0) s = da(s, dface[f]);
+    });
     pl[c] = s;
   }
 }
 
 // ---- Green-Gauss gradient -----------------------------------------------------------
+// The kernels over components come with NC = 3 (all the components of a
+// vector field in one thread: the geometry is read and the auxiliary points
+// are formed once) and NC = 1 (one component a thread, blockIdx.y of nc).
+template <int NC>
 __global__ void k_fv_gradient(Geo g, int nc, const double* __restrict__ phi,
                               double* __restrict__ grad) {
-  const long long tot = (long long)g.n_cell * nc;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(t / nc), k = (int)(t % nc);
-    double gx = 0.0, gy = 0.0, gz = 0.0;
-    for (int q = g.cf_ptr[c]; q < g.cf_ptr[c + 1]; ++q) {
-      const int f = g.cf[q];
-      const int a = g.ip[f], b = g.in[f];
-      const double pa = phi[(size_t)a * nc + k];
-      const double pf = b >= 0 ? lerp(g.w[f], phi[(size_t)b * nc + k], pa) : pa;
-      const double ps = dm(pf, g.s[f]);
-      const double tx = dm(ps, g.nrm[3 * f]), ty = dm(ps, g.nrm[3 * f + 1]),
-                   tz = dm(ps, g.nrm[3 * f + 2]);
-      if (a == c) {
-        gx = da(gx, tx); gy = da(gy, ty); gz = da(gz, tz);
-      } else {
-        gx = ds(gx, tx); gy = ds(gy, ty); gz = ds(gz, tz);
-      }
+  const int k0 = NC == 1 ? blockIdx.y : 0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
+    double gx[NC], gy[NC], gz[NC], own_phi[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      gx[k] = gy[k] = gz[k] = 0.0;
+      own_phi[k] = phi[(size_t)c * nc + k0 + k];
     }
-    const double v = g.vol[c];
-    double* o = grad + ((size_t)c * nc + k) * 3;
-    o[0] = dd(gx, v);
-    o[1] = dd(gy, v);
-    o[2] = dd(gz, v);
+    faces_of(g, c, [&](int f, bool own, int other) {
+      const Face F = face_of(g, f);
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        double pf = own_phi[k];
+        if (other >= 0) {
+          const double po = phi[(size_t)other * nc + k0 + k];
+          pf = own ? lerp(F.w, po, pf) : lerp(F.w, pf, po);
+        }
+        const double ps = dm(pf, F.s);
+        const double tx = dm(ps, F.nx), ty = dm(ps, F.ny), tz = dm(ps, F.nz);
+        gx[k] = own ? da(gx[k], tx) : ds(gx[k], tx);
+        gy[k] = own ? da(gy[k], ty) : ds(gy[k], ty);
+        gz[k] = own ? da(gz[k], tz) : ds(gz[k], tz);
+      }
+    });
+    const double v = g.cr[c].w;
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      double* o = grad + ((size_t)c * nc + k0 + k) * 3;
+      o[0] = dd(gx[k], v);
+      o[1] = dd(gy[k], v);
+      o[2] = dd(gz[k], v);
+    }
   }
 }
 
@@ -200,70 +256,77 @@ __global__ void k_fv_gradient(Geo g, int nc, const double* __restrict__ phi,
 // of each face (previous sweep's gradient g0 at the auxiliary points after
 // the first sweep; walls by neu), its term ((phi_f s) n) / V added by each
 // of the face's cells in ascending face order, 1/V (vr) formed once per
-// cell.  bval[f*nc + k] are the wall values for neu = 0.
-__device__ __forceinline__ double sweep_face_value(const Geo& g, int f, int nc, int k,
-                                                   const double* __restrict__ phi,
-                                                   const double* __restrict__ bval, int neu,
-                                                   const double* __restrict__ g0) {
-  const int a = g.ip[f], b = g.in[f];
-  const double pa = phi[(size_t)a * nc + k];
-  const double* ga0 = g0 ? g0 + ((size_t)a * nc + k) * 3 : nullptr;
-  if (b >= 0) {
-    const double pb = phi[(size_t)b * nc + k];
-    if (g0) {
-      const double* gb0 = g0 + ((size_t)b * nc + k) * 3;
-      const Dx xa = aux_dx(g, f, a), xb = aux_dx(g, f, b);
-      const double pp = da(pa, dot3(ga0[0], ga0[1], ga0[2], xa.x, xa.y, xa.z));
-      const double pn = da(pb, dot3(gb0[0], gb0[1], gb0[2], xb.x, xb.y, xb.z));
-      return lerp(g.w[f], pn, pp);
-    }
-    return lerp(g.w[f], pb, pa);
-  }
-  if (neu > 0) {
-    double pf = pa;
-    if (g0 && neu == 2) {
-      const double* xf = g.xf + 3 * f;
-      const double* xc = g.xc + 3 * a;
-      pf = da(pf, dot3(ga0[0], ga0[1], ga0[2], ds(xf[0], xc[0]), ds(xf[1], xc[1]),
-                       ds(xf[2], xc[2])));
-    }
-    return pf;
-  }
-  return bval[(size_t)f * nc + k];
-}
-
+// cell.  bval[f*nc + k] are the wall values for neu = 0.  The gradients
+// between sweeps (g0, and grad where PAD) are records of four.
+template <int NC, bool CORR, bool PAD>
 __global__ void k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi,
                                 const double* __restrict__ bval, int neu,
-                                const double* __restrict__ vr, const double* __restrict__ g0,
+                                const double* __restrict__ vr, const D4* __restrict__ g0,
                                 double* __restrict__ grad) {
-  const long long tot = (long long)g.n_cell * nc;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(t / nc), k = (int)(t % nc);
-    double gx = 0.0, gy = 0.0, gz = 0.0;
+  const int k0 = NC == 1 ? blockIdx.y : 0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
+    double gx[NC], gy[NC], gz[NC], pc[NC];
+    D4 gc[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const size_t q = (size_t)c * nc + k0 + k;
+      gx[k] = gy[k] = gz[k] = 0.0;
+      pc[k] = phi[q];
+      gc[k] = CORR ? ld4(g0 + q) : D4{};
+    }
     const double v = vr[c];
-    for (int q = g.cf_ptr[c]; q < g.cf_ptr[c + 1]; ++q) {
-      const int f = g.cf[q];
-      const double ps = dm(sweep_face_value(g, f, nc, k, phi, bval, neu, g0), g.s[f]);
-      const double* nn = g.nrm + 3 * f;
-      const double tx = dm(dm(ps, nn[0]), v), ty = dm(dm(ps, nn[1]), v),
-                   tz = dm(dm(ps, nn[2]), v);
-      if (g.ip[f] == c) {
-        gx = da(gx, tx); gy = da(gy, ty); gz = da(gz, tz);
+    const Cell C = cell_of(g, c);
+    faces_of(g, c, [&](int f, bool own, int other) {
+      const Face F = face_of(g, f);
+      Dx xc{}, xo{};  // this cell's auxiliary point and the other's
+      if (CORR && other >= 0) {
+        xc = aux_dx(F, C);
+        xo = aux_dx(F, cell_of(g, other));
+      }
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        double pf;
+        if (other >= 0) {
+          const size_t q = (size_t)other * nc + k0 + k;
+          double me = pc[k], po = phi[q];
+          if (CORR) {
+            const D4 go = ld4(g0 + q);
+            me = da(me, dot3(gc[k].x, gc[k].y, gc[k].z, xc.x, xc.y, xc.z));
+            po = da(po, dot3(go.x, go.y, go.z, xo.x, xo.y, xo.z));
+          }
+          pf = own ? lerp(F.w, po, me) : lerp(F.w, me, po);
+        } else if (neu > 0) {
+          pf = pc[k];
+          if (CORR && neu == 2)
+            pf = da(pf, dot3(gc[k].x, gc[k].y, gc[k].z, ds(F.x, C.x), ds(F.y, C.y),
+                             ds(F.z, C.z)));
+        } else {
+          pf = bval[(size_t)f * nc + k0 + k];
+        }
+        const double ps = dm(pf, F.s);
+        const double tx = dm(dm(ps, F.nx), v), ty = dm(dm(ps, F.ny), v), tz = dm(dm(ps, F.nz), v);
+        gx[k] = own ? da(gx[k], tx) : ds(gx[k], tx);
+        gy[k] = own ? da(gy[k], ty) : ds(gy[k], ty);
+        gz[k] = own ? da(gz[k], tz) : ds(gz[k], tz);
+      }
+    });
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const size_t q = (size_t)c * nc + k0 + k;
+      if (PAD) {
+        reinterpret_cast<D4*>(grad)[q] = {gx[k], gy[k], gz[k], 0.0};
       } else {
-        gx = ds(gx, tx); gy = ds(gy, ty); gz = ds(gz, tz);
+        grad[3 * q] = gx[k];
+        grad[3 * q + 1] = gy[k];
+        grad[3 * q + 2] = gz[k];
       }
     }
-    double* o = grad + ((size_t)c * nc + k) * 3;
-    o[0] = gx;
-    o[1] = gy;
-    o[2] = gz;
   }
 }
 
-__global__ void k_fv_recip(int n, const double* __restrict__ vol, double* __restrict__ vr) {
+__global__ void k_fv_recip(int n, const D4* __restrict__ cr, double* __restrict__ vr) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-    vr[c] = dd(1.0, vol[c]);  // cfd_grid.f90:546
+    vr[c] = dd(1.0, cr[c].w);  // cfd_grid.f90:546
 }
 
 // ---- explicit momentum terms: fvm_momentum_deferred ------------------------------------
@@ -272,78 +335,90 @@ __global__ void k_fv_recip(int n, const double* __restrict__ vol, double* __rest
 // the face value by `scheme` (0 central, 1 min-mod, 2 van Leer, 3 superbee
 // on the auxiliary-point values); then each cell adds +cor (owner) or
 // -cor (neighbour) of its faces in ascending face order.
+template <int NC>
 __global__ void k_fv_deferred_faces(Geo g, int nc, const double* __restrict__ phi,
                                     const double* __restrict__ grad,
                                     const double* __restrict__ flux, double mu, double c_bl,
                                     int scheme, double* __restrict__ cor) {
-  const long long tot = (long long)g.n_face * nc;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int f = (int)(t / nc), k = (int)(t % nc);
-    const int a = g.ip[f], b = g.in[f];
+  const int k0 = NC == 1 ? blockIdx.y : 0;
+  for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
+    const int2 ab = g.ab[f];
+    const int a = ab.x, b = ab.y;
     if (b < 0) {
-      cor[t] = 0.0;
+#pragma unroll
+      for (int k = 0; k < NC; ++k) cor[(size_t)f * nc + k0 + k] = 0.0;
       continue;
     }
-    const double w = g.w[f];
-    const Dx xa = aux_dx(g, f, a), xb = aux_dx(g, f, b);
-    const double c = flux[f], d = dd(dm(mu, g.s[f]), g.l[f]);
-    const double pa = phi[(size_t)a * nc + k], pb = phi[(size_t)b * nc + k];
-    const double* ga = grad + ((size_t)a * nc + k) * 3;
-    const double* gb = grad + ((size_t)b * nc + k) * 3;
-    const double pa_aux = da(pa, dot3(ga[0], ga[1], ga[2], xa.x, xa.y, xa.z));
-    const double pb_aux = da(pb, dot3(gb[0], gb[1], gb[2], xb.x, xb.y, xb.z));
-    double r_cor = 0.0;
-    if (c != 0.0) {
-      double pf;
-      if (scheme == 0) {
-        pf = lerp(w, pb_aux, pa_aux);
-      } else {
-        const bool fwd = c > 0.0;
-        const double pc = fwd ? pa_aux : pb_aux, pd = fwd ? pb_aux : pa_aux;
-        const double* gc = fwd ? ga : gb;
-        const double* xcA = g.xc + 3 * a;
-        const double* xcB = g.xc + 3 * b;
-        const double xpa[3] = {da(xcA[0], xa.x), da(xcA[1], xa.y), da(xcA[2], xa.z)};
-        const double xpb[3] = {da(xcB[0], xb.x), da(xcB[1], xb.y), da(xcB[2], xb.z)};
-        double dx[3];
-        for (int q = 0; q < 3; ++q) dx[q] = fwd ? ds(xpb[q], xpa[q]) : ds(xpa[q], xpb[q]);
-        const double pu = ds(pd, dm(2.0, dot3(gc[0], gc[1], gc[2], dx[0], dx[1], dx[2])));
-        double r = dd(ds(pc, pu), da(ds(pd, pc), 1e-20));
-        if (scheme == 1) {
-          r = smax(0.0, smin(1.0, r));
-        } else if (scheme == 2) {
-          r = dd(da(r, fabs(r)), da(da(1.0, fabs(r)), 1e-20));
-        } else {  // std::max({0, min(1, 2r), min(2, r)}): the first largest
-          double m = 0.0;
-          const double c1 = smin(1.0, dm(2.0, r)), c2 = smin(2.0, r);
-          if (m < c1) m = c1;
-          if (m < c2) m = c2;
-          r = m;
+    const Face F = face_of(g, f);
+    const Cell A = cell_of(g, a), B = cell_of(g, b);
+    const double w = F.w;
+    const Dx xa = aux_dx(F, A), xb = aux_dx(F, B);
+    const double c = flux[f], d = dd(dm(mu, F.s), g.l[f]);
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const size_t qa = (size_t)a * nc + k0 + k, qb = (size_t)b * nc + k0 + k;
+      const double pa = phi[qa], pb = phi[qb];
+      const double ga[3] = {grad[3 * qa], grad[3 * qa + 1], grad[3 * qa + 2]};
+      const double gb[3] = {grad[3 * qb], grad[3 * qb + 1], grad[3 * qb + 2]};
+      const double pa_aux = da(pa, dot3(ga[0], ga[1], ga[2], xa.x, xa.y, xa.z));
+      const double pb_aux = da(pb, dot3(gb[0], gb[1], gb[2], xb.x, xb.y, xb.z));
+      double r_cor = 0.0;
+      if (c != 0.0) {
+        double pf;
+        if (scheme == 0) {
+          pf = lerp(w, pb_aux, pa_aux);
+        } else {
+          const bool fwd = c > 0.0;
+          const double pc = fwd ? pa_aux : pb_aux, pd = fwd ? pb_aux : pa_aux;
+          const double xpa[3] = {da(A.x, xa.x), da(A.y, xa.y), da(A.z, xa.z)};
+          const double xpb[3] = {da(B.x, xb.x), da(B.y, xb.y), da(B.z, xb.z)};
+          double dx[3], gc[3];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            dx[q] = fwd ? ds(xpb[q], xpa[q]) : ds(xpa[q], xpb[q]);
+            gc[q] = fwd ? ga[q] : gb[q];
+          }
+          const double pu = ds(pd, dm(2.0, dot3(gc[0], gc[1], gc[2], dx[0], dx[1], dx[2])));
+          double r = dd(ds(pc, pu), da(ds(pd, pc), 1e-20));
+          if (scheme == 1) {
+            r = smax(0.0, smin(1.0, r));
+          } else if (scheme == 2) {
+            r = dd(da(r, fabs(r)), da(da(1.0, fabs(r)), 1e-20));
+          } else {  // std::max({0, min(1, 2r), min(2, r)}): the first largest
+            double m = 0.0;
+            const double c1 = smin(1.0, dm(2.0, r)), c2 = smin(2.0, r);
+            if (m < c1) m = c1;
+            if (m < c2) m = c2;
+            r = m;
+          }
+          pf = da(pc, dm(dm(0.5, r), ds(pd, pc)));
         }
-        pf = da(pc, dm(dm(0.5, r), ds(pd, pc)));
+        const double up = c > 0.0 ? pa : pb;
+        r_cor = dm(dm(c_bl, c), ds(up, pf));
       }
-      const double up = c > 0.0 ? pa : pb;
-      r_cor = dm(dm(c_bl, c), ds(up, pf));
+      cor[(size_t)f * nc + k0 + k] = da(r_cor, dm(d, ds(ds(pb_aux, pa_aux), ds(pb, pa))));
     }
-    cor[t] = da(r_cor, dm(d, ds(ds(pb_aux, pa_aux), ds(pb, pa))));
   }
 }
 
+template <int NC>
 __global__ void k_fv_deferred_cells(Geo g, int nc, const double* __restrict__ cor,
                                     double* __restrict__ rhs) {
-  const long long tot = (long long)g.n_cell * nc;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(t / nc), k = (int)(t % nc);
-    double acc = rhs[t];
-    for (int q = g.cf_ptr[c]; q < g.cf_ptr[c + 1]; ++q) {
-      const int f = g.cf[q];
-      if (g.in[f] < 0) continue;
-      const double x = cor[(size_t)f * nc + k];
-      acc = g.ip[f] == c ? da(acc, x) : ds(acc, x);
-    }
-    rhs[t] = acc;
+  const int k0 = NC == 1 ? blockIdx.y : 0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
+    double acc[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) acc[k] = rhs[(size_t)c * nc + k0 + k];
+    faces_of(g, c, [&](int f, bool own, int other) {
+      if (other < 0) return;
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        const double x = cor[(size_t)f * nc + k0 + k];
+        acc[k] = own ? da(acc[k], x) : ds(acc[k], x);
+      }
+    });
+#pragma unroll
+    for (int k = 0; k < NC; ++k) rhs[(size_t)c * nc + k0 + k] = acc[k];
   }
 }
 
@@ -352,29 +427,30 @@ __global__ void k_fv_face_flux(Geo g, const double* __restrict__ u, const double
                                const double* __restrict__ gp, const double* __restrict__ ap,
                                double rho, int aux, double* __restrict__ flux) {
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
-    const int a = g.ip[f], b = g.in[f];
+    const int2 ab = g.ab[f];
+    const int a = ab.x, b = ab.y;
     if (b < 0) {
       flux[f] = 0.0;
       continue;
     }
-    const double w = g.w[f];
-    const double* nn = g.nrm + 3 * f;
+    const Face F = face_of(g, f);
+    const Cell A = cell_of(g, a), B = cell_of(g, b);
+    const double w = F.w;
     const double ufx = lerp(w, u[3 * b], u[3 * a]), ufy = lerp(w, u[3 * b + 1], u[3 * a + 1]),
                  ufz = lerp(w, u[3 * b + 2], u[3 * a + 2]);
-    const double d = pc_coef(g, f, a, b, ap, rho);
+    const double d = pc_coef(w, F.s, g.l[f], B.vol, A.vol, ap[b], ap[a], rho);
     const double gx = lerp(w, gp[3 * b], gp[3 * a]), gy = lerp(w, gp[3 * b + 1], gp[3 * a + 1]),
                  gz = lerp(w, gp[3 * b + 2], gp[3 * a + 2]);
-    const double dx = ds(g.xc[3 * b], g.xc[3 * a]), dy = ds(g.xc[3 * b + 1], g.xc[3 * a + 1]),
-                 dz = ds(g.xc[3 * b + 2], g.xc[3 * a + 2]);
+    const double dx = ds(B.x, A.x), dy = ds(B.y, A.y), dz = ds(B.z, A.z);
     double pa = pr[a], pb = pr[b];
     if (aux) {  // cfd_setup.f90:611-614
-      const Dx xa = aux_dx(g, f, a), xb = aux_dx(g, f, b);
+      const Dx xa = aux_dx(F, A), xb = aux_dx(F, B);
       pa = da(pa, dot3(gp[3 * a], gp[3 * a + 1], gp[3 * a + 2], xa.x, xa.y, xa.z));
       pb = da(pb, dot3(gp[3 * b], gp[3 * b + 1], gp[3 * b + 2], xb.x, xb.y, xb.z));
     }
     const double dp = ds(ds(pb, pa), da(da(dm(gx, dx), dm(gy, dy)), dm(gz, dz)));
-    const double un = da(da(dm(ufx, nn[0]), dm(ufy, nn[1])), dm(ufz, nn[2]));
-    flux[f] = ds(dm(dm(rho, g.s[f]), un), dm(d, dp));
+    const double un = da(da(dm(ufx, F.nx), dm(ufy, F.ny)), dm(ufz, F.nz));
+    flux[f] = ds(dm(dm(rho, F.s), un), dm(d, dp));
   }
 }
 
@@ -385,11 +461,9 @@ __global__ void k_fv_imbalance(Geo g, const double* __restrict__ flux, int pc,
   double acc = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int q = g.cf_ptr[c]; q < g.cf_ptr[c + 1]; ++q) {
-      const int f = g.cf[q];
-      if (g.in[f] < 0) continue;
-      s = g.ip[f] == c ? ds(s, flux[f]) : da(s, flux[f]);
-    }
+    faces_of(g, c, [&](int f, bool own, int other) {
+      if (other >= 0) s = own ? ds(s, flux[f]) : da(s, flux[f]);
+    });
     if (c == pc) s = 0.0;
     bvec[c] = s;
     acc += fabs(s);
@@ -433,9 +507,12 @@ __global__ void k_fv_correct_faces(Geo g, const double* __restrict__ pp,
                                    const double* __restrict__ ap, double rho,
                                    double* __restrict__ flux) {
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
-    const int a = g.ip[f], b = g.in[f];
+    const int2 ab = g.ab[f];
+    const int a = ab.x, b = ab.y;
     if (b < 0) continue;
-    flux[f] = ds(flux[f], dm(pc_coef(g, f, a, b, ap, rho), ds(pp[b], pp[a])));
+    const double2 sw = g.sw[f];
+    const double d = pc_coef(sw.y, sw.x, g.l[f], g.vol[b], g.vol[a], ap[b], ap[a], rho);
+    flux[f] = ds(flux[f], dm(d, ds(pp[b], pp[a])));
   }
 }
 
@@ -451,7 +528,7 @@ struct fv_gpu {
   int dev = 0;
   cudaStream_t stream = nullptr;
   Geo g{};
-  DBuf ip, in, s, nrm, xf, l, w, xc, vol, vr, cf_ptr, cf, dface, part, total, tmp;
+  DBuf ab, fn, fc, cr, sw, l, vol, vr, cs_ptr, cs, dface, part, total, tmp;
   size_t tmp_bytes = 0;
 };
 
@@ -497,45 +574,63 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
   if (n_cell <= 0 || n_face < 0 || !ip || !in || !area || !nrm || !xf || !l_pn || !w_fp || !xc ||
       !vol)
     return SOLV_GPU_BAD_INPUT;
-  std::vector<int> a(n_face), b(n_face), cnt(n_cell + 1, 0);
+  std::vector<int2> ab(n_face);
+  std::vector<int> deg(n_cell, 0);
   for (int f = 0; f < n_face; ++f) {
-    a[f] = ip[f] - 1;
-    b[f] = in[f] - 1;
-    if (a[f] < 0 || a[f] >= n_cell || b[f] < -1 || b[f] >= n_cell || a[f] == b[f])
-      return SOLV_GPU_BAD_INPUT;
-    cnt[a[f] + 1]++;
-    if (b[f] >= 0) cnt[b[f] + 1]++;
+    const int a = ip[f] - 1, b = in[f] - 1;
+    if (a < 0 || a >= n_cell || b < -1 || b >= n_cell || a == b) return SOLV_GPU_BAD_INPUT;
+    ab[f] = make_int2(a, b);
+    deg[a]++;
+    if (b >= 0) deg[b]++;
   }
-  for (int c = 0; c < n_cell; ++c) cnt[c + 1] += cnt[c];
-  std::vector<int> cf(cnt[n_cell]);
-  std::vector<int> pos(cnt.begin(), cnt.end() - 1);
-  for (int f = 0; f < n_face; ++f) {  // ascending faces: each list comes out sorted
-    cf[pos[a[f]]++] = f;
-    if (b[f] >= 0) cf[pos[b[f]]++] = f;
+  const int ns = (n_cell + 31) / 32;
+  std::vector<int> cs_ptr(ns + 1, 0);
+  for (int s = 0; s < ns; ++s) {
+    int w = 0;
+    for (int c = s * 32; c < std::min(n_cell, s * 32 + 32); ++c) w = std::max(w, deg[c]);
+    const long long end = (long long)cs_ptr[s] + 32LL * w;
+    if (end > 0x7fffffffLL) return SOLV_GPU_BAD_INPUT;  // beyond int32 slot offsets
+    cs_ptr[s + 1] = (int)end;
   }
+  std::vector<int2> cs(cs_ptr[ns], make_int2(-1, -1));
+  std::vector<int> pos(n_cell, 0);
+  for (int f = 0; f < n_face; ++f) {  // ascending faces: each cell's slots come out sorted
+    auto put = [&](int c, int side, int other) {
+      cs[cs_ptr[c >> 5] + pos[c]++ * 32 + (c & 31)] = make_int2(2 * f + side, other);
+    };
+    put(ab[f].x, 0, ab[f].y);
+    if (ab[f].y >= 0) put(ab[f].y, 1, ab[f].x);
+  }
+  std::vector<D4> fn(n_face), fc(n_face), cr(n_cell);
+  std::vector<double2> sw(n_face);
+  for (size_t f = 0; f < (size_t)n_face; ++f) {
+    fn[f] = {nrm[3 * f], nrm[3 * f + 1], nrm[3 * f + 2], area[f]};
+    fc[f] = {xf[3 * f], xf[3 * f + 1], xf[3 * f + 2], w_fp[f]};
+    sw[f] = make_double2(area[f], w_fp[f]);
+  }
+  for (size_t c = 0; c < (size_t)n_cell; ++c)
+    cr[c] = {xc[3 * c], xc[3 * c + 1], xc[3 * c + 2], vol[c]};
   if (cudaSetDevice(device) != cudaSuccess) return SOLV_GPU_DEVICE_ERROR;
   fv_gpu* fv = new fv_gpu;
   fv->dev = device;
   const size_t F = n_face, N = n_cell;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-  chk(up(fv->ip, a.data(), F));
-  chk(up(fv->in, b.data(), F));
-  chk(up(fv->s, area, F));
-  chk(up(fv->nrm, nrm, 3 * F));
-  chk(up(fv->xf, xf, 3 * F));
+  chk(up(fv->ab, ab.data(), F));
+  chk(up(fv->fn, fn.data(), F));
+  chk(up(fv->fc, fc.data(), F));
+  chk(up(fv->cr, cr.data(), N));
+  chk(up(fv->sw, sw.data(), F));
   chk(up(fv->l, l_pn, F));
-  chk(up(fv->w, w_fp, F));
-  chk(up(fv->xc, xc, 3 * N));
   chk(up(fv->vol, vol, N));
-  chk(up(fv->cf_ptr, cnt.data(), N + 1));
-  chk(up(fv->cf, cf.data(), cf.size()));
+  chk(up(fv->cs_ptr, cs_ptr.data(), cs_ptr.size()));
+  chk(up(fv->cs, cs.data(), cs.size()));
   chk(cudaMalloc(&fv->dface.p, std::max<size_t>(F, 1) * sizeof(double)));
   chk(cudaMalloc(&fv->part.p, kRedBlocks * sizeof(double)));
   chk(cudaMalloc(&fv->total.p, sizeof(double)));
   chk(cudaMalloc(&fv->vr.p, std::max<size_t>(N, 1) * sizeof(double)));
   if (e == cudaSuccess) {
-    k_fv_recip<<<grid(n_cell), kBlock>>>(n_cell, fv->vol.as<double>(), fv->vr.as<double>());
+    k_fv_recip<<<grid(n_cell), kBlock>>>(n_cell, fv->cr.as<D4>(), fv->vr.as<double>());
     chk(cudaGetLastError());
     chk(cudaDeviceSynchronize());
   }
@@ -546,17 +641,15 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
   Geo& g = fv->g;
   g.n_cell = n_cell;
   g.n_face = n_face;
-  g.ip = fv->ip.as<int>();
-  g.in = fv->in.as<int>();
-  g.s = fv->s.as<double>();
-  g.nrm = fv->nrm.as<double>();
-  g.xf = fv->xf.as<double>();
-  g.l = fv->l.as<double>();
-  g.w = fv->w.as<double>();
-  g.xc = fv->xc.as<double>();
+  g.ab = fv->ab.as<int2>();
+  g.fn = fv->fn.as<D4>();
+  g.fc = fv->fc.as<D4>();
+  g.sw = fv->sw.as<double2>();
   g.vol = fv->vol.as<double>();
-  g.cf_ptr = fv->cf_ptr.as<int>();
-  g.cf = fv->cf.as<int>();
+  g.cr = fv->cr.as<D4>();
+  g.l = fv->l.as<double>();
+  g.cs_ptr = fv->cs_ptr.as<int>();
+  g.cs = fv->cs.as<int2>();
   *out = fv;
   return SOLV_GPU_OK;
 }
@@ -604,8 +697,10 @@ int fv_gpu_gradient(fv_gpu* fv, int ncomp, const double* phi, double* grad) {
   if (rc) return rc;
   if (ncomp < 1 || ncomp > 16 || !phi || !grad) return SOLV_GPU_BAD_INPUT;
   const Geo& g = fv->g;
-  k_fv_gradient<<<grid((long long)g.n_cell * ncomp), kBlock, 0, fv->stream>>>(g, ncomp, phi,
-                                                                              grad);
+  if (ncomp == 3)
+    k_fv_gradient<3><<<grid(g.n_cell), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad);
+  else
+    k_fv_gradient<1><<<dim3(grid(g.n_cell), ncomp), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad);
   return done();
 }
 
@@ -637,14 +732,19 @@ int fv_gpu_gradient_sweeps(fv_gpu* fv, int ncomp, const double* phi, const doubl
       neu > 2 || (neu == 0 && !bval))
     return SOLV_GPU_BAD_INPUT;
   const Geo& g = fv->g;
-  const size_t G = (size_t)3 * ncomp * g.n_cell;
-  double* t = scratch(fv, n_iter > 1 ? 2 * G * sizeof(double) : sizeof(double));
+  const size_t G = (size_t)4 * ncomp * g.n_cell;  // a sweep's gradients, in records of four
+  double* t = scratch(fv, n_iter > 1 ? std::min(n_iter - 1, 2) * G * sizeof(double) : sizeof(double));
   if (!t) return SOLV_GPU_DEVICE_ERROR;
   const double* g0 = nullptr;
   for (int it = 1; it <= n_iter; ++it) {
-    double* out = it == n_iter ? grad : t + ((it & 1) ? 0 : G);
-    k_fv_grad_sweep<<<grid((long long)g.n_cell * ncomp), kBlock, 0, fv->stream>>>(
-        g, ncomp, phi, bval, neu, fv->vr.as<double>(), g0, out);
+    const bool pad = it < n_iter;
+    double* out = pad ? t + ((it & 1) ? 0 : G) : grad;
+    auto kern = ncomp == 3 ? (!g0 ? (pad ? k_fv_grad_sweep<3, false, true> : k_fv_grad_sweep<3, false, false>)
+                                  : (pad ? k_fv_grad_sweep<3, true, true> : k_fv_grad_sweep<3, true, false>))
+                           : (!g0 ? (pad ? k_fv_grad_sweep<1, false, true> : k_fv_grad_sweep<1, false, false>)
+                                  : (pad ? k_fv_grad_sweep<1, true, true> : k_fv_grad_sweep<1, true, false>));
+    kern<<<dim3(grid(g.n_cell), ncomp == 3 ? 1 : ncomp), kBlock, 0, fv->stream>>>(
+        g, ncomp, phi, bval, neu, fv->vr.as<double>(), reinterpret_cast<const D4*>(g0), out);
     g0 = out;
   }
   return done();
@@ -660,10 +760,12 @@ int fv_gpu_momentum_deferred(fv_gpu* fv, int ncomp, const double* phi, const dou
   const Geo& g = fv->g;
   double* cor = scratch(fv, std::max<size_t>((size_t)g.n_face * ncomp, 1) * sizeof(double));
   if (!cor) return SOLV_GPU_DEVICE_ERROR;
-  k_fv_deferred_faces<<<grid((long long)g.n_face * ncomp), kBlock, 0, fv->stream>>>(
-      g, ncomp, phi, grad, flux, mu, c_bl, scheme, cor);
-  k_fv_deferred_cells<<<grid((long long)g.n_cell * ncomp), kBlock, 0, fv->stream>>>(g, ncomp, cor,
-                                                                                    rhs);
+  const int ny = ncomp == 3 ? 1 : ncomp;
+  auto faces = ncomp == 3 ? k_fv_deferred_faces<3> : k_fv_deferred_faces<1>;
+  auto cells = ncomp == 3 ? k_fv_deferred_cells<3> : k_fv_deferred_cells<1>;
+  faces<<<dim3(grid(g.n_face), ny), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad, flux, mu, c_bl,
+                                                             scheme, cor);
+  cells<<<dim3(grid(g.n_cell), ny), kBlock, 0, fv->stream>>>(g, ncomp, cor, rhs);
   return done();
 }
 
