@@ -512,34 +512,53 @@ __global__ void k_mg_pre(int n, sg::Rows<float> R, const float* __restrict__ din
 // The coarse levels' rows hold 17-27 slots, and from the second level on
 // there are too few rows to fill the SMs with one thread each, so G lanes
 // share a row: lane = part * (32/G) + row, so a load still reads 32/G
-// consecutive words per slot.  Returns sum_j a_ij (x(j) - xi) in every lane.
-template <int G, typename X>
+// consecutive words per slot.  Returns y + sum_j a_ij (x(j) - xi) in every
+// lane.  ORD keeps the sum slot by slot (values by shuffle), as in row_apply:
+// the training's loss gradient, a difference of nearly equal terms, moves by
+// 2e-5 when the V-cycle's rounding does, so its V-cycle keeps the order the
+// network was trained with; a solve takes the lanes' partial sums (V-cycle
+// at 64^3 86 us, ordered 101).
+template <int G, bool ORD, typename X>
 __device__ __forceinline__ float row_diff(const sg::Rows<float>& R, int i, int part, float xi,
-                                          X&& x) {
-  constexpr int CH = 4;
+                                          float y0, X&& x) {
+  constexpr int CH = 4, RW = 32 / G;
   sg::RowIt<float> it(R, i);
-  float y = 0.0f;
-  for (int k0 = part; k0 < it.w; k0 += CH * G) {
+  const int rl = (threadIdx.x & 31) % RW;
+  float y = ORD ? y0 : 0.0f;
+  for (int k0 = 0; k0 < it.w; k0 += CH * G) {  // w is the slice's, the same for the whole warp
     int j[CH];
-    float a[CH], xj[CH];
+    float a[CH], dx[CH];
 #pragma unroll
     for (int u = 0; u < CH; ++u) {
       j[u] = -1;
       a[u] = 0.0f;
-      if (k0 + u * G < it.w) {
-        const int e = it.base + (k0 + u * G) * sg::kWarp;
+      if (k0 + u * G + part < it.w) {
+        const int e = it.base + (k0 + u * G + part) * sg::kWarp;
         j[u] = __ldg(&R.col[e]);
         a[u] = __ldg(&R.val[e]);
       }
     }
 #pragma unroll
-    for (int u = 0; u < CH; ++u) xj[u] = j[u] >= 0 ? x(j[u]) : xi;
+    for (int u = 0; u < CH; ++u) dx[u] = (j[u] >= 0 ? x(j[u]) : xi) - xi;
 #pragma unroll
-    for (int u = 0; u < CH; ++u)
-      if (j[u] >= 0) y = fmaf(a[u], xj[u] - xi, y);
+    for (int u = 0; u < CH; ++u) {
+      if (!ORD) {
+        if (j[u] >= 0) y = fmaf(a[u], dx[u], y);
+        continue;
+      }
+      if (k0 + u * G >= it.w) break;
+      const float v = j[u] >= 0 ? a[u] : 0.0f;
+#pragma unroll
+      for (int q = 0; q < G; ++q)  // padding and slots past w add 0
+        y = fmaf(__shfl_sync(0xffffffffu, v, q * RW + rl),
+                 __shfl_sync(0xffffffffu, dx[u], q * RW + rl), y);
+    }
   }
+  if (!ORD) {
 #pragma unroll
-  for (int o = 16; o >= 32 / G; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    for (int o = 16; o >= RW; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    y = y0 + y;
+  }
   return y;
 }
 
@@ -557,6 +576,7 @@ __device__ __forceinline__ void rows_by_group(int n, int thread, int n_threads, 
 // kCoarseCells rows, 4 lanes a row.
 constexpr int kCoarseLanes = 4;
 constexpr int kCoarseCells = 100000;
+template <bool ORD>
 __global__ void k_mg_pre_coarse(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
                                 const float* __restrict__ b, float* __restrict__ x,
                                 float* __restrict__ t, const int* __restrict__ n_active) {
@@ -565,15 +585,15 @@ __global__ void k_mg_pre_coarse(int n, sg::Rows<float> R, const float* __restric
       n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
       [&](int i, int part, bool store) {
         const float bi = b[i], xi = w * dinv[i] * bi;
-        const float y = R.diag[i] * xi + row_diff<kCoarseLanes>(R, i, part, xi, [&](int j) {
-                          return w * dinv[j] * b[j];
-                        });
+        const float y = row_diff<kCoarseLanes, ORD>(R, i, part, xi, R.diag[i] * xi,
+                                               [&](int j) { return w * dinv[j] * b[j]; });
         if (store) {
           x[i] = xi;
           t[i] = bi - y;
         }
       });
 }
+template <bool ORD>
 __global__ void k_mg_post_coarse(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
                                  const float* __restrict__ b, const float* __restrict__ x,
                                  float* __restrict__ y, const int* __restrict__ n_active) {
@@ -582,8 +602,8 @@ __global__ void k_mg_post_coarse(int n, sg::Rows<float> R, const float* __restri
       n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
       [&](int i, int part, bool store) {
         const float xi = x[i];
-        const float ax = R.diag[i] * xi +
-                         row_diff<kCoarseLanes>(R, i, part, xi, [&](int j) { return x[j]; });
+        const float ax = row_diff<kCoarseLanes, ORD>(R, i, part, xi, R.diag[i] * xi,
+                                                [&](int j) { return x[j]; });
         if (store) y[i] = xi + w * dinv[i] * (b[i] - ax);
       });
 }
@@ -615,29 +635,30 @@ constexpr int kFuseCells = 6000;
 constexpr int kFuseThreads = 1024;
 constexpr int kFuseCluster = 16;
 
-template <int G>
+template <int G, bool ORD>
 __device__ __forceinline__ void fuse_pre(const FuseLevel& L, float w, int t, int nt) {
   rows_by_group<G>(L.n, t, nt, [&](int i, int part, bool store) {
     const float bi = __ldcg(&L.b[i]), xi = w * __ldg(&L.dinv[i]) * bi;
-    const float y = __ldg(&L.R.diag[i]) * xi + row_diff<G>(L.R, i, part, xi, [&](int j) {
-                      return w * __ldg(&L.dinv[j]) * __ldcg(&L.b[j]);
-                    });
+    const float y = row_diff<G, ORD>(L.R, i, part, xi, __ldg(&L.R.diag[i]) * xi, [&](int j) {
+      return w * __ldg(&L.dinv[j]) * __ldcg(&L.b[j]);
+    });
     if (store) {
       __stcg(&L.x[i], xi);
       __stcg(&L.t[i], bi - y);
     }
   });
 }
-template <int G>
+template <int G, bool ORD>
 __device__ __forceinline__ void fuse_post(const FuseLevel& L, float w, int t, int nt) {
   rows_by_group<G>(L.n, t, nt, [&](int i, int part, bool store) {
     const float xi = __ldcg(&L.x[i]);
-    const float ax = __ldg(&L.R.diag[i]) * xi +
-                     row_diff<G>(L.R, i, part, xi, [&](int j) { return __ldcg(&L.x[j]); });
+    const float ax = row_diff<G, ORD>(L.R, i, part, xi, __ldg(&L.R.diag[i]) * xi,
+                                 [&](int j) { return __ldcg(&L.x[j]); });
     if (store) __stcg(&L.y[i], xi + w * __ldg(&L.dinv[i]) * (__ldcg(&L.b[i]) - ax));
   });
 }
 
+template <bool ORD>
 __global__ void __launch_bounds__(kFuseThreads) k_mg_bottom(FuseArgs A, float w, float alpha,
                                                             const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;  // the same for every block
@@ -658,22 +679,33 @@ __global__ void __launch_bounds__(kFuseThreads) k_mg_bottom(FuseArgs A, float w,
     }
     cl.sync();
     if (l == last) break;
-    if (L.n * 2 > nt) fuse_pre<2>(L, w, t, nt);
-    else if (L.n * 8 > nt) fuse_pre<8>(L, w, t, nt);
-    else fuse_pre<16>(L, w, t, nt);
+    if (L.n * 2 > nt) fuse_pre<2, ORD>(L, w, t, nt);
+    else if (L.n * 8 > nt) fuse_pre<8, ORD>(L, w, t, nt);
+    else fuse_pre<16, ORD>(L, w, t, nt);
     cl.sync();
   }
   {  // x = Ainv b, a warp a row
     const FuseLevel& L = A.lv[last];
     for (int i = threadIdx.x; i < L.n; i += kFuseThreads) sb[i] = __ldcg(&L.b[i]);
     __syncthreads();
+    const int lane = threadIdx.x & 31;
     for (int i = t >> 5; i < L.n; i += nt >> 5) {
       float s = 0.0f;
-      for (int j = threadIdx.x & 31; j < L.n; j += 32)
-        s = fmaf(__ldg(&A.ainv[(size_t)i * L.n + j]), sb[j], s);
+      for (int j0 = 0; j0 < L.n; j0 += 32) {
+        const float a = j0 + lane < L.n ? __ldg(&A.ainv[(size_t)i * L.n + j0 + lane]) : 0.0f;
+        if (!ORD) {
+          if (j0 + lane < L.n) s = fmaf(a, sb[j0 + lane], s);
+          continue;
+        }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if ((threadIdx.x & 31) == 0) __stcg(&L.y[i], s);
+        for (int q = 0; q < 32; ++q)
+          if (j0 + q < L.n) s = fmaf(__shfl_sync(0xffffffffu, a, q), sb[j0 + q], s);
+      }
+      if (!ORD) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      }
+      if (lane == 0) __stcg(&L.y[i], s);
     }
   }
   for (int l = last - 1; l >= 0; --l) {
@@ -683,9 +715,9 @@ __global__ void __launch_bounds__(kFuseThreads) k_mg_bottom(FuseArgs A, float w,
     for (int i = t; i < L.n; i += nt)
       __stcg(&L.x[i], __ldcg(&L.x[i]) + alpha * __ldcg(&C.y[__ldg(&C.agg_of[i])]));
     cl.sync();
-    if (L.n * 2 > nt) fuse_post<2>(L, w, t, nt);
-    else if (L.n * 8 > nt) fuse_post<8>(L, w, t, nt);
-    else fuse_post<16>(L, w, t, nt);
+    if (L.n * 2 > nt) fuse_post<2, ORD>(L, w, t, nt);
+    else if (L.n * 8 > nt) fuse_post<8, ORD>(L, w, t, nt);
+    else fuse_post<16, ORD>(L, w, t, nt);
   }
 }
 

@@ -1023,8 +1023,10 @@ int mg_fuse_from(const solv_gpu_ctx* c) {
 int mg_bottom_blocks(solv_gpu_ctx* c) {
   if (c->mg_bottom_cs) return c->mg_bottom_cs;
   int n16 = 0;
-  if (cudaFuncSetAttribute(mg::k_mg_bottom, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-      cudaSuccess) {
+  if (cudaFuncSetAttribute(mg::k_mg_bottom<false>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                           1) == cudaSuccess &&
+      cudaFuncSetAttribute(mg::k_mg_bottom<true>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                           1) == cudaSuccess) {
     cudaLaunchConfig_t qc = {};
     qc.gridDim = dim3(mg::kFuseCluster);
     qc.blockDim = dim3(mg::kFuseThreads);
@@ -1035,7 +1037,7 @@ int mg_bottom_blocks(solv_gpu_ctx* c) {
     qa[0].val.clusterDim.z = 1;
     qc.attrs = qa;
     qc.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n16, mg::k_mg_bottom, &qc) != cudaSuccess) n16 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n16, mg::k_mg_bottom<true>, &qc) != cudaSuccess) n16 = 0;
   }
   cudaGetLastError();  // a refused query leaves the portable size
   c->mg_bottom_cs = n16 > 0 ? mg::kFuseCluster : 8;
@@ -1043,8 +1045,9 @@ int mg_bottom_blocks(solv_gpu_ctx* c) {
 }
 
 // The V-cycle below level 0: level 0's residual t0 in, level 1's correction
-// mg[0]->y out.  Returns the number of kernels launched.
-int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na) {
+// mg[0]->y out; ordered: the sums slot by slot (mg.cuh, row_diff).  Returns
+// the number of kernels launched.
+int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordered) {
   cudaStream_t s = c->stream;
   const int B = c->block;
   const float w = (float)c->mg_omega, a = (float)c->mg_alpha;
@@ -1055,7 +1058,8 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na) {
     mg::k_mg_restrict<<<grid_for(c, F.n), B, 0, s>>>(F.n, F.agg_ptr.as<int>(),
                                                      F.agg_cells.as<int>(), t, F.b.as<float>(), na);
     if (F.n <= mg::kCoarseCells)
-      mg::k_mg_pre_coarse<<<grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
+      (ordered ? mg::k_mg_pre_coarse<true> : mg::k_mg_pre_coarse<false>)<<<
+          grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
           F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.t.as<float>(),
           na);
     else
@@ -1076,14 +1080,16 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na) {
                     F.agg_of.as<int>(), F.x.as<float>(), F.b.as<float>(), F.t.as<float>(),
                     F.y.as<float>()};
   }
-  cluster_launch(c, mg::k_mg_bottom, mg_bottom_blocks(c), mg::kFuseThreads, A, w, a, na);
+  cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, mg_bottom_blocks(c),
+                 mg::kFuseThreads, A, w, a, na);
   for (int l = lf - 1; l >= 0; --l) {
     MgLevel& F = *c->mg[l];
     MgLevel& C = *c->mg[l + 1];
     mg::k_mg_prolong<<<grid_for(c, F.n), B, 0, s>>>(F.n, C.agg_of.as<int>(), a, C.y.as<float>(),
                                                     F.x.as<float>(), na);
     if (F.n <= mg::kCoarseCells)
-      mg::k_mg_post_coarse<<<grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
+      (ordered ? mg::k_mg_post_coarse<true> : mg::k_mg_post_coarse<false>)<<<
+          grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
           F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.y.as<float>(),
           na);
     else
@@ -1104,7 +1110,7 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na) {
 // kernels launched.
 template <typename TZ>
 int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, const float* ge,
-              float* x0, float* t0, const int* na) {
+              float* x0, float* t0, const int* na, bool ordered = false) {
   const bool net = mode == 1;
   cudaStream_t s = c->stream;
   const int B = c->block;
@@ -1128,7 +1134,7 @@ int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, 
     });
     k += 1;
   }
-  k += mg_coarse_cycle(c, t0, na);
+  k += mg_coarse_cycle(c, t0, na, ordered);
   mg::k_mg_prolong<<<grid_resident(c, N), B, 0, s>>>(N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0,
                                                 na);
   k += 1;
@@ -3592,7 +3598,7 @@ static int mg_train_sample(solv_gpu_ctx* c, float** B) {
                                             B[TB_DS], B[TB_ES]);
   };
   mg::k_mg_normalise<<<G, Bk, 0, s>>>(N, B[TB_RS], c->lanes.as<Lane>(), b);
-  mg_vcycle<float>(c, b, z, 1, q, ge, x0, t0, nullptr);  // t0 = b - A x before post-smoothing
+  mg_vcycle<float>(c, b, z, 1, q, ge, x0, t0, nullptr, true);  // t0 = b - A x before post-smoothing
   CUDA_TRY(c, cudaMemsetAsync(sums, 0, 2 * sizeof(double), s));
   mg::k_mg_loss_sums<<<G, 256, 0, s>>>(N, R0, z, b, az, sums);
   mg::k_mg_loss_grad<<<G, Bk, 0, s>>>(N, az, b, sums, gz, c->g_jsum.as<double>());
@@ -3603,7 +3609,7 @@ static int mg_train_sample(solv_gpu_ctx* c, float** B) {
   mg::k_mg_net<false, float><<<G, Bk, 0, s>>>(N, R0, ge, q, w, gz, nullptr, tmp, nullptr);
   mg::k_mg_resid<<<G, Bk, 0, s>>>(N, R0, gz, tmp, gx, nullptr);
   // through the coarse correction x += a P C P^T (b - A x): gx -= A (a P C P^T gx)
-  mg_coarse_cycle(c, gx, nullptr);
+  mg_coarse_cycle(c, gx, nullptr, true);
   CUDA_TRY(c, cudaMemsetAsync(tmp, 0, (size_t)N * sizeof(float), s));
   mg::k_mg_prolong<<<G, Bk, 0, s>>>(N, L1.agg_of.as<int>(), a, L1.y.as<float>(), tmp, nullptr);
   mg::k_mg_resid<<<G, Bk, 0, s>>>(N, R0, gx, tmp, az, nullptr);  // az = adjoint at x = w K b
