@@ -358,6 +358,7 @@ template <typename T>
 __global__ void k_gnn_apply(int n, sg::Rows<float> R, const float* __restrict__ gE,
                             const float* __restrict__ q, const T* __restrict__ r,
                             T* __restrict__ z, const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     sg::RowIt<float> it(R, i);

@@ -174,6 +174,17 @@ __device__ __forceinline__ void lane_stop(Lane& L, int status, int* n_active) {
   }
 }
 
+// The kernels of an iteration are launched as a chain of programmatic
+// dependents (chain_launch in solv_gpu.cu): the next one is set up while this
+// one drains, and waits here, before it touches anything, until the one before
+// is complete.  Every kernel of a chain has to wait, also one with nothing to
+// do: its completion stands for all before it.  (Letting the next one's blocks
+// start early as well, griddepcontrol.launch_dependents, cost 3-9% on systems
+// of 0.5-0.9M cells, where they came to stand in the way of blocks at work.)
+__device__ __forceinline__ void chain_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Kernels on the reduction grid (SegMap) are meant to run every block of the
 // grid at once: the grid holds at most 2048 threads per SM (blocks of at
 // most 256 threads), and the register budget of the one-component kernels
@@ -920,6 +931,7 @@ __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_
 template <typename T, int V>
 __global__ void k_jacobi(int n, const T* __restrict__ c, const T* __restrict__ bvec,
                          T* __restrict__ x) {
+  chain_enter();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const T ci = c[i];
 #pragma unroll
@@ -962,6 +974,7 @@ template <typename T, int V, bool JAC, bool FLEX = false>
 __global__ void SG_BOUNDS(V) k_cg_rz(SegMap sm, const T* __restrict__ c, const T* __restrict__ r,
                         const T* __restrict__ z, double* __restrict__ part,
                         Lane* __restrict__ lanes, const T* __restrict__ q = nullptr) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool any = false;
 #pragma unroll
@@ -1005,6 +1018,7 @@ template <typename T, int V, bool JAC, bool FLEX = false>
 __global__ void SG_BOUNDS(V) k_cg_p(SegMap sm, const T* __restrict__ c, const T* __restrict__ r,
                        const T* __restrict__ z, T* __restrict__ p,
                        Lane* __restrict__ lanes, double* __restrict__ part = nullptr) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool act[V];
   T beta[V];
@@ -1048,6 +1062,7 @@ __global__ void SG_BOUNDS(V) k_cg_p(SegMap sm, const T* __restrict__ c, const T*
 template <typename T, int V, int CH = kRowChunk>
 __global__ void SG_BOUNDS(V) k_cg_spmv(Rows<T> R, SegMap sm, const T* __restrict__ p, T* __restrict__ q,
                           double* __restrict__ part, Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool any = false;
 #pragma unroll
@@ -1088,6 +1103,7 @@ __global__ void SG_BOUNDS(V) k_cg_update(SegMap sm, const T* __restrict__ c, T* 
                             T* __restrict__ r, const T* __restrict__ p,
                             const T* __restrict__ q, double* __restrict__ part,
                             Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool act[V];
   T alpha[V];
@@ -1182,6 +1198,7 @@ template <typename T, int V, bool JAC>
 __global__ void SG_BOUNDS(V) k_bi_p(SegMap sm, const T* __restrict__ c, const T* __restrict__ r,
                        T* __restrict__ p, const T* __restrict__ u, T* __restrict__ z,
                        const Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool act[V];
   T om[V], al[V];
@@ -1215,6 +1232,7 @@ template <typename T, int V, int MODE, int CH = kRowChunk>
 __global__ void SG_BOUNDS(V) k_bi_spmv(Rows<T> R, SegMap sm, const T* __restrict__ z, T* __restrict__ y,
                           const T* __restrict__ w, double* __restrict__ part,
                           Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool any = false;
 #pragma unroll
@@ -1258,6 +1276,7 @@ template <typename T, int V, bool JAC>
 __global__ void SG_BOUNDS(V) k_bi_half(SegMap sm, const T* __restrict__ c, T* __restrict__ phi,
                           T* __restrict__ r, T* __restrict__ z, const T* __restrict__ u,
                           const Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool act[V];
   T g[V];
@@ -1291,6 +1310,7 @@ __global__ void SG_BOUNDS(V) k_bi_update(SegMap sm, T* __restrict__ phi, T* __re
                             const T* __restrict__ z, const T* __restrict__ vv,
                             const T* __restrict__ r0, double* __restrict__ part,
                             Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   bool act[V];
   T al[V];
@@ -1410,6 +1430,7 @@ __global__ void SG_BOUNDS(1) k_fcg_scale(SegMap sm, const T* __restrict__ r, con
 template <typename T>
 __global__ void SG_BOUNDS(1) k_fcg_beta(SegMap sm, const T* __restrict__ z, const T* __restrict__ q,
                            double* __restrict__ part, Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   if (!lanes[s].active) return;
   const int c0 = sm.seg_c0[s], c1 = sm.seg_c1[s];
@@ -1428,6 +1449,7 @@ template <typename T, int CH = kRowChunk>
 __global__ void SG_BOUNDS(1) k_fcg_spmv(Rows<T> R, SegMap sm, const T* __restrict__ p, T* __restrict__ q,
                            const T* __restrict__ r, double* __restrict__ part,
                            Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   if (!lanes[s].active) return;
   const int c0 = sm.seg_c0[s], c1 = sm.seg_c1[s];
@@ -1457,6 +1479,7 @@ template <typename T>
 __global__ void SG_BOUNDS(1) k_fcg_update(SegMap sm, T* __restrict__ phi, T* __restrict__ r,
                              const T* __restrict__ p, const T* __restrict__ q,
                              double* __restrict__ part, Lane* __restrict__ lanes) {
+  chain_enter();
   const int b = blockIdx.x, s = sm.blk_seg[b];
   if (!lanes[s].active) return;
   const T alpha = (T)lanes[s].alpha;
@@ -2735,6 +2758,7 @@ __global__ void k_near_slots(int n, Rows<double> R, unsigned long long* __restri
 // iteration, on until every lane has stopped or the budget is spent.
 __global__ void k_loop_ctl(cudaGraphConditionalHandle h, const int* __restrict__ n_active,
                            int* __restrict__ budget) {
+  chain_enter();
   if (threadIdx.x == 0) {
     const int b = *budget - 1;
     *budget = b;

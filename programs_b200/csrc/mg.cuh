@@ -479,6 +479,7 @@ template <int CH = sg::kRowChunk>
 __global__ void k_mg_pre(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
                          const float* __restrict__ b, float* __restrict__ x,
                          float* __restrict__ t, const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     sg::RowIt<float> it(R, i);
@@ -580,6 +581,7 @@ template <bool ORD>
 __global__ void k_mg_pre_coarse(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
                                 const float* __restrict__ b, float* __restrict__ x,
                                 float* __restrict__ t, const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   rows_by_group<kCoarseLanes>(
       n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
@@ -597,6 +599,7 @@ template <bool ORD>
 __global__ void k_mg_post_coarse(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
                                  const float* __restrict__ b, const float* __restrict__ x,
                                  float* __restrict__ y, const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   rows_by_group<kCoarseLanes>(
       n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
@@ -661,6 +664,7 @@ __device__ __forceinline__ void fuse_post(const FuseLevel& L, float w, int t, in
 template <bool ORD>
 __global__ void __launch_bounds__(kFuseThreads) k_mg_bottom(FuseArgs A, float w, float alpha,
                                                             const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;  // the same for every block
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -726,6 +730,7 @@ template <int CH = sg::kRowChunk>
 __global__ void k_mg_resid(int n, sg::Rows<float> R, const float* __restrict__ b,
                            const float* __restrict__ x, float* __restrict__ t,
                            const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float y[1];
@@ -739,6 +744,7 @@ template <typename TO, int CH = sg::kRowChunk>
 __global__ void k_mg_post(int n, sg::Rows<float> R, const float* __restrict__ dinv, float w,
                           const float* __restrict__ b, const float* __restrict__ x,
                           TO* __restrict__ y, const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float ax[1];
@@ -754,6 +760,7 @@ __global__ void k_mg_net(int n, sg::Rows<float> R, const float* __restrict__ gE,
                          const float* __restrict__ q, float w, const float* __restrict__ in,
                          const float* __restrict__ base, TO* __restrict__ out,
                          const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     sg::RowIt<float> it(R, i);
@@ -842,6 +849,7 @@ __global__ void k_mg_square(int n, const float* __restrict__ q, float* __restric
 __global__ void k_mg_restrict(int nc, const int* __restrict__ aptr,
                               const int* __restrict__ acell, const float* __restrict__ t,
                               float* __restrict__ bc, const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < nc; I += gridDim.x * blockDim.x) {
     float s = 0.0f;
@@ -854,6 +862,7 @@ __global__ void k_mg_restrict(int nc, const int* __restrict__ aptr,
 __global__ void k_mg_prolong(int n, const int* __restrict__ agg_of, float a,
                              const float* __restrict__ xc, float* __restrict__ x,
                              const int* __restrict__ n_active) {
+  sg::chain_enter();
   if (n_active && *n_active == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     x[i] += a * xc[agg_of[i]];

@@ -960,20 +960,41 @@ int mg_setup(solv_gpu_ctx* c) {
   return SOLV_GPU_OK;
 }
 
-// One thread-block cluster of cs blocks.
+// A kernel of an iteration's chain (kernels.cuh, chain_enter).  Launched on a
+// stream, a V-cycle at 64^3 (ten kernels) takes 66 us where it took 86; inside
+// a graph, whose launches are closer to begin with, the learned solve at 64^3
+// gains 4%, u, v, w momentum at 96^3 2.5%, large systems nothing.
 template <typename... KArgs, typename... Args>
-int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), int cs, int threads, Args... args) {
+void chain_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), int grid, int block, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, args...);  // a failure is the caller's cudaGetLastError()
+}
+
+// One thread-block cluster of cs blocks; chain: as chain_launch.
+template <typename... KArgs, typename... Args>
+int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), bool chain, int cs, int threads,
+                   Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)cs);
   cfg.blockDim = dim3((unsigned)threads);
   cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cs;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chain ? 2 : 1;
   CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, args...));
   return SOLV_GPU_OK;
 }
@@ -1002,7 +1023,7 @@ int mg_values(solv_gpu_ctx* c) {
   mg::k_mg_dense<<<(C.n + 31) / 32, 32, 0, s>>>(C.n, C.rows(), c->mg_dense.as<double>());
   if (C.n <= 128)
     mg::k_mg_invert<128, 1><<<1, 1024, 0, s>>>(C.n, c->mg_dense.as<double>(), c->mg_ainv.as<float>());
-  else if ((rc = cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, 8, 512, C.n,
+  else if ((rc = cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, false, 8, 512, C.n,
                                 (const double*)c->mg_dense.as<double>(), c->mg_ainv.as<float>())))
     return rc;
   c->launches += 2 + 3 * (int)c->mg.size() + 2;
@@ -1055,16 +1076,15 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
   const float* t = t0;
   for (int l = 0; l < lf; ++l) {
     MgLevel& F = *c->mg[l];
-    mg::k_mg_restrict<<<grid_for(c, F.n), B, 0, s>>>(F.n, F.agg_ptr.as<int>(),
+    chain_launch(c, mg::k_mg_restrict, grid_for(c, F.n), B, F.n, F.agg_ptr.as<int>(),
                                                      F.agg_cells.as<int>(), t, F.b.as<float>(), na);
     if (F.n <= mg::kCoarseCells)
-      (ordered ? mg::k_mg_pre_coarse<true> : mg::k_mg_pre_coarse<false>)<<<
-          grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
+      chain_launch(c, (ordered ? mg::k_mg_pre_coarse<true> : mg::k_mg_pre_coarse<false>), grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 
           F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.t.as<float>(),
           na);
     else
       with_chunk(c->row_chunk, [&](auto ch) {
-        mg::k_mg_pre<decltype(ch)::value><<<grid_for(c, F.n), B, 0, s>>>(
+        chain_launch(c, mg::k_mg_pre<decltype(ch)::value>, grid_for(c, F.n), B, 
             F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(),
             F.t.as<float>(), na);
       });
@@ -1080,21 +1100,20 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
                     F.agg_of.as<int>(), F.x.as<float>(), F.b.as<float>(), F.t.as<float>(),
                     F.y.as<float>()};
   }
-  cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, mg_bottom_blocks(c),
-                 mg::kFuseThreads, A, w, a, na);
+  cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, true,
+                 mg_bottom_blocks(c), mg::kFuseThreads, A, w, a, na);
   for (int l = lf - 1; l >= 0; --l) {
     MgLevel& F = *c->mg[l];
     MgLevel& C = *c->mg[l + 1];
-    mg::k_mg_prolong<<<grid_for(c, F.n), B, 0, s>>>(F.n, C.agg_of.as<int>(), a, C.y.as<float>(),
+    chain_launch(c, mg::k_mg_prolong, grid_for(c, F.n), B, F.n, C.agg_of.as<int>(), a, C.y.as<float>(),
                                                     F.x.as<float>(), na);
     if (F.n <= mg::kCoarseCells)
-      (ordered ? mg::k_mg_post_coarse<true> : mg::k_mg_post_coarse<false>)<<<
-          grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 0, s>>>(
+      chain_launch(c, (ordered ? mg::k_mg_post_coarse<true> : mg::k_mg_post_coarse<false>), grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 
           F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.y.as<float>(),
           na);
     else
       with_chunk(c->row_chunk, [&](auto ch) {
-        mg::k_mg_post<float, decltype(ch)::value><<<grid_for(c, F.n), B, 0, s>>>(
+        chain_launch(c, mg::k_mg_post<float, decltype(ch)::value>, grid_for(c, F.n), B, 
             F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(),
             F.y.as<float>(), na);
       });
@@ -1122,31 +1141,31 @@ int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, 
   int k = 0;
   const int ch = c->row_chunk;
   if (net) {
-    mg::k_mg_net<false, float><<<grid_resident(c, N), B, 0, s>>>(N, R0, ge, q, w, r, nullptr, x0, na);
+    chain_launch(c, mg::k_mg_net<false, float>, grid_resident(c, N), B, N, R0, ge, q, w, r, nullptr, x0, na);
     with_chunk(ch, [&](auto cc) {
-      mg::k_mg_resid<decltype(cc)::value><<<grid_resident(c, N), B, 0, s>>>(N, R0, r, x0, t0, na);
+      chain_launch(c, mg::k_mg_resid<decltype(cc)::value>, grid_resident(c, N), B, N, R0, r, x0, t0, na);
     });
     k += 2;
   } else {
     with_chunk(ch, [&](auto cc) {
-      mg::k_mg_pre<decltype(cc)::value><<<grid_resident(c, N), B, 0, s>>>(N, R0, d0, w, r, x0,
+      chain_launch(c, mg::k_mg_pre<decltype(cc)::value>, grid_resident(c, N), B, N, R0, d0, w, r, x0,
                                                                           t0, na);
     });
     k += 1;
   }
   k += mg_coarse_cycle(c, t0, na, ordered);
-  mg::k_mg_prolong<<<grid_resident(c, N), B, 0, s>>>(N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0,
+  chain_launch(c, mg::k_mg_prolong, grid_resident(c, N), B, N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0,
                                                 na);
   k += 1;
   if (net) {
     with_chunk(ch, [&](auto cc) {
-      mg::k_mg_resid<decltype(cc)::value><<<grid_resident(c, N), B, 0, s>>>(N, R0, r, x0, t0, na);
+      chain_launch(c, mg::k_mg_resid<decltype(cc)::value>, grid_resident(c, N), B, N, R0, r, x0, t0, na);
     });
-    mg::k_mg_net<true, TZ><<<grid_resident(c, N), B, 0, s>>>(N, R0, ge, q, w, t0, x0, z, na);
+    chain_launch(c, mg::k_mg_net<true, TZ>, grid_resident(c, N), B, N, R0, ge, q, w, t0, x0, z, na);
     k += 2;
   } else {
     with_chunk(ch, [&](auto cc) {
-      mg::k_mg_post<TZ, decltype(cc)::value><<<grid_resident(c, N), B, 0, s>>>(N, R0, d0, w, r,
+      chain_launch(c, mg::k_mg_post<TZ, decltype(cc)::value>, grid_resident(c, N), B, N, R0, d0, w, r,
                                                                                x0, z, na);
     });
     k += 1;
@@ -1328,7 +1347,7 @@ template <typename T, int V>
 int launch_direct(solv_gpu_ctx* c, int imat, const T* cc, const T* cr, T* x, const T* b,
                   const int* n_active) {
   if (imat <= 0) {
-    sg::k_jacobi<T, V><<<grid_for(c, c->N), c->block, 0, c->stream>>>(c->N, cc, b, x);
+    chain_launch(c, sg::k_jacobi<T, V>, grid_for(c, c->N), c->block, c->N, cc, b, x);
     c->launches++;
     return SOLV_GPU_OK;
   }
@@ -1398,11 +1417,11 @@ void cg_spmv(solv_gpu_ctx* c, const SegMap& sm, WS<T>& w, double* part, Lane* la
   const int G = c->seg.total_blk, B = c->block;
   if constexpr (std::is_same<T, float>::value) {
     with_chunk(c->row_chunk, [&](auto ch) {
-      sg::k_cg_spmv<T, V, decltype(ch)::value><<<G, B, 0, c->stream>>>(rows<T>(c), sm, w.p, w.q,
+      chain_launch(c, sg::k_cg_spmv<T, V, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q,
                                                                       part, lanes);
     });
   } else {
-    sg::k_cg_spmv<T, V><<<G, B, 0, c->stream>>>(rows<T>(c), sm, w.p, w.q, part, lanes);
+    chain_launch(c, sg::k_cg_spmv<T, V>, G, B, rows<T>(c), sm, w.p, w.q, part, lanes);
   }
 }
 
@@ -1413,11 +1432,11 @@ void bi_spmv(solv_gpu_ctx* c, const SegMap& sm, const T* z, T* y, const T* wv, d
   const int G = c->seg.total_blk, B = c->block;
   if constexpr (std::is_same<T, float>::value) {
     with_chunk(c->row_chunk, [&](auto ch) {
-      sg::k_bi_spmv<T, V, MODE, decltype(ch)::value><<<G, B, 0, c->stream>>>(rows<T>(c), sm, z, y,
+      chain_launch(c, sg::k_bi_spmv<T, V, MODE, decltype(ch)::value>, G, B, rows<T>(c), sm, z, y,
                                                                             wv, part, lanes);
     });
   } else {
-    sg::k_bi_spmv<T, V, MODE><<<G, B, 0, c->stream>>>(rows<T>(c), sm, z, y, wv, part, lanes);
+    chain_launch(c, sg::k_bi_spmv<T, V, MODE>, G, B, rows<T>(c), sm, z, y, wv, part, lanes);
   }
 }
 
@@ -1436,16 +1455,16 @@ int cg_iteration(solv_gpu_ctx* c, int imat, WS<T>& w) {
   cudaStream_t st = c->stream;
   if (imat > 0) {
     if (int rc = launch_direct<T, V>(c, imat, w.c, w.cr, w.z, w.r, sm.n_active)) return rc;
-    sg::k_cg_rz<T, V, false, FLEX><<<G, B, 0, st>>>(sm, w.c, w.r, w.z, part, lanes, w.q);
-    sg::k_cg_p<T, V, false, FLEX><<<G, B, 0, st>>>(sm, w.c, w.r, w.z, w.p, lanes, part);
+    chain_launch(c, sg::k_cg_rz<T, V, false, FLEX>, G, B, sm, w.c, w.r, w.z, part, lanes, w.q);
+    chain_launch(c, sg::k_cg_p<T, V, false, FLEX>, G, B, sm, w.c, w.r, w.z, w.p, lanes, part);
     cg_spmv<T, V>(c, sm, w, part, lanes);
-    sg::k_cg_update<T, V, false, FLEX><<<G, B, 0, st>>>(sm, w.c, w.phi, w.r, w.p, w.q, part,
+    chain_launch(c, sg::k_cg_update<T, V, false, FLEX>, G, B, sm, w.c, w.phi, w.r, w.p, w.q, part,
                                                         lanes);
     c->launches += 4;
   } else {
-    sg::k_cg_p<T, V, true, FLEX><<<G, B, 0, st>>>(sm, w.c, w.r, w.z, w.p, lanes, part);
+    chain_launch(c, sg::k_cg_p<T, V, true, FLEX>, G, B, sm, w.c, w.r, w.z, w.p, lanes, part);
     cg_spmv<T, V>(c, sm, w, part, lanes);
-    sg::k_cg_update<T, V, true, FLEX><<<G, B, 0, st>>>(sm, w.c, w.phi, w.r, w.p, w.q, part,
+    chain_launch(c, sg::k_cg_update<T, V, true, FLEX>, G, B, sm, w.c, w.phi, w.r, w.p, w.q, part,
                                                        lanes);
     c->launches += 3;
   }
@@ -1463,20 +1482,20 @@ int bicg_iteration(solv_gpu_ctx* c, int imat, WS<T>& w) {
   cudaStream_t st = c->stream;
   // w.q holds u, w.v holds v
   if (imat > 0) {
-    sg::k_bi_p<T, V, false><<<G, B, 0, st>>>(sm, w.c, w.r, w.p, w.q, w.z, lanes);
+    chain_launch(c, sg::k_bi_p<T, V, false>, G, B, sm, w.c, w.r, w.p, w.q, w.z, lanes);
     if (int rc = launch_direct<T, V>(c, imat, w.c, w.cr, w.z, w.p, sm.n_active)) return rc;
   } else {
-    sg::k_bi_p<T, V, true><<<G, B, 0, st>>>(sm, w.c, w.r, w.p, w.q, w.z, lanes);
+    chain_launch(c, sg::k_bi_p<T, V, true>, G, B, sm, w.c, w.r, w.p, w.q, w.z, lanes);
   }
   bi_spmv<T, V, 0>(c, sm, w.z, w.q, w.r0, part, lanes);
   if (imat > 0) {
-    sg::k_bi_half<T, V, false><<<G, B, 0, st>>>(sm, w.c, w.phi, w.r, w.z, w.q, lanes);
+    chain_launch(c, sg::k_bi_half<T, V, false>, G, B, sm, w.c, w.phi, w.r, w.z, w.q, lanes);
     if (int rc = launch_direct<T, V>(c, imat, w.c, w.cr, w.z, w.r, sm.n_active)) return rc;
   } else {
-    sg::k_bi_half<T, V, true><<<G, B, 0, st>>>(sm, w.c, w.phi, w.r, w.z, w.q, lanes);
+    chain_launch(c, sg::k_bi_half<T, V, true>, G, B, sm, w.c, w.phi, w.r, w.z, w.q, lanes);
   }
   bi_spmv<T, V, 1>(c, sm, w.z, w.v, w.r, part, lanes);
-  sg::k_bi_update<T, V><<<G, B, 0, st>>>(sm, w.phi, w.r, w.z, w.v, w.r0, part, lanes);
+  chain_launch(c, sg::k_bi_update<T, V>, G, B, sm, w.phi, w.r, w.z, w.v, w.r0, part, lanes);
   c->launches += 5;
   return SOLV_GPU_OK;
 }
@@ -1499,17 +1518,17 @@ void fcg_iteration(solv_gpu_ctx* c, WS<T>& w) {
                         sm.n_active);
   }
   if (!mg_on(c))
-    gnn::k_gnn_apply<T><<<grid_for(c, c->N), B, 0, st>>>(c->N, rows<float>(c),
+    chain_launch(c, gnn::k_gnn_apply<T>, grid_for(c, c->N), B, c->N, rows<float>(c),
                                                           c->g_ge.as<float>(), c->g_q.as<float>(),
                                                           w.r, w.z, sm.n_active);  // z = M^-1 r
   c->launches += nk - 1;
-  sg::k_fcg_beta<T><<<G, B, 0, st>>>(sm, w.z, w.q, part, lanes);            // beta
-  sg::k_cg_p<T, 1, false><<<G, B, 0, st>>>(sm, w.c, w.r, w.z, w.p, lanes);   // p = z + beta p
+  chain_launch(c, sg::k_fcg_beta<T>, G, B, sm, w.z, w.q, part, lanes);            // beta
+  chain_launch(c, sg::k_cg_p<T, 1, false>, G, B, sm, w.c, w.r, w.z, w.p, lanes, nullptr);   // p = z + beta p
   with_chunk(c->row_chunk, [&](auto ch) {
-    sg::k_fcg_spmv<T, decltype(ch)::value><<<G, B, 0, st>>>(rows<T>(c), sm, w.p, w.q, w.r, part,
+    chain_launch(c, sg::k_fcg_spmv<T, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q, w.r, part,
                                                             lanes);
   });
-  sg::k_fcg_update<T><<<G, B, 0, st>>>(sm, w.phi, w.r, w.p, w.q, part, lanes);
+  chain_launch(c, sg::k_fcg_update<T>, G, B, sm, w.phi, w.r, w.p, w.q, part, lanes);
   c->launches += 5;
 }
 
@@ -1548,7 +1567,7 @@ cudaError_t build_while_graph(solv_gpu_ctx* c, Body&& body, int& rc, cudaGraphEx
       if (e == cudaSuccess) {
         rc = body();
         if (!rc)
-          sg::k_loop_ctl<<<1, 32, 0, c->stream>>>(h, c->n_active.as<int>(),
+          chain_launch(c, sg::k_loop_ctl, 1, 32, h, c->n_active.as<int>(),
                                                   c->loop_budget.as<int>());
         cudaGraph_t out = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(c->stream, &out);
