@@ -1388,22 +1388,47 @@ __global__ void SG_BOUNDS(V) k_mp_flush(SegMap sm, const int* __restrict__ mask,
   }
 }
 
-// r_f = (float) r for the lanes in mask
+// The FP64 residual b - A x (solv_res.f90:12-29, k_res's operations) straight
+// into the FP32 one, r_f = (float)(b - A x), for the lanes in mask, and its L1
+// norm: one pass where a copy of b, the residual and the conversion took
+// three.
 template <int V>
-__global__ void SG_BOUNDS(V) k_mp_replace(SegMap sm, const int* __restrict__ mask, const double* __restrict__ r,
-                             float* __restrict__ rf) {
+__global__ void SG_BOUNDS(V) k_mp_res(Rows<double> R, SegMap sm, const int* __restrict__ mask,
+                         const double* __restrict__ bvec, const double* __restrict__ phi,
+                         float* __restrict__ rf, double* __restrict__ part,
+                         double* __restrict__ l1_out) {
   const int b = blockIdx.x, s = sm.blk_seg[b];
-  bool on[V];
-  bool any = false;
-#pragma unroll
-  for (int v = 0; v < V; ++v) { on[v] = mask[s * V + v] != 0; any |= on[v]; }
-  if (!any) return;
   const int c0 = sm.seg_c0[s], c1 = sm.seg_c1[s];
   const int stride = sm.seg_nblk[s] * blockDim.x;
+  double l1[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) l1[v] = 0.0;
   for (int i = c0 + sm.blk_rank[b] * blockDim.x + threadIdx.x; i < c1; i += stride) {
+    double y[V];
+    RowIt<double> it(R, i);
+    const double d = R.diag[i];
 #pragma unroll
     for (int v = 0; v < V; ++v)
-      if (on[v]) rf[(size_t)i * V + v] = (float)r[(size_t)i * V + v];
+      y[v] = sub(bvec[(size_t)i * V + v], mul(d, phi[(size_t)i * V + v]));
+    for (int k = 0; k < it.w; ++k) {
+      const int e = it.base + k * kWarp;
+      const int j = __ldg(&R.col[e]);
+      if (j >= 0) {
+        const double a = R.val[e];
+#pragma unroll
+        for (int v = 0; v < V; ++v) y[v] = sub(y[v], mul(a, phi[(size_t)j * V + v]));
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      if (mask[s * V + v]) rf[(size_t)i * V + v] = (float)y[v];
+      l1[v] += fabs(y[v]);
+    }
+  }
+  double tot[V];
+  if (seg_commit<V>(sm, b, s, part, l1, tot) && threadIdx.x == 0) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) l1_out[s * V + v] = tot[v];
   }
 }
 
@@ -1427,6 +1452,7 @@ __global__ void SG_BOUNDS(1) k_fcg_scale(SegMap sm, const T* __restrict__ r, con
     lanes[s].gs = tot[0] / (double)(c1 - c0);
 }
 
+// (for the one-level operator; the V-cycle's last kernel takes z.q itself)
 template <typename T>
 __global__ void SG_BOUNDS(1) k_fcg_beta(SegMap sm, const T* __restrict__ z, const T* __restrict__ q,
                            double* __restrict__ part, Lane* __restrict__ lanes) {

@@ -793,6 +793,65 @@ __global__ void k_mg_net(int n, sg::Rows<float> R, const float* __restrict__ gE,
   }
 }
 
+// The last kernel of a V-cycle inside flexible CG: z = x + w K t (NET, as
+// k_mg_net<true>) or z = x + w D^-1 (b - A x) (as k_mg_post), and beta =
+// -(z.q)/(p.q) with it, on the reduction grid -- k_fcg_beta's pass over z and
+// q and its reduction tail in a kernel of their own were 7.6 us of a 64^3
+// iteration.  in: t, or b; dq: q, or D^-1.
+template <bool NET, int CH>
+__global__ void SG_BOUNDS(1) k_mg_last(sg::SegMap sm, sg::Rows<float> R, const float* __restrict__ gE,
+                          const float* __restrict__ dq, float w, const float* __restrict__ in,
+                          const float* __restrict__ x, float* __restrict__ z,
+                          const float* __restrict__ qv, double* __restrict__ part,
+                          sg::Lane* __restrict__ lanes) {
+  sg::chain_enter();
+  const int b = blockIdx.x, s = sm.blk_seg[b];
+  if (!lanes[s].active) return;
+  const int c0 = sm.seg_c0[s], c1 = sm.seg_c1[s];
+  const int stride = sm.seg_nblk[s] * blockDim.x;
+  double acc[1] = {0.0};
+  for (int i = c0 + sm.blk_rank[b] * blockDim.x + threadIdx.x; i < c1; i += stride) {
+    float zi;
+    if (NET) {
+      sg::RowIt<float> it(R, i);
+      const float qi = dq[i];
+      float t = qi * in[i];
+      for (int k0 = 0; k0 < it.w; k0 += CH) {
+        int j[CH];
+        float g[CH], vj[CH];
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          j[u] = -1;
+          g[u] = 0.0f;
+          if (k0 + u < it.w) {
+            const int e = it.base + (k0 + u) * sg::kWarp;
+            j[u] = __ldg(&R.col[e]);
+            g[u] = gE[e];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          if (j[u] >= 0) g[u] *= dq[j[u]];
+          vj[u] = j[u] >= 0 ? in[j[u]] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < CH; ++u)
+          if (j[u] >= 0) t = fmaf(g[u], vj[u], t);
+      }
+      zi = x[i] + w * qi * t;
+    } else {
+      float ax[1];
+      sg::row_apply<float, 1, CH>(R, i, x, ax);
+      zi = x[i] + w * dq[i] * (in[i] - ax[0]);
+    }
+    z[i] = zi;
+    acc[0] += sg::prod(zi, qv[i]);
+  }
+  double tot[1];
+  if (sg::seg_commit<1>(sm, b, s, part, acc, tot) && threadIdx.x == 0)
+    lanes[s].beta = sg::flex_beta(lanes[s], tot[0], c1 - c0);
+}
+
 // ---- device: bounding the network smoother -----------------------------------------
 // v_i = a fixed pseudo-random value in [-1, 1) (power-iteration start)
 __global__ void k_mg_hashfill(int n, float* __restrict__ v) {
@@ -819,6 +878,58 @@ __global__ void __launch_bounds__(256) k_mg_norm2(int n, const float* __restrict
     double t = 0.0;
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += sh[k];
     atomicAdd(out, t);
+  }
+}
+
+// One step of the power iteration for lambda_max(w K A): v = (w / |v|) K y,
+// y = A v taken before, |v|^2 = norm2[0], the new |v|^2 added to norm2[1]
+// (zeroed before).  The norms stay on the device until the last step: the
+// scaling and the norm as passes of their own, with the host reading each
+// norm, were 250 us of a 64^3 solve.
+__global__ void __launch_bounds__(256)
+k_mg_power(int n, sg::Rows<float> R, const float* __restrict__ gE, const float* __restrict__ q,
+           float w, const float* __restrict__ y, float* __restrict__ v,
+           double* __restrict__ norm2) {
+  __shared__ double sh[8];
+  const float f = (float)(1.0 / sqrt(norm2[0]));
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    sg::RowIt<float> it(R, i);
+    const float qi = q[i];
+    float t = qi * y[i];
+    for (int k0 = 0; k0 < it.w; k0 += sg::kRowChunk) {
+      int j[sg::kRowChunk];
+      float g[sg::kRowChunk], yj[sg::kRowChunk];
+#pragma unroll
+      for (int u = 0; u < sg::kRowChunk; ++u) {
+        j[u] = -1;
+        g[u] = 0.0f;
+        if (k0 + u < it.w) {
+          const int e = it.base + (k0 + u) * sg::kWarp;
+          j[u] = __ldg(&R.col[e]);
+          g[u] = gE[e];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < sg::kRowChunk; ++u) {
+        if (j[u] >= 0) g[u] *= q[j[u]];
+        yj[u] = j[u] >= 0 ? y[j[u]] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < sg::kRowChunk; ++u)
+        if (j[u] >= 0) t = fmaf(g[u], yj[u], t);
+    }
+    const float x = f * (w * qi * t);
+    v[i] = x;
+    acc += (double)x * x;
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[k];
+    atomicAdd(&norm2[1], s);
   }
 }
 

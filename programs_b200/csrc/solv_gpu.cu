@@ -93,6 +93,8 @@ struct solv_gpu_ctx {
   int dev = 0;
   cudaStream_t own = nullptr;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;         // the coarsest inverse beside the main stream
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   std::string err;
   int n_sm = 148;
   // options
@@ -156,6 +158,7 @@ struct solv_gpu_ctx {
   // learned preconditioner (gnn.cuh)
   DevBuf g_param, g_grad, g_m, g_v, g_wcat;  // FP32 master, grads, Adam moments, BF16 packed
   DevBuf g_rsd, g_frs, g_fdeg, g_gw;         // per-matrix features
+  DevBuf g_norm2;                            // power iteration: |v|^2 of each step
   DevBuf g_h0, g_h1, g_u, g_r, g_out, g_jsum, g_q, g_he, g_ge;
   DevBuf g_train;                            // training activations
   bool g_feat_valid = false, g_wcat_valid = false, g_has_params = false;
@@ -980,12 +983,12 @@ void chain_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), int grid, int block, 
 
 // One thread-block cluster of cs blocks; chain: as chain_launch.
 template <typename... KArgs, typename... Args>
-int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), bool chain, int cs, int threads,
-                   Args... args) {
+int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), cudaStream_t stream, bool chain, int cs,
+                   int threads, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)cs);
   cfg.blockDim = dim3((unsigned)threads);
-  cfg.stream = c->stream;
+  cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cs;
@@ -1005,6 +1008,7 @@ int mg_values(solv_gpu_ctx* c) {
   int rc = ensure_f32_matrix(c);
   if (rc) return rc;
   cudaStream_t s = c->stream;
+  if (c->side) CUDA_TRY(c, cudaStreamWaitEvent(s, c->ev_join, 0));  // the inverse before
   const int B = c->block;
   mg::k_mg_dinv<<<grid_for(c, c->N), B, 0, s>>>(c->N, rows<float>(c), c->mg_dinv0.as<float>());
   const float* vprev = c->valf.as<float>();
@@ -1018,16 +1022,33 @@ int mg_values(solv_gpu_ctx* c) {
     vprev = L->val.as<float>();
     rsprev = L->rs.as<float>();
   }
+  // the coarsest inverse, a serial chain on one or eight SMs, beside what the
+  // stream does next (mg_join)
+  if (!c->side) {
+    CUDA_TRY(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+    CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+    CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+  }
+  CUDA_TRY(c, cudaEventRecord(c->ev_fork, s));
+  CUDA_TRY(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
   MgLevel& C = *c->mg.back();
-  CUDA_TRY(c, cudaMemsetAsync(c->mg_dense.p, 0, (size_t)C.n * C.n * sizeof(double), s));
-  mg::k_mg_dense<<<(C.n + 31) / 32, 32, 0, s>>>(C.n, C.rows(), c->mg_dense.as<double>());
+  CUDA_TRY(c, cudaMemsetAsync(c->mg_dense.p, 0, (size_t)C.n * C.n * sizeof(double), c->side));
+  mg::k_mg_dense<<<(C.n + 31) / 32, 32, 0, c->side>>>(C.n, C.rows(), c->mg_dense.as<double>());
   if (C.n <= 128)
-    mg::k_mg_invert<128, 1><<<1, 1024, 0, s>>>(C.n, c->mg_dense.as<double>(), c->mg_ainv.as<float>());
-  else if ((rc = cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, false, 8, 512, C.n,
+    mg::k_mg_invert<128, 1><<<1, 1024, 0, c->side>>>(C.n, c->mg_dense.as<double>(),
+                                                     c->mg_ainv.as<float>());
+  else if ((rc = cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, c->side, false, 8, 512, C.n,
                                 (const double*)c->mg_dense.as<double>(), c->mg_ainv.as<float>())))
     return rc;
+  CUDA_TRY(c, cudaEventRecord(c->ev_join, c->side));
   c->launches += 2 + 3 * (int)c->mg.size() + 2;
   CUDA_TRY(c, cudaGetLastError());
+  return SOLV_GPU_OK;
+}
+
+// The stream's further work waits for mg_values' inverse.
+int mg_join(solv_gpu_ctx* c) {
+  CUDA_TRY(c, cudaStreamWaitEvent(c->stream, c->ev_join, 0));
   return SOLV_GPU_OK;
 }
 
@@ -1100,7 +1121,7 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
                     F.agg_of.as<int>(), F.x.as<float>(), F.b.as<float>(), F.t.as<float>(),
                     F.y.as<float>()};
   }
-  cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, true,
+  cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, s, true,
                  mg_bottom_blocks(c), mg::kFuseThreads, A, w, a, na);
   for (int l = lf - 1; l >= 0; --l) {
     MgLevel& F = *c->mg[l];
@@ -1125,11 +1146,13 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
 // matrix).  Level 0 is smoothed by the network's operator (q, gE) for
 // mode 1, by Jacobi with the network's per-cell weights q^2 for mode 2 and
 // by damped Jacobi for mode 0.  x0 and t0 hold, afterwards, the level-0
-// iterate before post-smoothing and its residual.  Returns the number of
-// kernels launched.
+// iterate before post-smoothing and its residual.  beta_q: flexible CG's q,
+// for beta of the lane with the last kernel.  Returns the number of kernels
+// launched.
 template <typename TZ>
 int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, const float* ge,
-              float* x0, float* t0, const int* na, bool ordered = false) {
+              float* x0, float* t0, const int* na, bool ordered = false,
+              const float* beta_q = nullptr) {
   const bool net = mode == 1;
   cudaStream_t s = c->stream;
   const int B = c->block;
@@ -1157,17 +1180,28 @@ int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, 
   chain_launch(c, mg::k_mg_prolong, grid_resident(c, N), B, N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0,
                                                 na);
   k += 1;
+  auto last = [&](auto is_net, const float* dq, const float* in) {
+    if constexpr (std::is_same<TZ, float>::value)
+      with_chunk(decltype(is_net)::value ? sg::kRowChunk : ch, [&](auto cc) {
+        chain_launch(c, mg::k_mg_last<decltype(is_net)::value, decltype(cc)::value>,
+                     c->seg.total_blk, B, segmap(c), R0, ge, dq, w, in, x0, z, beta_q,
+                     c->part.as<double>(), c->lanes.as<Lane>());
+      });
+  };
   if (net) {
     with_chunk(ch, [&](auto cc) {
       chain_launch(c, mg::k_mg_resid<decltype(cc)::value>, grid_resident(c, N), B, N, R0, r, x0, t0, na);
     });
-    chain_launch(c, mg::k_mg_net<true, TZ>, grid_resident(c, N), B, N, R0, ge, q, w, t0, x0, z, na);
+    if (beta_q) last(std::true_type(), q, t0);
+    else chain_launch(c, mg::k_mg_net<true, TZ>, grid_resident(c, N), B, N, R0, ge, q, w, t0, x0, z, na);
     k += 2;
   } else {
-    with_chunk(ch, [&](auto cc) {
-      chain_launch(c, mg::k_mg_post<TZ, decltype(cc)::value>, grid_resident(c, N), B, N, R0, d0, w, r,
-                                                                               x0, z, na);
-    });
+    if (beta_q) last(std::false_type(), d0, r);
+    else
+      with_chunk(ch, [&](auto cc) {
+        chain_launch(c, mg::k_mg_post<TZ, decltype(cc)::value>, grid_resident(c, N), B, N, R0, d0, w,
+                     r, x0, z, na);
+      });
     k += 1;
   }
   return k;
@@ -1200,27 +1234,27 @@ int mg_bound_smoother(solv_gpu_ctx* c, double* applied) {
   Rows<float> R0 = rows<float>(c);
   float* v = c->mg_t0.as<float>();
   float* y = c->mg_x0.as<float>();
-  CUDA_TRY(c, c->g_jsum.ensure(3 * sizeof(double)));
-  double* acc = c->g_jsum.as<double>();
+  CUDA_TRY(c, c->g_norm2.ensure((kPowerIters + 1) * sizeof(double)));
+  double* norm2 = c->g_norm2.as<double>();
+  CUDA_TRY(c, cudaMemsetAsync(norm2, 0, (kPowerIters + 1) * sizeof(double), s));
   mg::k_mg_floor<<<G, B, 0, s>>>(N, c->mg_scale_min, c->g_rsd.as<float>(), c->g_q.as<float>());
   mg::k_mg_hashfill<<<G, B, 0, s>>>(N, v);
-  c->launches += 2;
-  double prev = 0.0, lam = 0.0, h = 0.0;
-  for (int it = 0; it <= kPowerIters; ++it) {
-    CUDA_TRY(c, cudaMemsetAsync(acc, 0, sizeof(double), s));
-    mg::k_mg_norm2<<<std::min(G, 1184), 256, 0, s>>>(N, v, acc);
-    CUDA_TRY(c, cudaMemcpyAsync(&h, acc, sizeof(double), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(c, cudaStreamSynchronize(s));
-    const double nrm = std::sqrt(h);
-    if (!(nrm > 0.0) || !std::isfinite(nrm)) break;
-    if (it > 0) lam = nrm / prev;  // |w K A v| / |v| for the previous, unit v
-    if (it == kPowerIters) break;
-    mg::k_mg_scale<<<G, B, 0, s>>>(N, (float)(1.0 / nrm), v);
-    prev = 1.0;
+  mg::k_mg_norm2<<<std::min(G, 1184), 256, 0, s>>>(N, v, norm2);
+  for (int it = 0; it < kPowerIters; ++it) {
     sg::k_spmv<float, 1><<<G, B, 0, s>>>(N, R0, v, y);  // y = A v
-    mg::k_mg_net<false, float><<<G, B, 0, s>>>(N, R0, c->g_ge.as<float>(), c->g_q.as<float>(),
-                                                (float)c->mg_omega, y, nullptr, v, nullptr);
-    c->launches += 4;
+    mg::k_mg_power<<<grid_resident(c, N), B, 0, s>>>(N, R0, c->g_ge.as<float>(),
+                                                     c->g_q.as<float>(), (float)c->mg_omega, y, v,
+                                                     norm2 + it);
+  }
+  c->launches += 3 + 2 * kPowerIters;
+  double h[kPowerIters + 1];
+  CUDA_TRY(c, cudaMemcpyAsync(h, norm2, sizeof(h), cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(c, cudaStreamSynchronize(s));
+  double lam = 0.0;  // |w K A v| / |v|, from the last step that stayed finite
+  for (int it = 0; it <= kPowerIters; ++it) {
+    const double nrm = std::sqrt(h[it]);
+    if (!(nrm > 0.0) || !std::isfinite(nrm)) break;
+    if (it > 0) lam = nrm;
   }
   CUDA_TRY(c, cudaGetLastError());
   lam *= 1.05;
@@ -1515,14 +1549,14 @@ void fcg_iteration(solv_gpu_ctx* c, WS<T>& w) {
     if (mg_on(c))  // z = V-cycle(r)
       nk = mg_vcycle<T>(c, w.r, w.z, c->mg_smoother, c->g_q.as<float>(),
                         c->g_ge.as<float>(), c->mg_x0.as<float>(), c->mg_t0.as<float>(),
-                        sm.n_active);
+                        sm.n_active, false, w.q) - 1;
   }
   if (!mg_on(c))
     chain_launch(c, gnn::k_gnn_apply<T>, grid_for(c, c->N), B, c->N, rows<float>(c),
                                                           c->g_ge.as<float>(), c->g_q.as<float>(),
                                                           w.r, w.z, sm.n_active);  // z = M^-1 r
   c->launches += nk - 1;
-  chain_launch(c, sg::k_fcg_beta<T>, G, B, sm, w.z, w.q, part, lanes);            // beta
+  if (!mg_on(c)) chain_launch(c, sg::k_fcg_beta<T>, G, B, sm, w.z, w.q, part, lanes);  // beta
   chain_launch(c, sg::k_cg_p<T, 1, false>, G, B, sm, w.c, w.r, w.z, w.p, lanes, nullptr);   // p = z + beta p
   with_chunk(c->row_chunk, [&](auto ch) {
     chain_launch(c, sg::k_fcg_spmv<T, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q, w.r, part,
@@ -1583,8 +1617,10 @@ cudaError_t build_while_graph(solv_gpu_ctx* c, Body&& body, int& rc, cudaGraphEx
 // Run Krylov iterations until every lane stops (device counter): one launch
 // of a WHILE graph where conditional nodes are available, else
 // `graph_iters` iterations per CUDA-graph launch.
+// lanes_out: also read the lanes back, with the counters.
 template <typename T, int V>
-int iterate(solv_gpu_ctx* c, int solver, int imat, int n_iter, WS<T>& w, int& graph_launches) {
+int iterate(solv_gpu_ctx* c, int solver, int imat, int n_iter, WS<T>& w, int& graph_launches,
+            std::vector<Lane>* lanes_out = nullptr) {
   const int K = c->graph_iters;
   auto body = [&]() -> int {
     if (solver == 0) return cg_iteration<T, V>(c, imat, w);
@@ -1658,7 +1694,7 @@ int iterate(solv_gpu_ctx* c, int solver, int imat, int n_iter, WS<T>& w, int& gr
     int sweep = imat > 0 ? 2 : 1;  // forward + backward recurrence, or Jacobi
     if (solver == 0) per_launch_kernels = imat > 0 ? sweep + 4 : 3;
     else if (solver == 1) per_launch_kernels = imat > 0 ? 2 * sweep + 5 : 5;
-    else per_launch_kernels = 4 + (mg_on(c) ? mg_kernels(c) : 1);
+    else per_launch_kernels = mg_on(c) ? 3 + mg_kernels(c) : 5;
     c->launches = l0;
   }
   while (done < n_iter) {
@@ -1682,6 +1718,9 @@ int iterate(solv_gpu_ctx* c, int solver, int imat, int n_iter, WS<T>& w, int& gr
     }
     CUDA_TRY(c, cudaGetLastError());
     CUDA_TRY(c, cudaMemcpyAsync(c->h_n_active, c->n_active.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (lanes_out)
+      CUDA_TRY(c, cudaMemcpyAsync(lanes_out->data(), c->lanes.p, lanes_out->size() * sizeof(Lane),
+                                  cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (loop) {
       const int ran = std::max(1, n_iter - done - c->h_n_active[1]);
@@ -2416,6 +2455,7 @@ int solve_mixed_reliable(solv_gpu_ctx* c, int solver, int imat, double reduc, in
   const int G = c->seg.total_blk, B = c->block;
   if (solver == 2) {  // the learned preconditioner of this solve, from r0
     if (c->mg_max_levels > 0 && (rc = mg_setup(c))) return rc;  // may build no levels
+    if (mg_on(c) && (rc = mg_values(c))) return rc;
     if (!mg_on(c) || c->mg_smoother >= 1) {
       if ((rc = gnn_prepare(c))) return rc;
       sg::k_fcg_scale<float><<<G, B, 0, s>>>(sm, f.r, c->g_rsd.as<float>(),
@@ -2427,12 +2467,12 @@ int solve_mixed_reliable(solv_gpu_ctx* c, int solver, int imat, double reduc, in
         c->launches++;
       }
     }
-    if (mg_on(c) && (rc = mg_values(c))) return rc;
     if (mg_on(c) && c->mg_smoother == 1) {
       double f = 1.0;
       if ((rc = mg_bound_smoother(c, &f))) return rc;
       c->mg_smooth_scale = f;
     }
+    if (mg_on(c) && (rc = mg_join(c))) return rc;
   } else if (imat <= 0) {
     sg::k_cg_rz<float, V, true><<<G, B, 0, s>>>(sm, f.c, f.r, f.z, c->part.as<double>(),
                                                 c->lanes.as<Lane>());
@@ -2492,11 +2532,9 @@ int solve_mixed_reliable(solv_gpu_ctx* c, int solver, int imat, double reduc, in
   const int K = std::max(1, c->graph_iters);
   while (na > 0) {
     int gl = 0;
-    if ((rc = iterate<float, V>(c, cur, imat_cur, K, f, gl))) return rc;  // K iterations at most
+    if ((rc = iterate<float, V>(c, cur, imat_cur, K, f, gl, &hl))) return rc;  // K iterations at most
     gl_total += gl;
     launched += K;
-    CUDA_TRY(c, cudaMemcpyAsync(hl.data(), c->lanes.p, nl * sizeof(Lane), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(c, cudaStreamSynchronize(s));
     bool need = false;
     fell_back = false;
     std::vector<char> trig(nl, 0);
@@ -2520,10 +2558,10 @@ int solve_mixed_reliable(solv_gpu_ctx* c, int solver, int imat, double reduc, in
     for (int l = 0; l < nl; ++l) mask[l] = !final_[l];
     CUDA_TRY(c, cudaMemcpyAsync(c->mp_mask.p, mask.data(), nl * sizeof(int), cudaMemcpyHostToDevice, s));
     sg::k_mp_flush<V><<<G, B, 0, s>>>(sm, c->mp_mask.as<int>(), w.phi, f.phi);
-    CUDA_TRY(c, cudaMemcpyAsync(w.r, b, NV * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if ((rc = run_res(c, V, w.phi, w.r, 0))) return rc;
-    sg::k_mp_replace<V><<<G, B, 0, s>>>(sm, c->mp_mask.as<int>(), w.r, f.r);
-    c->launches += 3;
+    sg::k_mp_res<V><<<G, B, 0, s>>>(rows<double>(c), sm, c->mp_mask.as<int>(), b, w.phi, f.r,
+                                    c->part.as<double>(), c->l1.as<double>());
+    CUDA_TRY(c, cudaGetLastError());
+    c->launches += 2;
     ++updates;
     CUDA_TRY(c, cudaMemcpyAsync(l1.data(), c->l1.p, nl * sizeof(double), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(c, cudaStreamSynchronize(s));
@@ -2769,6 +2807,12 @@ int solv_gpu_destroy(solv_gpu_ctx* c) {
   if (c->h_n_active) cudaFreeHost(c->h_n_active);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->side) {
+    cudaStreamSynchronize(c->side);
+    cudaStreamDestroy(c->side);
+  }
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+  if (c->ev_join) cudaEventDestroy(c->ev_join);
   cudaStream_t own = c->own;
   delete c;  // DevBufs free their memory
   if (own) cudaStreamDestroy(own);
@@ -3128,7 +3172,7 @@ int solv_gpu_kernel_time(solv_gpu_ctx* c, int which, int repeat, float* ms_per_l
       if (c->mg_max_levels <= 0) return set_err(c, SOLV_GPU_BAD_INPUT, "kernel_time: multigrid is off");
       if ((rc = mg_setup(c))) return rc;
       if (!mg_on(c)) return set_err(c, SOLV_GPU_BAD_INPUT, "kernel_time: no hierarchy for this matrix");
-      if ((rc = mg_values(c))) return rc;
+      if ((rc = mg_values(c)) || (rc = mg_join(c))) return rc;
     }
     if (which == 2 || (which == 3 && c->mg_smoother >= 1)) {
       if ((rc = gnn_prepare(c))) return rc;
@@ -3679,7 +3723,7 @@ int solv_gpu_gnn_grad_dev(solv_gpu_ctx* c, const double* r0_dev, const double* s
       CUDA_TRY(c, cudaMemsetAsync(c->g_zero.p, 0, std::max<long long>(c->n_slots, 1) * sizeof(float),
                                   c->stream));
     }
-    if ((rc = mg_values(c))) return rc;
+    if ((rc = mg_values(c)) || (rc = mg_join(c))) return rc;
     CUDA_TRY(c, c->mg_train.ensure((size_t)8 * N * sizeof(float)));
     k_gnn_mul<<<grid_for(c, N), c->block, 0, c->stream>>>(N, B[TB_S], c->g_rsd.as<float>(),
                                                            B[TB_Q]);
