@@ -89,7 +89,12 @@ extern "C" {
                                    launch; 2 (default): WHILE graphs for
                                    the learned flexible CG, whose lanes
                                    stop inside a graph for each reliable
-                                   update, fixed ones for CG and BiCGSTAB.
+                                   update, fixed ones for CG and BiCGSTAB;
+                                   FP64 CG and BiCGSTAB of small systems,
+                                   and FP64 Jacobi PCG that fits the SMs,
+                                   then run as one launch (0 and 1 keep
+                                   the graphs, as GRAPH_ITERS 0 does the
+                                   plain launches).
                                    Where the CUDA driver has no conditional
                                    graph nodes, 0 is used                  */
 #define SOLV_OPT_BLOCK 4        /* threads per block for the cell kernels
@@ -134,10 +139,11 @@ extern "C" {
                                    network makes them)                     */
 #define SOLV_OPT_PERSISTENT 19  /* FP64 Jacobi PCG (imat 0, n_vc 1, one
                                    system or a batch): 1 runs the whole
-                                   Krylov loop as one launch, a cluster of
-                                   8 thread blocks per system with the step
-                                   kernels fused (no host polls, no graph);
-                                   0 (default) the graph of step kernels   */
+                                   Krylov loop as one launch (no host
+                                   polls, no graph): over the SMs where the
+                                   matrix fits them, otherwise a cluster of
+                                   16 or 8 thread blocks per system;
+                                   0 (default) as GRAPH_LOOP says          */
 #define SOLV_OPT_VECTOR_WIDTH 18 /* FP32 matrix products (mixed-precision
                                    Krylov, flexible CG, V-cycle): matrix
                                    slots each thread loads before it sums
