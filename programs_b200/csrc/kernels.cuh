@@ -848,26 +848,32 @@ __global__ void k_precond_jacobi(int n, const double* __restrict__ diag, double*
   }
 }
 
-// slots per chunk: fewer for several components, which would spill
-template <int V> struct SweepChunk {
-  static constexpr int value = V <= 2 ? 8 : 6;
-};
-// Blocks per SM the sweeps' registers are held to: none where the levels'
-// latency counts, enough warps for bandwidth in an order of a few levels.
-template <int V, bool GATE> struct SweepBlocks {
-  static constexpr int value = GATE ? 1 : (V <= 2 ? 4 : 3);
+// Slots per chunk and blocks per SM (what the registers are held to) of the
+// sweeps.  In an order of many levels (GATE) a step's latency counts, not the
+// blocks; in one of a few levels bandwidth does, so as many warps as hold a
+// chunk of 6 slots, a hex row, without a spill: FP64 rows of two components
+// take 72 registers for it, of four 112.  With 8 slots in 64 and 6 in 80
+// registers they spilled 16-34 words a thread: BiCGSTAB + DILU in multicolour
+// order, ms at 72x73x71 and 100x101x99, two components 1.95 and 4.18, now 1.69
+// and 3.55 (8 slots at 3 blocks 1.71 and 3.65, 4 at 4 blocks 1.77 and 3.71);
+// four components 3.61 and 7.65, now 3.26 and 7.02 (4 slots at 3 blocks 3.44
+// and 7.05).
+template <typename T, int V, bool GATE> struct SweepShape {
+  static constexpr bool wide = sizeof(T) == 8 && !GATE;
+  static constexpr int chunk = V == 1 || (V == 2 && !wide) ? 8 : 6;
+  static constexpr int blocks = GATE ? 1 : V == 1 || (V == 2 && !wide) ? 4 : V == 4 && wide ? 2 : 3;
 };
 
 // solv_direct.f90:12-24 forward sweep, x_i = (b_i - sum_{j<i} n x_j) c_i, into
 // t (which starts out pending); the backward sweep's output x is reset to
 // pending on the way.
 template <typename T, int V, bool GATE>
-__global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_fwd_sf(
+__global__ void __launch_bounds__(kSweepThreads, (SweepShape<T, V, GATE>::blocks)) k_fwd_sf(
     int n, Rows<T> R, SweepMap sm, const T* __restrict__ c, const T* __restrict__ bvec, T* t, T* x,
     SweepCtl* ctl, const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;
   T acc[V], ci = T(0);
-  sweep_rows<false, GATE, SweepChunk<V>::value, V, T>(
+  sweep_rows<false, GATE, SweepShape<T, V, GATE>::chunk, V, T>(
       n, R, sm, t, ctl,
       [&](int i) {
         ci = __ldg(&c[i]);
@@ -896,12 +902,12 @@ __global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_
 // x_i = (t_i c_r_i - sum_{j>i} p x_j) c_i; x starts out pending, and each
 // t_i is reset to pending once read, ready for the next forward sweep.
 template <typename T, int V, bool GATE>
-__global__ void __launch_bounds__(kSweepThreads, SweepBlocks<V, GATE>::value) k_bwd_sf(
+__global__ void __launch_bounds__(kSweepThreads, (SweepShape<T, V, GATE>::blocks)) k_bwd_sf(
     int n, Rows<T> R, SweepMap sm, const T* __restrict__ c, const T* __restrict__ c_r, T* t, T* x,
     SweepCtl* ctl, const int* __restrict__ n_active) {
   if (n_active && *n_active == 0) return;
   T acc[V], ci = T(0);
-  sweep_rows<true, GATE, SweepChunk<V>::value, V, T>(
+  sweep_rows<true, GATE, SweepShape<T, V, GATE>::chunk, V, T>(
       n, R, sm, x, ctl,
       [&](int i) {
         ci = __ldg(&c[i]);
