@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/fv_gpu.h"
@@ -36,10 +37,10 @@ __device__ __forceinline__ double lerp(double w, double an, double ap) {
 // (unit normal and area; centre and weight), one per cell (centre and volume),
 // one per gradient carried from sweep to sweep.  As arrays of single values
 // the same visit took 18 requests.  The face kernels that need a few of these
-// values, in face order, read them as plain arrays (sw, vol).  A cell's faces stand in a sliced
-// ELL (32 cells a slice, slot-major, faces ascending) with the cell on the
-// face's other side beside them, so a warp reads consecutive words and the
-// neighbour's values need no trip through the face.
+// values, in face order, read them as plain arrays (sw, w, vol).  A cell's
+// faces stand in a sliced ELL (32 cells a slice, slot-major, faces ascending)
+// with the cell on the face's other side beside them, so a warp reads
+// consecutive words and the neighbour's values need no trip through the face.
 struct alignas(32) D4 {
   double x, y, z, w;
 };
@@ -56,7 +57,7 @@ struct Geo {
   const D4 *fn, *fc;           // per face {unit normal, area}; {centre, w_fp}
   const D4* cr;                // per cell {centre, volume}
   const double2* sw;           // per face {area, w_fp}
-  const double *l, *vol;       // l_pn; cell volumes
+  const double *l, *w, *vol;   // l_pn, w_fp; cell volumes
   const int* cs_ptr;           // first slot of each slice of 32 cells
   const int2* cs;              // slots: {2 face + (1 for the neighbour's side), other cell};
                                // {-1, -1} padding, other cell -1 on boundary faces
@@ -65,8 +66,12 @@ struct Geo {
 struct Face {
   double nx, ny, nz, s, x, y, z, w;
 };
+// CENTRE off: the centre is not needed, the weight comes without it
+template <bool CENTRE = true>
 __device__ __forceinline__ Face face_of(const Geo& g, int f) {
-  const D4 a = ld4(g.fn + f), b = ld4(g.fc + f);
+  const D4 a = ld4(g.fn + f);
+  if (!CENTRE) return {a.x, a.y, a.z, a.w, 0.0, 0.0, 0.0, g.w[f]};
+  const D4 b = ld4(g.fc + f);
   return {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
 struct Cell {
@@ -76,14 +81,44 @@ __device__ __forceinline__ Cell cell_of(const Geo& g, int c) {
   const D4 a = ld4(g.cr + c);
   return {a.x, a.y, a.z, a.w};
 }
+// A cell's slots, S at a time and before the faces are looked at: on a mesh
+// of a few thousand cells a kernel is one wave whose time is the chain of its
+// loads, and with a test for the list's end between them each slot waited for
+// the face before it (9x9x9, us: two sweeps 12.1, now 9.3; the imbalance's
+// sums 5.2, now 3.6).  S = 6, a hex cell's faces, where the registers allow.
+template <int S>
+__device__ __forceinline__ void slots_of(const Geo& g, int q, int e, int2 (&t)[S]) {
+#pragma unroll
+  for (int k = 0; k < S; ++k) t[k] = q + 32 * k < e ? g.cs[q + 32 * k] : make_int2(-1, -1);
+}
 // f(face, owner side, other cell) for the faces of cell c, ascending
-template <typename F>
+template <int S, typename F>
 __device__ __forceinline__ void faces_of(const Geo& g, int c, F&& f) {
   const int b = g.cs_ptr[c >> 5], e = g.cs_ptr[(c >> 5) + 1];
-  for (int q = b + (c & 31); q < e; q += 32) {
-    const int2 t = g.cs[q];
-    if (t.x < 0) break;  // padding only follows a cell's faces
-    f(t.x >> 1, (t.x & 1) == 0, t.y);
+  for (int q = b + (c & 31); q < e; q += 32 * S) {
+    int2 t[S];
+    slots_of(g, q, e, t);
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+      if (t[k].x >= 0) f(t[k].x >> 1, (t[k].x & 1) == 0, t[k].y);
+  }
+}
+// The same where a face gives a value or a few, load(face, owner side): the
+// chunk's are loaded side by side, then folded in by f(value, face, owner
+// side, other cell) in order.
+template <int S, typename L, typename F>
+__device__ __forceinline__ void fold_faces(const Geo& g, int c, L&& load, F&& f) {
+  const int b = g.cs_ptr[c >> 5], e = g.cs_ptr[(c >> 5) + 1];
+  for (int q = b + (c & 31); q < e; q += 32 * S) {
+    int2 t[S];
+    decltype(load(0, true)) v[S];
+    slots_of(g, q, e, t);
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+      if (t[k].x >= 0) v[k] = load(t[k].x >> 1, (t[k].x & 1) == 0);
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+      if (t[k].x >= 0) f(v[k], t[k].x >> 1, (t[k].x & 1) == 0, t[k].y);
   }
 }
 
@@ -109,6 +144,17 @@ __device__ __forceinline__ Dx aux_dx(const Face& F, const Cell& C) {
 constexpr int kBlock = 256;
 constexpr int kRedBlocks = 1024;
 
+// Above these many cells a vector field's components are one thread's work
+// (K = 3 of each()); below, a thread for each has the shorter chain.  us, one
+// thread a cell against three, in RCM order: two sweeps at 11.5k cells 17.3 /
+// 10.3, 28k 15.0 / 11.6, 64k 19.7 / 19.9, 125k 32.6 / 35.6, 942k 226 / 266;
+// deferred terms at 2.2k 5.6 / 5.2, 11.5k 5.9 / 5.9, 28k 7.2 / 8.8, 64k 10.4 /
+// 13.3; gradient at 64k 8.8 / 8.0, 238k 20.4 / 19.4, 512k 47.5 / 52.1
+// (unordered 80.6 / 65.4), 942k 76.6 / 87.2.
+constexpr int kSweepVector = 64000;
+constexpr int kDeferredVector = 16000;
+constexpr int kGradientVector = 600000;
+
 int grid(long long n) { return (int)std::max(1LL, std::min((n + kBlock - 1) / kBlock, 148LL * 16)); }
 
 // d = rho (1/a_P)_f area V_f / l_pn (cfd_setup.f90:604-634)
@@ -126,19 +172,19 @@ __global__ void k_fv_mom_faces(Geo g, const double* __restrict__ u, const double
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
     const int2 ab = g.ab[f];
     const int a = ab.x, b = ab.y;
-    const double2 sw = g.sw[f];
-    const double d = dd(dm(mu, sw.x), g.l[f]);
+    const D4 F = flux ? D4{0.0, 0.0, 0.0, g.sw[f].x} : ld4(g.fn + f);
+    const double d = dd(dm(mu, F.w), g.l[f]);
     if (b >= 0) {
       double c;
       if (flux) {
         c = flux[f];
       } else {
-        const D4 F = ld4(g.fn + f);
-        const double uf = lerp(sw.y, u[3 * b], u[3 * a]);
-        const double vf = lerp(sw.y, u[3 * b + 1], u[3 * a + 1]);
-        const double wf = lerp(sw.y, u[3 * b + 2], u[3 * a + 2]);
+        const double w = g.w[f];
+        const double uf = lerp(w, u[3 * b], u[3 * a]);
+        const double vf = lerp(w, u[3 * b + 1], u[3 * a + 1]);
+        const double wf = lerp(w, u[3 * b + 2], u[3 * a + 2]);
         const double un = da(da(dm(uf, F.x), dm(vf, F.y)), dm(wf, F.z));
-        c = dm(dm(rho, sw.x), un);
+        c = dm(dm(rho, F.w), un);
       }
       if (flux_out) flux_out[f] = c;
       const double mn = (0.0 < c) ? 0.0 : c;  // std::min(c, 0.0)
@@ -158,17 +204,19 @@ __global__ void k_fv_mom_cells(Geo g, const double* __restrict__ u, const double
                                double* __restrict__ pl, double* __restrict__ rhs) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
     double s = 0.0, rx = 0.0;
-    faces_of(g, c, [&](int f, bool own, int other) {
-      if (other < 0) {
-        const double d = -p[f];
-        s = da(s, d);
-        // the moving lid: the y = 1 wall (outward normal +y)
-        const Face F = face_of(g, f);
-        if (F.ny > 0.9 && F.y > 1.0 - 1e-9) rx = da(rx, dm(d, u_lid));
-      } else {
-        s = ds(s, own ? p[f] : n[f]);
-      }
-    });
+    fold_faces<6>(
+        g, c, [&](int f, bool own) { return own ? p[f] : n[f]; },
+        [&](double v, int f, bool, int other) {
+          if (other < 0) {
+            const double d = -v;
+            s = da(s, d);
+            // the moving lid: the y = 1 wall (outward normal +y)
+            const Face F = face_of(g, f);
+            if (F.ny > 0.9 && F.y > 1.0 - 1e-9) rx = da(rx, dm(d, u_lid));
+          } else {
+            s = ds(s, v);
+          }
+        });
     s = dd(s, urf);
     pl[c] = s;
     if (rhs) {
@@ -202,35 +250,55 @@ __global__ void k_fv_pc_faces(Geo g, const double* __restrict__ ap, double rho, 
 __global__ void k_fv_pc_cells(Geo g, const double* __restrict__ dface, double* __restrict__ pl) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
     double s = 0.0;
-    faces_of(g, c, [&](int f, bool, int other) {
-      if (other >= 0) s = da(s, dface[f]);
-    });
+    fold_faces<6>(
+        g, c, [&](int f, bool) { return dface[f]; },
+        [&](double d, int, bool, int other) {
+          if (other >= 0) s = da(s, d);
+        });
     pl[c] = s;
   }
 }
 
 // ---- Green-Gauss gradient -----------------------------------------------------------
-// The kernels over components come with NC = 3 (all the components of a
-// vector field in one thread: the geometry is read and the auxiliary points
-// are formed once) and NC = 1 (one component a thread, blockIdx.y of nc).
-template <int NC>
+// The kernels over components come in three forms: K = 1, a scalar; K = 3,
+// a vector field's components in one thread (the geometry is read and the
+// auxiliary points are formed once); K = 0, one of nc components a thread, a
+// cell's components in neighbouring lanes, which then read the geometry
+// together (apart, in blocks of their own, four components of an 80^3
+// gradient took 163 us; 66 like this).  each() gives a thread its cells (or
+// faces) i, the first of their M components that is its own, and M.
+template <int K, typename F>
+__device__ __forceinline__ void each(int n, int nc, F&& f) {
+  if constexpr (K != 0) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+      f(i, 0, K);
+  } else {
+    const long long tot = (long long)n * nc;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
+         t += (long long)gridDim.x * blockDim.x) {
+      const int i = tot <= 0xffffffffll ? (int)((unsigned)t / (unsigned)nc) : (int)(t / nc);
+      f(i, (int)(t - (long long)i * nc), nc);
+    }
+  }
+}
+template <int K>
 __global__ void k_fv_gradient(Geo g, int nc, const double* __restrict__ phi,
                               double* __restrict__ grad) {
-  const int k0 = NC == 1 ? blockIdx.y : 0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
+  constexpr int NC = K == 3 ? 3 : 1;
+  each<K>(g.n_cell, nc, [&](int c, int k0, int M) {
     double gx[NC], gy[NC], gz[NC], own_phi[NC];
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
       gx[k] = gy[k] = gz[k] = 0.0;
-      own_phi[k] = phi[(size_t)c * nc + k0 + k];
+      own_phi[k] = phi[(size_t)c * M + k0 + k];
     }
-    faces_of(g, c, [&](int f, bool own, int other) {
-      const Face F = face_of(g, f);
+    faces_of<6>(g, c, [&](int f, bool own, int other) {
+      const Face F = face_of<false>(g, f);
 #pragma unroll
       for (int k = 0; k < NC; ++k) {
         double pf = own_phi[k];
         if (other >= 0) {
-          const double po = phi[(size_t)other * nc + k0 + k];
+          const double po = phi[(size_t)other * M + k0 + k];
           pf = own ? lerp(F.w, po, pf) : lerp(F.w, pf, po);
         }
         const double ps = dm(pf, F.s);
@@ -243,12 +311,12 @@ __global__ void k_fv_gradient(Geo g, int nc, const double* __restrict__ phi,
     const double v = g.cr[c].w;
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      double* o = grad + ((size_t)c * nc + k0 + k) * 3;
+      double* o = grad + ((size_t)c * M + k0 + k) * 3;
       o[0] = dd(gx[k], v);
       o[1] = dd(gy[k], v);
       o[2] = dd(gz[k], v);
     }
-  }
+  });
 }
 
 // ---- solv_grad in full: corrected Green-Gauss sweeps ---------------------------------
@@ -258,26 +326,26 @@ __global__ void k_fv_gradient(Geo g, int nc, const double* __restrict__ phi,
 // of the face's cells in ascending face order, 1/V (vr) formed once per
 // cell.  bval[f*nc + k] are the wall values for neu = 0.  The gradients
 // between sweeps (g0, and grad where PAD) are records of four.
-template <int NC, bool CORR, bool PAD>
-__global__ void k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi,
-                                const double* __restrict__ bval, int neu,
-                                const double* __restrict__ vr, const D4* __restrict__ g0,
-                                double* __restrict__ grad) {
-  const int k0 = NC == 1 ? blockIdx.y : 0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
+template <int K, bool CORR, bool PAD>
+__global__ void __launch_bounds__(kBlock, !CORR || K == 1 ? 4 : K == 0 ? 3 : 2)
+k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi, const double* __restrict__ bval,
+                int neu, const double* __restrict__ vr, const D4* __restrict__ g0,
+                double* __restrict__ grad) {
+  constexpr int NC = K == 3 ? 3 : 1;
+  each<K>(g.n_cell, nc, [&](int c, int k0, int M) {
     double gx[NC], gy[NC], gz[NC], pc[NC];
     D4 gc[NC];
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      const size_t q = (size_t)c * nc + k0 + k;
+      const size_t q = (size_t)c * M + k0 + k;
       gx[k] = gy[k] = gz[k] = 0.0;
       pc[k] = phi[q];
       gc[k] = CORR ? ld4(g0 + q) : D4{};
     }
     const double v = vr[c];
-    const Cell C = cell_of(g, c);
-    faces_of(g, c, [&](int f, bool own, int other) {
-      const Face F = face_of(g, f);
+    const Cell C = CORR ? cell_of(g, c) : Cell{};
+    faces_of<K == 1 && CORR ? 3 : 6>(g, c, [&](int f, bool own, int other) {
+      const Face F = face_of<CORR>(g, f);
       Dx xc{}, xo{};  // this cell's auxiliary point and the other's
       if (CORR && other >= 0) {
         xc = aux_dx(F, C);
@@ -287,7 +355,7 @@ __global__ void k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi,
       for (int k = 0; k < NC; ++k) {
         double pf;
         if (other >= 0) {
-          const size_t q = (size_t)other * nc + k0 + k;
+          const size_t q = (size_t)other * M + k0 + k;
           double me = pc[k], po = phi[q];
           if (CORR) {
             const D4 go = ld4(g0 + q);
@@ -301,7 +369,7 @@ __global__ void k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi,
             pf = da(pf, dot3(gc[k].x, gc[k].y, gc[k].z, ds(F.x, C.x), ds(F.y, C.y),
                              ds(F.z, C.z)));
         } else {
-          pf = bval[(size_t)f * nc + k0 + k];
+          pf = bval[(size_t)f * M + k0 + k];
         }
         const double ps = dm(pf, F.s);
         const double tx = dm(dm(ps, F.nx), v), ty = dm(dm(ps, F.ny), v), tz = dm(dm(ps, F.nz), v);
@@ -312,7 +380,7 @@ __global__ void k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi,
     });
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      const size_t q = (size_t)c * nc + k0 + k;
+      const size_t q = (size_t)c * M + k0 + k;
       if (PAD) {
         reinterpret_cast<D4*>(grad)[q] = {gx[k], gy[k], gz[k], 0.0};
       } else {
@@ -321,7 +389,7 @@ __global__ void k_fv_grad_sweep(Geo g, int nc, const double* __restrict__ phi,
         grad[3 * q + 2] = gz[k];
       }
     }
-  }
+  });
 }
 
 __global__ void k_fv_recip(int n, const D4* __restrict__ cr, double* __restrict__ vr) {
@@ -335,19 +403,19 @@ __global__ void k_fv_recip(int n, const D4* __restrict__ cr, double* __restrict_
 // the face value by `scheme` (0 central, 1 min-mod, 2 van Leer, 3 superbee
 // on the auxiliary-point values); then each cell adds +cor (owner) or
 // -cor (neighbour) of its faces in ascending face order.
-template <int NC>
-__global__ void k_fv_deferred_faces(Geo g, int nc, const double* __restrict__ phi,
-                                    const double* __restrict__ grad,
-                                    const double* __restrict__ flux, double mu, double c_bl,
-                                    int scheme, double* __restrict__ cor) {
-  const int k0 = NC == 1 ? blockIdx.y : 0;
-  for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < g.n_face; f += gridDim.x * blockDim.x) {
+template <int K>
+__global__ void __launch_bounds__(kBlock, K == 3 ? 3 : 4)
+k_fv_deferred_faces(Geo g, int nc, const double* __restrict__ phi, const double* __restrict__ grad,
+                    const double* __restrict__ flux, double mu, double c_bl, int scheme,
+                    double* __restrict__ cor) {
+  constexpr int NC = K == 3 ? 3 : 1;
+  each<K>(g.n_face, nc, [&](int f, int k0, int M) {
     const int2 ab = g.ab[f];
     const int a = ab.x, b = ab.y;
     if (b < 0) {
 #pragma unroll
-      for (int k = 0; k < NC; ++k) cor[(size_t)f * nc + k0 + k] = 0.0;
-      continue;
+      for (int k = 0; k < NC; ++k) cor[(size_t)f * M + k0 + k] = 0.0;
+      return;
     }
     const Face F = face_of(g, f);
     const Cell A = cell_of(g, a), B = cell_of(g, b);
@@ -356,7 +424,7 @@ __global__ void k_fv_deferred_faces(Geo g, int nc, const double* __restrict__ ph
     const double c = flux[f], d = dd(dm(mu, F.s), g.l[f]);
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      const size_t qa = (size_t)a * nc + k0 + k, qb = (size_t)b * nc + k0 + k;
+      const size_t qa = (size_t)a * M + k0 + k, qb = (size_t)b * M + k0 + k;
       const double pa = phi[qa], pb = phi[qb];
       const double ga[3] = {grad[3 * qa], grad[3 * qa + 1], grad[3 * qa + 2]};
       const double gb[3] = {grad[3 * qb], grad[3 * qb + 1], grad[3 * qb + 2]};
@@ -396,30 +464,38 @@ __global__ void k_fv_deferred_faces(Geo g, int nc, const double* __restrict__ ph
         const double up = c > 0.0 ? pa : pb;
         r_cor = dm(dm(c_bl, c), ds(up, pf));
       }
-      cor[(size_t)f * nc + k0 + k] = da(r_cor, dm(d, ds(ds(pb_aux, pa_aux), ds(pb, pa))));
+      cor[(size_t)f * M + k0 + k] = da(r_cor, dm(d, ds(ds(pb_aux, pa_aux), ds(pb, pa))));
     }
-  }
+  });
 }
 
-template <int NC>
-__global__ void k_fv_deferred_cells(Geo g, int nc, const double* __restrict__ cor,
-                                    double* __restrict__ rhs) {
-  const int k0 = NC == 1 ? blockIdx.y : 0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
+template <int K>
+__global__ void __launch_bounds__(kBlock, K == 3 ? 3 : 4)
+k_fv_deferred_cells(Geo g, int nc, const double* __restrict__ cor, double* __restrict__ rhs) {
+  constexpr int NC = K == 3 ? 3 : 1;
+  struct Cor {
+    double x[NC];
+  };
+  each<K>(g.n_cell, nc, [&](int c, int k0, int M) {
     double acc[NC];
 #pragma unroll
-    for (int k = 0; k < NC; ++k) acc[k] = rhs[(size_t)c * nc + k0 + k];
-    faces_of(g, c, [&](int f, bool own, int other) {
-      if (other < 0) return;
+    for (int k = 0; k < NC; ++k) acc[k] = rhs[(size_t)c * M + k0 + k];
+    fold_faces<6>(
+        g, c,
+        [&](int f, bool) {
+          Cor v;
 #pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        const double x = cor[(size_t)f * nc + k0 + k];
-        acc[k] = own ? da(acc[k], x) : ds(acc[k], x);
-      }
-    });
+          for (int k = 0; k < NC; ++k) v.x[k] = cor[(size_t)f * M + k0 + k];
+          return v;
+        },
+        [&](const Cor& v, int, bool own, int other) {
+          if (other < 0) return;
 #pragma unroll
-    for (int k = 0; k < NC; ++k) rhs[(size_t)c * nc + k0 + k] = acc[k];
-  }
+          for (int k = 0; k < NC; ++k) acc[k] = own ? da(acc[k], v.x[k]) : ds(acc[k], v.x[k]);
+        });
+#pragma unroll
+    for (int k = 0; k < NC; ++k) rhs[(size_t)c * M + k0 + k] = acc[k];
+  });
 }
 
 // ---- Rhie-Chow face fluxes ------------------------------------------------------------
@@ -461,9 +537,11 @@ __global__ void k_fv_imbalance(Geo g, const double* __restrict__ flux, int pc,
   double acc = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.n_cell; c += gridDim.x * blockDim.x) {
     double s = 0.0;
-    faces_of(g, c, [&](int f, bool own, int other) {
-      if (other >= 0) s = own ? ds(s, flux[f]) : da(s, flux[f]);
-    });
+    fold_faces<6>(
+        g, c, [&](int f, bool) { return flux[f]; },
+        [&](double d, int, bool own, int other) {
+          if (other >= 0) s = own ? ds(s, d) : da(s, d);
+        });
     if (c == pc) s = 0.0;
     bvec[c] = s;
     acc += fabs(s);
@@ -528,7 +606,7 @@ struct fv_gpu {
   int dev = 0;
   cudaStream_t stream = nullptr;
   Geo g{};
-  DBuf ab, fn, fc, cr, sw, l, vol, vr, cs_ptr, cs, dface, part, total, tmp;
+  DBuf ab, fn, fc, cr, sw, l, w, vol, vr, cs_ptr, cs, dface, part, total, tmp;
   size_t tmp_bytes = 0;
 };
 
@@ -556,6 +634,22 @@ double* scratch(fv_gpu* fv, size_t bytes) {
 int enter(fv_gpu* fv) {
   if (!fv) return SOLV_GPU_BAD_INPUT;
   return cudaSetDevice(fv->dev) == cudaSuccess ? SOLV_GPU_OK : SOLV_GPU_DEVICE_ERROR;
+}
+
+// f(the form of the component kernels for this call: each(), kSweepVector)
+template <typename F>
+void with_form(const Geo& g, int ncomp, int vector_cells, F&& f) {
+  if (ncomp == 1)
+    f(std::integral_constant<int, 1>());
+  else if (ncomp == 3 && g.n_cell > vector_cells)
+    f(std::integral_constant<int, 3>());
+  else
+    f(std::integral_constant<int, 0>());
+}
+// Blocks for n cells or faces in form K
+template <int K>
+int grid_of(int n, int ncomp) {
+  return grid(K == 0 ? (long long)n * ncomp : n);
 }
 
 int done() {
@@ -622,6 +716,7 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
   chk(up(fv->cr, cr.data(), N));
   chk(up(fv->sw, sw.data(), F));
   chk(up(fv->l, l_pn, F));
+  chk(up(fv->w, w_fp, F));
   chk(up(fv->vol, vol, N));
   chk(up(fv->cs_ptr, cs_ptr.data(), cs_ptr.size()));
   chk(up(fv->cs, cs.data(), cs.size()));
@@ -648,6 +743,7 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
   g.vol = fv->vol.as<double>();
   g.cr = fv->cr.as<D4>();
   g.l = fv->l.as<double>();
+  g.w = fv->w.as<double>();
   g.cs_ptr = fv->cs_ptr.as<int>();
   g.cs = fv->cs.as<int2>();
   *out = fv;
@@ -697,10 +793,10 @@ int fv_gpu_gradient(fv_gpu* fv, int ncomp, const double* phi, double* grad) {
   if (rc) return rc;
   if (ncomp < 1 || ncomp > 16 || !phi || !grad) return SOLV_GPU_BAD_INPUT;
   const Geo& g = fv->g;
-  if (ncomp == 3)
-    k_fv_gradient<3><<<grid(g.n_cell), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad);
-  else
-    k_fv_gradient<1><<<dim3(grid(g.n_cell), ncomp), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad);
+  with_form(g, ncomp, kGradientVector, [&](auto form) {
+    constexpr int K = decltype(form)::value;
+    k_fv_gradient<K><<<grid_of<K>(g.n_cell, ncomp), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad);
+  });
   return done();
 }
 
@@ -733,18 +829,19 @@ int fv_gpu_gradient_sweeps(fv_gpu* fv, int ncomp, const double* phi, const doubl
     return SOLV_GPU_BAD_INPUT;
   const Geo& g = fv->g;
   const size_t G = (size_t)4 * ncomp * g.n_cell;  // a sweep's gradients, in records of four
-  double* t = scratch(fv, n_iter > 1 ? std::min(n_iter - 1, 2) * G * sizeof(double) : sizeof(double));
+  double* t = scratch(fv, std::max<size_t>(std::min(n_iter - 1, 2) * G, 1) * sizeof(double));
   if (!t) return SOLV_GPU_DEVICE_ERROR;
   const double* g0 = nullptr;
   for (int it = 1; it <= n_iter; ++it) {
     const bool pad = it < n_iter;
     double* out = pad ? t + ((it & 1) ? 0 : G) : grad;
-    auto kern = ncomp == 3 ? (!g0 ? (pad ? k_fv_grad_sweep<3, false, true> : k_fv_grad_sweep<3, false, false>)
-                                  : (pad ? k_fv_grad_sweep<3, true, true> : k_fv_grad_sweep<3, true, false>))
-                           : (!g0 ? (pad ? k_fv_grad_sweep<1, false, true> : k_fv_grad_sweep<1, false, false>)
-                                  : (pad ? k_fv_grad_sweep<1, true, true> : k_fv_grad_sweep<1, true, false>));
-    kern<<<dim3(grid(g.n_cell), ncomp == 3 ? 1 : ncomp), kBlock, 0, fv->stream>>>(
-        g, ncomp, phi, bval, neu, fv->vr.as<double>(), reinterpret_cast<const D4*>(g0), out);
+    with_form(g, ncomp, kSweepVector, [&](auto form) {
+      constexpr int K = decltype(form)::value;
+      auto kern = !g0 ? (pad ? k_fv_grad_sweep<K, false, true> : k_fv_grad_sweep<K, false, false>)
+                      : (pad ? k_fv_grad_sweep<K, true, true> : k_fv_grad_sweep<K, true, false>);
+      kern<<<grid_of<K>(g.n_cell, ncomp), kBlock, 0, fv->stream>>>(
+          g, ncomp, phi, bval, neu, fv->vr.as<double>(), reinterpret_cast<const D4*>(g0), out);
+    });
     g0 = out;
   }
   return done();
@@ -760,12 +857,13 @@ int fv_gpu_momentum_deferred(fv_gpu* fv, int ncomp, const double* phi, const dou
   const Geo& g = fv->g;
   double* cor = scratch(fv, std::max<size_t>((size_t)g.n_face * ncomp, 1) * sizeof(double));
   if (!cor) return SOLV_GPU_DEVICE_ERROR;
-  const int ny = ncomp == 3 ? 1 : ncomp;
-  auto faces = ncomp == 3 ? k_fv_deferred_faces<3> : k_fv_deferred_faces<1>;
-  auto cells = ncomp == 3 ? k_fv_deferred_cells<3> : k_fv_deferred_cells<1>;
-  faces<<<dim3(grid(g.n_face), ny), kBlock, 0, fv->stream>>>(g, ncomp, phi, grad, flux, mu, c_bl,
-                                                             scheme, cor);
-  cells<<<dim3(grid(g.n_cell), ny), kBlock, 0, fv->stream>>>(g, ncomp, cor, rhs);
+  with_form(g, ncomp, kDeferredVector, [&](auto form) {
+    constexpr int K = decltype(form)::value;
+    k_fv_deferred_faces<K><<<grid_of<K>(g.n_face, ncomp), kBlock, 0, fv->stream>>>(
+        g, ncomp, phi, grad, flux, mu, c_bl, scheme, cor);
+    k_fv_deferred_cells<K><<<grid_of<K>(g.n_cell, ncomp), kBlock, 0, fv->stream>>>(g, ncomp, cor,
+                                                                                  rhs);
+  });
   return done();
 }
 
