@@ -347,7 +347,9 @@ int solv_gpu_gnn_adam(solv_gpu_ctx *ctx, float lr, float grad_scale);
  * the context's precision, and leaves the fastest set on the context.
  * ms_per_iter_before is the per-iteration time of the settings in effect
  * before the call, measured the same way; those settings stay eligible, so
- * ms_per_iter <= ms_per_iter_before. */
+ * ms_per_iter <= ms_per_iter_before.  What is timed is the step kernels,
+ * also where the solve itself runs as one launch (SOLV_OPT_GRAPH_LOOP,
+ * SOLV_OPT_PERSISTENT), which has no use for these settings. */
 typedef struct {
   int block, grid_per_sm, graph_iters, candidates;
   double ms_per_iter;

@@ -3374,6 +3374,21 @@ int solv_gpu_autotune(solv_gpu_ctx* c, int solver, int imat, int n_vc, solv_gpu_
     }
   } delta_keep{c, c->reliable_delta, c->fcg_reliable_delta};
   c->reliable_delta = c->fcg_reliable_delta = 1e-300;
+  // What is tuned is the step kernels.  An FP64 CG or BiCGSTAB that would run
+  // as one launch (solve_fp64) has no use for these settings, and timing it
+  // would choose by noise what the context's other solves then run with.
+  struct FormKeep {  // restored on every way out
+    solv_gpu_ctx* c;
+    int loop, persistent;
+    ~FormKeep() {
+      c->graph_loop = loop;
+      c->persistent = persistent;
+    }
+  } form_keep{c, c->graph_loop, c->persistent};
+  if (!fp32) {
+    if (c->graph_loop == 2) c->graph_loop = 0;  // the same graphs of step kernels
+    c->persistent = 0;
+  }
   const int blocks[] = {128, 256};
   const int gps[] = {4, 8, 16};
   const int graphs[] = {8, 32};
