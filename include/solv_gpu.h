@@ -267,6 +267,13 @@ int solv_gpu_kernel_time(solv_gpu_ctx *ctx, int which, int repeat,
  * context stays usable. */
 int solv_gpu_selftest_sweep_wait(solv_gpu_ctx *ctx);
 
+/* Diagnostic (no counterpart in the reference): from now on, the nth of the
+ * context's launches by configuration -- the kernels of an iteration,
+ * clusters, cooperative launches, also those recorded into a graph -- is not
+ * made but answered with `error`, a cudaError_t, as if the CUDA runtime had
+ * refused it; nth 0 calls it off.  Nothing reaches the GPU. */
+int solv_gpu_selftest_fail_launch(solv_gpu_ctx *ctx, int nth, int error);
+
 /* -- learned preconditioner ---------------------------------------------- */
 /* No counterpart in the reference.  Flexible CG, FCG(1), in FP32 with
  * FP64 reliable updates.  A 3-layer, width-32 message-passing network over

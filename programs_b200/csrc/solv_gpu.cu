@@ -96,6 +96,9 @@ struct solv_gpu_ctx {
   cudaStream_t side = nullptr;         // the coarsest inverse beside the main stream
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   std::string err;
+  cudaError_t launch_err = cudaSuccess;  // a launch refused since launch_status
+  int fail_launch = 0;                   // launches until one is refused on purpose
+  cudaError_t fail_with = cudaSuccess;
   int n_sm = 148;
   // options
   int precision = 0;
@@ -963,6 +966,29 @@ int mg_setup(solv_gpu_ctx* c) {
   return SOLV_GPU_OK;
 }
 
+// Every launch by configuration (chains, clusters, cooperative ones) goes
+// through here, where solv_gpu_selftest_fail_launch can have one refused.
+template <typename... KArgs, typename... Args>
+cudaError_t launch(solv_gpu_ctx* c, const cudaLaunchConfig_t& cfg, void (*kern)(KArgs...),
+                   Args... args) {
+  if (c->fail_launch > 0 && --c->fail_launch == 0) return c->fail_with;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// Chains are launched by functions that count kernels; a refused launch is
+// kept here for launch_status, which who started the chain asks: a graph
+// whose capture lacks a kernel must not be kept.
+void note_launch(solv_gpu_ctx* c, cudaError_t e) {
+  if (e != cudaSuccess && c->launch_err == cudaSuccess) c->launch_err = e;
+}
+int launch_status(solv_gpu_ctx* c) {
+  const cudaError_t e = c->launch_err;
+  if (e == cudaSuccess) return SOLV_GPU_OK;
+  c->launch_err = cudaSuccess;
+  cudaGetLastError();  // reported here, not by the next call
+  return set_err(c, SOLV_GPU_DEVICE_ERROR, std::string("kernel launch: ") + cudaGetErrorString(e));
+}
+
 // A kernel of an iteration's chain (kernels.cuh, chain_enter).  Launched on a
 // stream, a V-cycle at 64^3 (ten kernels) takes 66 us where it took 86; inside
 // a graph, whose launches are closer to begin with, the learned solve at 64^3
@@ -978,13 +1004,13 @@ void chain_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), int grid, int block, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, args...);  // a failure is the caller's cudaGetLastError()
+  note_launch(c, launch(c, cfg, kern, args...));
 }
 
 // One thread-block cluster of cs blocks; chain: as chain_launch.
 template <typename... KArgs, typename... Args>
-int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), cudaStream_t stream, bool chain, int cs,
-                   int threads, Args... args) {
+cudaError_t cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), cudaStream_t stream, bool chain,
+                           int cs, int threads, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)cs);
   cfg.blockDim = dim3((unsigned)threads);
@@ -998,8 +1024,7 @@ int cluster_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), cudaStream_t stream,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = chain ? 2 : 1;
-  CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, args...));
-  return SOLV_GPU_OK;
+  return launch(c, cfg, kern, args...);
 }
 
 // Coefficients of every coarse level for the current values (each solve):
@@ -1037,9 +1062,9 @@ int mg_values(solv_gpu_ctx* c) {
   if (C.n <= 128)
     mg::k_mg_invert<128, 1><<<1, 1024, 0, c->side>>>(C.n, c->mg_dense.as<double>(),
                                                      c->mg_ainv.as<float>());
-  else if ((rc = cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, c->side, false, 8, 512, C.n,
-                                (const double*)c->mg_dense.as<double>(), c->mg_ainv.as<float>())))
-    return rc;
+  else
+    CUDA_TRY(c, cluster_launch(c, mg::k_mg_invert<mg::kCoarsest, 8>, c->side, false, 8, 512, C.n,
+                               (const double*)c->mg_dense.as<double>(), c->mg_ainv.as<float>()));
   CUDA_TRY(c, cudaEventRecord(c->ev_join, c->side));
   c->launches += 2 + 3 * (int)c->mg.size() + 2;
   CUDA_TRY(c, cudaGetLastError());
@@ -1121,8 +1146,8 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
                     F.agg_of.as<int>(), F.x.as<float>(), F.b.as<float>(), F.t.as<float>(),
                     F.y.as<float>()};
   }
-  cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, s, true,
-                 mg_bottom_blocks(c), mg::kFuseThreads, A, w, a, na);
+  note_launch(c, cluster_launch(c, ordered ? mg::k_mg_bottom<true> : mg::k_mg_bottom<false>, s, true,
+                                mg_bottom_blocks(c), mg::kFuseThreads, A, w, a, na));
   for (int l = lf - 1; l >= 0; --l) {
     MgLevel& F = *c->mg[l];
     MgLevel& C = *c->mg[l + 1];
@@ -1321,7 +1346,7 @@ int coop_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), Args... args) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, args...));
+  CUDA_TRY(c, launch(c, cfg, kern, args...));
   c->launches++;
   return SOLV_GPU_OK;
 }
@@ -1383,7 +1408,7 @@ int launch_direct(solv_gpu_ctx* c, int imat, const T* cc, const T* cr, T* x, con
   if (imat <= 0) {
     chain_launch(c, sg::k_jacobi<T, V>, grid_for(c, c->N), c->block, c->N, cc, b, x);
     c->launches++;
-    return SOLV_GPU_OK;
+    return launch_status(c);
   }
   Rows<T> R = rows<T>(c);
   T* t = sweep_t<T>(c);
@@ -1391,8 +1416,10 @@ int launch_direct(solv_gpu_ctx* c, int imat, const T* cc, const T* cr, T* x, con
   int rc = coop_launch(c, gate ? sg::k_fwd_sf<T, V, true> : sg::k_fwd_sf<T, V, false>, c->N, R,
                        sweep_map(c), cc, b, t, x, sweep_ctl(c), n_active);
   if (rc) return rc;
-  return coop_launch(c, gate ? sg::k_bwd_sf<T, V, true> : sg::k_bwd_sf<T, V, false>, c->N, R,
-                     sweep_map(c), cc, cr, t, x, sweep_ctl(c), n_active);
+  rc = coop_launch(c, gate ? sg::k_bwd_sf<T, V, true> : sg::k_bwd_sf<T, V, false>, c->N, R,
+                   sweep_map(c), cc, cr, t, x, sweep_ctl(c), n_active);
+  if (rc) c->t_ready = c->tf_ready = false;  // t keeps the forward sweep's values
+  return rc;
 }
 
 // Workspace for V components in precision T.
@@ -1435,8 +1462,8 @@ int ensure_ws(solv_gpu_ctx* c, int V, WS<T>& w) {
     CUDA_TRY(c, cudaMemsetAsync(c->sweep_ctl.p, 0, sizeof(sg::SweepCtl), c->stream));
   }
   if (!ready) {
-    sg::k_fill_pending<T><<<grid_for(c, (long long)c->N * V), c->block, 0, c->stream>>>(
-        (long long)c->N * V, tb.as<T>());
+    const long long all = (long long)(tb.bytes / sizeof(T));  // also what more components will use
+    sg::k_fill_pending<T><<<grid_for(c, all), c->block, 0, c->stream>>>(all, tb.as<T>());
     CUDA_TRY(c, cudaGetLastError());
     ready = true;
   }
@@ -1600,9 +1627,10 @@ cudaError_t build_while_graph(solv_gpu_ctx* c, Body&& body, int& rc, cudaGraphEx
                                         cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
         rc = body();
-        if (!rc)
-          chain_launch(c, sg::k_loop_ctl, 1, 32, h, c->n_active.as<int>(),
-                                                  c->loop_budget.as<int>());
+        if (!rc) {
+          chain_launch(c, sg::k_loop_ctl, 1, 32, h, c->n_active.as<int>(), c->loop_budget.as<int>());
+          rc = launch_status(c);
+        }
         cudaGraph_t out = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(c->stream, &out);
         if (e == cudaSuccess) e = e2;
@@ -1623,10 +1651,12 @@ int iterate(solv_gpu_ctx* c, int solver, int imat, int n_iter, WS<T>& w, int& gr
             std::vector<Lane>* lanes_out = nullptr) {
   const int K = c->graph_iters;
   auto body = [&]() -> int {
-    if (solver == 0) return cg_iteration<T, V>(c, imat, w);
-    if (solver == 1) return bicg_iteration<T, V>(c, imat, w);
-    if constexpr (V == 1) fcg_iteration<T>(c, w);
-    return SOLV_GPU_OK;
+    int rc = SOLV_GPU_OK;
+    if (solver == 0) rc = cg_iteration<T, V>(c, imat, w);
+    else if (solver == 1) rc = bicg_iteration<T, V>(c, imat, w);
+    else if constexpr (V == 1) fcg_iteration<T>(c, w);
+    const int ls = launch_status(c);
+    return rc ? rc : ls;
   };
   cudaGraphExec_t exec = nullptr;
   bool loop = false;  // exec is a WHILE graph: one launch runs until the lanes stop
@@ -1859,7 +1889,7 @@ int resident_pcg(solv_gpu_ctx* c, const double* cc, double* phi, const double* r
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CUDA_TRY(c, cudaLaunchKernelEx(&cfg, G.kern, rows<double>(c), sm, std::max(c->max_w, 1),
+  CUDA_TRY(c, launch(c, cfg, G.kern, rows<double>(c), sm, std::max(c->max_w, 1),
                                  c->grid_res, cc, phi, r0, c->grid_zp.as<double2>(),
                                  c->grid_inbox.as<unsigned long long>(), c->lanes.as<Lane>(),
                                  sweep_ctl(c)));
@@ -2144,7 +2174,7 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, rows<double>(c), sm.seg_c0, sm.seg_c1,
+    CUDA_TRY(c, launch(c, cfg, kern, rows<double>(c), sm.seg_c0, sm.seg_c1,
                                    (const double*)w.c, w.phi, w.r, w.p, w.q, c->lanes.as<Lane>(),
                                    c->n_active.as<int>()));
     c->launches++;
@@ -3144,6 +3174,13 @@ int solv_gpu_selftest_sweep_wait(solv_gpu_ctx* c) {
   return sweep_check(c);  // synchronises; SOLV_GPU_TIMEOUT when the wait ran out
 }
 
+int solv_gpu_selftest_fail_launch(solv_gpu_ctx* c, int nth, int error) {
+  if (!c || nth < 0 || (nth > 0 && error == cudaSuccess)) return SOLV_GPU_BAD_INPUT;
+  c->fail_launch = nth;
+  c->fail_with = (cudaError_t)error;
+  return SOLV_GPU_OK;
+}
+
 int solv_gpu_kernel_time(solv_gpu_ctx* c, int which, int repeat, float* ms_per_launch) {
   if (!c) return SOLV_GPU_BAD_INPUT;
   if (!c->has_matrix) return set_err(c, SOLV_GPU_NO_MATRIX, "no matrix set");
@@ -3201,6 +3238,7 @@ int solv_gpu_kernel_time(solv_gpu_ctx* c, int which, int repeat, float* ms_per_l
     CUDA_TRY(c, cudaEventRecord(c->ev1, s));
   }
   CUDA_TRY(c, cudaEventSynchronize(c->ev1));
+  if (int rc = launch_status(c)) return rc;
   CUDA_TRY(c, cudaGetLastError());
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -3694,6 +3732,7 @@ static int mg_train_sample(solv_gpu_ctx* c, float** B) {
   // pre-smoother x = w K b: its input b, its output gradient az
   mg::k_mg_scaled_pair<<<G, Bk, 0, s>>>(N, rsd, w, b, az, uh, gh);
   back(uh, gh);
+  if (int rc = launch_status(c)) return rc;
   CUDA_TRY(c, cudaGetLastError());
   return SOLV_GPU_OK;
 }
