@@ -1835,6 +1835,13 @@ int resident_plan(solv_gpu_ctx* c) {
     if (2 * h[1] < h[0]) return SOLV_GPU_OK;
   }
   const GridShape& G = kGridShapes[shape];
+  // what cannot be had here leaves the step kernels, which need less
+  auto without = [&]() {
+    cudaGetLastError();
+    c->grid_inbox.release();
+    c->grid_zp.release();
+    return SOLV_GPU_OK;
+  };
   cudaFuncAttributes fa;
   int optin = 0;
   CUDA_TRY(c, cudaFuncGetAttributes(&fa, G.kern));
@@ -1843,6 +1850,10 @@ int resident_plan(solv_gpu_ctx* c) {
   const int res = std::min(G.rpt, (optin - (int)fa.sharedSizeBytes) / row);
   CUDA_TRY(c, cudaFuncSetAttribute(G.kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    optin - (int)fa.sharedSizeBytes));
+  int per_sm = 0;
+  CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, G.kern, G.threads,
+                                                            (size_t)res * row));
+  if (per_sm < 1) return without();
   std::vector<int> m;  // blk_seg, blk_rank, seg_nblk, seg_blk0, seg_c0, seg_c1
   for (int k = 0; k < ns; ++k) m.insert(m.end(), nb[k], k);
   for (int k = 0; k < ns; ++k)
@@ -1852,8 +1863,11 @@ int resident_plan(solv_gpu_ctx* c) {
   m.insert(m.end(), c->seg_c0_caller.begin(), c->seg_c0_caller.end());
   m.insert(m.end(), c->seg_c1_caller.begin(), c->seg_c1_caller.end());
   CUDA_TRY(c, upload(c->grid_map, m, c->stream));
-  CUDA_TRY(c, c->grid_inbox.ensure((size_t)2 * sg::kInboxWords * total * sizeof(double)));
-  CUDA_TRY(c, c->grid_zp.ensure((size_t)c->N * sizeof(double2)));
+  if (c->grid_inbox.ensure((size_t)2 * sg::kInboxWords * total * sizeof(double)) != cudaSuccess ||
+      c->grid_zp.ensure((size_t)c->N * sizeof(double2)) != cudaSuccess) {
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // m dies here
+    return without();
+  }
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // m dies here
   c->grid_blk = total;
   c->grid_smem = res * row;
@@ -1863,7 +1877,10 @@ int resident_plan(solv_gpu_ctx* c) {
 }
 
 // The whole loop from r0 (the initial residual) and the Jacobi c into phi.
-int resident_pcg(solv_gpu_ctx* c, const double* cc, double* phi, const double* r0) {
+// Where the blocks cannot all be resident after all (a context on part of the
+// SMs) the launch is refused before it starts: ran is off, and the structure's
+// solves go on as before there was a resident form.
+int resident_pcg(solv_gpu_ctx* c, const double* cc, double* phi, const double* r0, bool& ran) {
   const int nb = c->grid_blk, ns = c->n_seg;
   const GridShape& G = kGridShapes[c->grid_shape];
   int* m = c->grid_map.as<int>();
@@ -1889,10 +1906,17 @@ int resident_pcg(solv_gpu_ctx* c, const double* cc, double* phi, const double* r
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CUDA_TRY(c, launch(c, cfg, G.kern, rows<double>(c), sm, std::max(c->max_w, 1),
-                                 c->grid_res, cc, phi, r0, c->grid_zp.as<double2>(),
-                                 c->grid_inbox.as<unsigned long long>(), c->lanes.as<Lane>(),
-                                 sweep_ctl(c)));
+  const cudaError_t e =
+      launch(c, cfg, G.kern, rows<double>(c), sm, std::max(c->max_w, 1), c->grid_res, cc, phi, r0,
+             c->grid_zp.as<double2>(), c->grid_inbox.as<unsigned long long>(), c->lanes.as<Lane>(),
+             sweep_ctl(c));
+  ran = e != cudaErrorCooperativeLaunchTooLarge;
+  if (!ran) {
+    cudaGetLastError();
+    c->grid_shape = -1;
+    return SOLV_GPU_OK;
+  }
+  CUDA_TRY(c, e);
   c->launches += 2;
   return SOLV_GPU_OK;
 }
@@ -2063,13 +2087,6 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
     if ((rc = resident_plan(c))) return rc;
     grid = c->grid_shape >= 0;
   }
-  if (!grid) {
-    CUDA_TRY(c, cudaMemcpyAsync(w.r, w.r0, (size_t)N * V * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    CUDA_TRY(c, cudaMemsetAsync(w.p, 0, (size_t)N * V * sizeof(double), s));
-    CUDA_TRY(c, cudaMemsetAsync(w.q, 0, (size_t)N * V * sizeof(double), s));
-    CUDA_TRY(c, cudaMemsetAsync(w.v, 0, (size_t)N * V * sizeof(double), s));
-    CUDA_TRY(c, cudaMemsetAsync(w.z, 0, (size_t)N * V * sizeof(double), s));
-  }
   {
     int na = nl;
     if (n_iter <= 0) na = 0;
@@ -2077,25 +2094,32 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
   }
   sg::k_lane_init<<<(nl + 255) / 256, 256, 0, s>>>(c->lanes.as<Lane>(), nl, n_iter, reduc,
                                                    c->n_active.as<int>());
+  c->launches += 2;
   SegMap sm = segmap(c);
+  if (grid) {
+    if ((rc = resident_pcg(c, w.c, w.phi, w.r0, grid))) return rc;
+    if (grid && (rc = sweep_check(c))) return rc;
+  }
   const bool fused = c->persistent && jac_cg && !grid;
-  if (solver == 0) {
-    if (imat <= 0 && !fused && !grid) {
+  if (!grid) {
+    CUDA_TRY(c, cudaMemcpyAsync(w.r, w.r0, (size_t)N * V * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    CUDA_TRY(c, cudaMemsetAsync(w.p, 0, (size_t)N * V * sizeof(double), s));
+    CUDA_TRY(c, cudaMemsetAsync(w.q, 0, (size_t)N * V * sizeof(double), s));
+    CUDA_TRY(c, cudaMemsetAsync(w.v, 0, (size_t)N * V * sizeof(double), s));
+    CUDA_TRY(c, cudaMemsetAsync(w.z, 0, (size_t)N * V * sizeof(double), s));
+    if (solver == 0 && imat <= 0 && !fused) {
       sg::k_cg_rz<double, V, true><<<c->seg.total_blk, c->block, 0, s>>>(
           sm, w.c, w.r, w.z, c->part.as<double>(), c->lanes.as<Lane>());
       c->launches++;
+    } else if (solver != 0) {
+      sg::k_bi_rho<double, V><<<c->seg.total_blk, c->block, 0, s>>>(
+          sm, w.r, w.r0, c->part.as<double>(), c->lanes.as<Lane>());
+      c->launches++;
     }
-  } else {
-    sg::k_bi_rho<double, V><<<c->seg.total_blk, c->block, 0, s>>>(
-        sm, w.r, w.r0, c->part.as<double>(), c->lanes.as<Lane>());
-    c->launches++;
   }
-  c->launches += 2;
   CUDA_TRY(c, cudaGetLastError());
   int gl = 0;
-  if (grid) {
-    if ((rc = resident_pcg(c, w.c, w.phi, w.r0)) || (rc = sweep_check(c))) return rc;
-  } else if (fused) {  // the whole loop in one launch: one cluster per system
+  if (fused) {  // the whole loop in one launch: one cluster per system
     // systems of at most 16 x 2048 cells run with their vectors in the
     // cluster's registers and shared memory (k_pcg_cluster_res), larger
     // ones from global memory (k_pcg_cluster); 16 blocks per cluster where
@@ -2178,7 +2202,7 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
                                    (const double*)w.c, w.phi, w.r, w.p, w.q, c->lanes.as<Lane>(),
                                    c->n_active.as<int>()));
     c->launches++;
-  } else {
+  } else if (!grid) {
     rc = iterate<double, V>(c, solver, imat, n_iter, w, gl);
     if (rc) return rc;
   }

@@ -101,3 +101,44 @@ def test_refused_launches_in_a_training_step(gpu, system):
         assert refused >= 6
     finally:
         gpu.set_option(OPT_GNN_LOSS, 1)
+
+
+@pytest.mark.parametrize("persistent", [0, 1])
+def test_a_resident_launch_too_large_for_the_gpu(gpu, persistent):
+    """Where the resident PCG's blocks cannot all run at once the solve takes
+    the form it would have without it: step kernels, or a cluster."""
+    from oracle.oracle import Oracle
+    from programs_b200.mesh import poisson_rhs
+    from programs_b200.solver import OPT_PERSISTENT
+    too_large = 720  # cudaErrorCooperativeLaunchTooLarge
+    m = Mesh.hex(24, jitter=0.15, seed=2, permute=True)
+    m.renumber(Mesh.RCM)
+    A = m.pressure(pin=1)
+    b = poisson_rhs(A.n_cell, 4).reshape(-1, 1)
+    ref = Oracle.from_matrix(A).solv_cg(0, 1e-10, 5000, np.zeros((A.n_cell, 1)), b)
+    gpu.matrix_set(A)
+    gpu.set_option(OPT_PERSISTENT, persistent)
+
+    def solve():
+        phi, res = np.zeros((A.n_cell, 1)), np.asfortranarray(b.copy())
+        st = gpu.solv_cg(0, 1e-10, 5000, phi, res, np.zeros(1))
+        assert st["status"] == OK and np.array_equal(res, ref[1])
+        assert abs(st["iters"][0] - int(ref[3][0])) <= 2
+        assert np.linalg.norm(phi - ref[0]) <= 1e-8 * np.linalg.norm(ref[0])
+        return st["graph_launches"]
+    try:
+        gpu.selftest_fail_launch(1, too_large)
+        assert (solve() == 0) == bool(persistent)
+        gpu.selftest_fail_launch(0)
+        assert (solve() == 0) == bool(persistent)  # not tried again on this structure
+        gpu.matrix_set(A)
+        assert solve() == 0
+        gpu.selftest_fail_launch(1, OUT_OF_RESOURCES)
+        with pytest.raises(SolverError) as e:
+            solve()
+        assert e.value.code == DEVICE_ERROR
+        gpu.selftest_fail_launch(0)
+        assert solve() == 0
+    finally:
+        gpu.selftest_fail_launch(0)
+        gpu.set_option(OPT_PERSISTENT, 0)
