@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <new>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -58,7 +59,7 @@ struct Geo {
   const D4* cr;                // per cell {centre, volume}
   const double2* sw;           // per face {area, w_fp}
   const double *l, *w, *vol;   // l_pn, w_fp; cell volumes
-  const int* cs_ptr;           // first slot of each slice of 32 cells
+  const int* cs_row;           // first row of 32 slots of each slice of 32 cells
   const int2* cs;              // slots: {2 face + (1 for the neighbour's side), other cell};
                                // {-1, -1} padding, other cell -1 on boundary faces
 };
@@ -87,20 +88,23 @@ __device__ __forceinline__ Cell cell_of(const Geo& g, int c) {
 // the face before it (9x9x9, us: two sweeps 12.1, now 9.3; the imbalance's
 // sums 5.2, now 3.6).  S = 6, a hex cell's faces, where the registers allow.
 template <int S>
-__device__ __forceinline__ void slots_of(const Geo& g, int q, int e, int2 (&t)[S]) {
+__device__ __forceinline__ void chunk_of(const Geo& g, int c, int r, int end, int2 (&t)[S]) {
+  const int2* p = g.cs + (32ll * r + (c & 31));
 #pragma unroll
-  for (int k = 0; k < S; ++k) t[k] = q + 32 * k < e ? g.cs[q + 32 * k] : make_int2(-1, -1);
+  for (int k = 0; k < S; ++k) t[k] = r + k < end ? p[32 * k] : make_int2(-1, -1);
 }
+__device__ __forceinline__ int face_in(int2 t) { return (int)((unsigned)t.x >> 1); }
+__device__ __forceinline__ bool own_side(int2 t) { return (t.x & 1) == 0; }
 // f(face, owner side, other cell) for the faces of cell c, ascending
 template <int S, typename F>
 __device__ __forceinline__ void faces_of(const Geo& g, int c, F&& f) {
-  const int b = g.cs_ptr[c >> 5], e = g.cs_ptr[(c >> 5) + 1];
-  for (int q = b + (c & 31); q < e; q += 32 * S) {
+  const int end = g.cs_row[(c >> 5) + 1];
+  for (int r = g.cs_row[c >> 5]; r < end; r += S) {
     int2 t[S];
-    slots_of(g, q, e, t);
+    chunk_of(g, c, r, end, t);
 #pragma unroll
     for (int k = 0; k < S; ++k)
-      if (t[k].x >= 0) f(t[k].x >> 1, (t[k].x & 1) == 0, t[k].y);
+      if (t[k].x != -1) f(face_in(t[k]), own_side(t[k]), t[k].y);
   }
 }
 // The same where a face gives a value or a few, load(face, owner side): the
@@ -108,17 +112,17 @@ __device__ __forceinline__ void faces_of(const Geo& g, int c, F&& f) {
 // side, other cell) in order.
 template <int S, typename L, typename F>
 __device__ __forceinline__ void fold_faces(const Geo& g, int c, L&& load, F&& f) {
-  const int b = g.cs_ptr[c >> 5], e = g.cs_ptr[(c >> 5) + 1];
-  for (int q = b + (c & 31); q < e; q += 32 * S) {
+  const int end = g.cs_row[(c >> 5) + 1];
+  for (int r = g.cs_row[c >> 5]; r < end; r += S) {
     int2 t[S];
     decltype(load(0, true)) v[S];
-    slots_of(g, q, e, t);
+    chunk_of(g, c, r, end, t);
 #pragma unroll
     for (int k = 0; k < S; ++k)
-      if (t[k].x >= 0) v[k] = load(t[k].x >> 1, (t[k].x & 1) == 0);
+      if (t[k].x != -1) v[k] = load(face_in(t[k]), own_side(t[k]));
 #pragma unroll
     for (int k = 0; k < S; ++k)
-      if (t[k].x >= 0) f(v[k], t[k].x >> 1, (t[k].x & 1) == 0, t[k].y);
+      if (t[k].x != -1) f(v[k], face_in(t[k]), own_side(t[k]), t[k].y);
   }
 }
 
@@ -606,7 +610,7 @@ struct fv_gpu {
   int dev = 0;
   cudaStream_t stream = nullptr;
   Geo g{};
-  DBuf ab, fn, fc, cr, sw, l, w, vol, vr, cs_ptr, cs, dface, part, total, tmp;
+  DBuf ab, fn, fc, cr, sw, l, w, vol, vr, cs_row, cs, dface, part, total, tmp;
   size_t tmp_bytes = 0;
 };
 
@@ -629,6 +633,17 @@ double* scratch(fv_gpu* fv, size_t bytes) {
   if (cudaMalloc(&fv->tmp.p, bytes) != cudaSuccess) return nullptr;
   fv->tmp_bytes = bytes;
   return fv->tmp.as<double>();
+}
+
+// First row of each slice, and the rows in all, from the cells' face counts:
+// a slice has as many rows of 32 slots as its widest cell has faces.  (Rows
+// fit 32 bits where the counts' sum does; slots need not, with one cell of
+// very many faces.)
+std::vector<int> slice_rows(int n_cell, const int* deg) {
+  std::vector<int> r(((long long)n_cell + 31) / 32 + 1, 0);
+  for (int c = 0; c < n_cell; ++c) r[c / 32 + 1] = std::max(r[c / 32 + 1], deg[c]);
+  for (size_t k = 1; k < r.size(); ++k) r[k] += r[k - 1];
+  return r;
 }
 
 int enter(fv_gpu* fv) {
@@ -656,18 +671,9 @@ int done() {
   return cudaGetLastError() == cudaSuccess ? SOLV_GPU_OK : SOLV_GPU_DEVICE_ERROR;
 }
 
-}  // namespace
-
-extern "C" {
-
-int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* ip, const int* in,
-                  const double* area, const double* nrm, const double* xf, const double* l_pn,
-                  const double* w_fp, const double* xc, const double* vol) {
-  if (!out) return SOLV_GPU_BAD_INPUT;
-  *out = nullptr;
-  if (n_cell <= 0 || n_face < 0 || !ip || !in || !area || !nrm || !xf || !l_pn || !w_fp || !xc ||
-      !vol)
-    return SOLV_GPU_BAD_INPUT;
+int create(fv_gpu** out, int device, int n_cell, int n_face, const int* ip, const int* in,
+           const double* area, const double* nrm, const double* xf, const double* l_pn,
+           const double* w_fp, const double* xc, const double* vol) {
   std::vector<int2> ab(n_face);
   std::vector<int> deg(n_cell, 0);
   for (int f = 0; f < n_face; ++f) {
@@ -677,20 +683,13 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
     deg[a]++;
     if (b >= 0) deg[b]++;
   }
-  const int ns = (n_cell + 31) / 32;
-  std::vector<int> cs_ptr(ns + 1, 0);
-  for (int s = 0; s < ns; ++s) {
-    int w = 0;
-    for (int c = s * 32; c < std::min(n_cell, s * 32 + 32); ++c) w = std::max(w, deg[c]);
-    const long long end = (long long)cs_ptr[s] + 32LL * w;
-    if (end > 0x7fffffffLL) return SOLV_GPU_BAD_INPUT;  // beyond int32 slot offsets
-    cs_ptr[s + 1] = (int)end;
-  }
-  std::vector<int2> cs(cs_ptr[ns], make_int2(-1, -1));
+  const std::vector<int> cs_row = slice_rows(n_cell, deg.data());
+  std::vector<int2> cs((size_t)cs_row.back() * 32, make_int2(-1, -1));
   std::vector<int> pos(n_cell, 0);
   for (int f = 0; f < n_face; ++f) {  // ascending faces: each cell's slots come out sorted
-    auto put = [&](int c, int side, int other) {
-      cs[cs_ptr[c >> 5] + pos[c]++ * 32 + (c & 31)] = make_int2(2 * f + side, other);
+    auto put = [&](int c, unsigned side, int other) {
+      const size_t row = cs_row[c >> 5] + pos[c]++;
+      cs[row * 32 + (c & 31)] = make_int2((int)(2u * f + side), other);
     };
     put(ab[f].x, 0, ab[f].y);
     if (ab[f].y >= 0) put(ab[f].y, 1, ab[f].x);
@@ -718,7 +717,7 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
   chk(up(fv->l, l_pn, F));
   chk(up(fv->w, w_fp, F));
   chk(up(fv->vol, vol, N));
-  chk(up(fv->cs_ptr, cs_ptr.data(), cs_ptr.size()));
+  chk(up(fv->cs_row, cs_row.data(), cs_row.size()));
   chk(up(fv->cs, cs.data(), cs.size()));
   chk(cudaMalloc(&fv->dface.p, std::max<size_t>(F, 1) * sizeof(double)));
   chk(cudaMalloc(&fv->part.p, kRedBlocks * sizeof(double)));
@@ -744,10 +743,29 @@ int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* i
   g.cr = fv->cr.as<D4>();
   g.l = fv->l.as<double>();
   g.w = fv->w.as<double>();
-  g.cs_ptr = fv->cs_ptr.as<int>();
+  g.cs_row = fv->cs_row.as<int>();
   g.cs = fv->cs.as<int2>();
   *out = fv;
   return SOLV_GPU_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int fv_gpu_create(fv_gpu** out, int device, int n_cell, int n_face, const int* ip, const int* in,
+                  const double* area, const double* nrm, const double* xf, const double* l_pn,
+                  const double* w_fp, const double* xc, const double* vol) {
+  if (!out) return SOLV_GPU_BAD_INPUT;
+  *out = nullptr;
+  if (n_cell <= 0 || n_face < 0 || !ip || !in || !area || !nrm || !xf || !l_pn || !w_fp || !xc ||
+      !vol)
+    return SOLV_GPU_BAD_INPUT;
+  try {
+    return create(out, device, n_cell, n_face, ip, in, area, nrm, xf, l_pn, w_fp, xc, vol);
+  } catch (const std::bad_alloc&) {
+    return SOLV_GPU_TOO_LARGE;
+  }
 }
 
 int fv_gpu_destroy(fv_gpu* fv) {
