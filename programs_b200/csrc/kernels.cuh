@@ -736,14 +736,14 @@ __device__ __forceinline__ void sweep_slice(int n, const Rows<T>& R, int s, int 
         T m[C][V];
 #pragma unroll
         for (int q = 0; q < C; ++q) {
-            T xv[V];
+          T xv[V];
 #pragma unroll
           for (int v = 0; v < V; ++v) xv[v] = P::from(bits[q][v]);
           term(a[q], xv, m[q]);
         }
 #pragma unroll
         for (int q = 0; q < C; ++q) {
-            if (GATE && q >= nd) break;
+          if (GATE && q >= nd) break;
           if (on(q)) fold(m[q]);
         }
         k0 += C;
@@ -1927,7 +1927,8 @@ __device__ __noinline__ void small_direct(const SmallArgs& A, int c0, int c1, co
 }
 
 template <int SOLVER, int V, bool SW>
-__global__ void __launch_bounds__(kSmallThreads, 1) k_small_solve(const __grid_constant__ SmallArgs A, int parts) {
+__global__ void __launch_bounds__(kSmallThreads, 1)
+k_small_solve(const __grid_constant__ SmallArgs A, int parts) {
   constexpr int NW = kSmallThreads / 32;
   extern __shared__ __align__(16) double dyn_s[];
   __shared__ double red[2][2 * V][NW];

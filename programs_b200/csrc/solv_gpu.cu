@@ -1123,16 +1123,15 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
   for (int l = 0; l < lf; ++l) {
     MgLevel& F = *c->mg[l];
     chain_launch(c, mg::k_mg_restrict, grid_for(c, F.n), B, F.n, F.agg_ptr.as<int>(),
-                                                     F.agg_cells.as<int>(), t, F.b.as<float>(), na);
+                 F.agg_cells.as<int>(), t, F.b.as<float>(), na);
     if (F.n <= mg::kCoarseCells)
-      chain_launch(c, (ordered ? mg::k_mg_pre_coarse<true> : mg::k_mg_pre_coarse<false>), grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 
-          F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.t.as<float>(),
-          na);
+      chain_launch(c, ordered ? mg::k_mg_pre_coarse<true> : mg::k_mg_pre_coarse<false>,
+                   grid_for(c, (long long)F.n * mg::kCoarseLanes), B, F.n, F.rows(),
+                   F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.t.as<float>(), na);
     else
       with_chunk(c->row_chunk, [&](auto ch) {
-        chain_launch(c, mg::k_mg_pre<decltype(ch)::value>, grid_for(c, F.n), B, 
-            F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(),
-            F.t.as<float>(), na);
+        chain_launch(c, mg::k_mg_pre<decltype(ch)::value>, grid_for(c, F.n), B, F.n, F.rows(),
+                     F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.t.as<float>(), na);
       });
     t = F.t.as<float>();
   }
@@ -1151,17 +1150,16 @@ int mg_coarse_cycle(solv_gpu_ctx* c, const float* t0, const int* na, bool ordere
   for (int l = lf - 1; l >= 0; --l) {
     MgLevel& F = *c->mg[l];
     MgLevel& C = *c->mg[l + 1];
-    chain_launch(c, mg::k_mg_prolong, grid_for(c, F.n), B, F.n, C.agg_of.as<int>(), a, C.y.as<float>(),
-                                                    F.x.as<float>(), na);
+    chain_launch(c, mg::k_mg_prolong, grid_for(c, F.n), B, F.n, C.agg_of.as<int>(), a,
+                 C.y.as<float>(), F.x.as<float>(), na);
     if (F.n <= mg::kCoarseCells)
-      chain_launch(c, (ordered ? mg::k_mg_post_coarse<true> : mg::k_mg_post_coarse<false>), grid_for(c, (long long)F.n * mg::kCoarseLanes), B, 
-          F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.y.as<float>(),
-          na);
+      chain_launch(c, ordered ? mg::k_mg_post_coarse<true> : mg::k_mg_post_coarse<false>,
+                   grid_for(c, (long long)F.n * mg::kCoarseLanes), B, F.n, F.rows(),
+                   F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.y.as<float>(), na);
     else
       with_chunk(c->row_chunk, [&](auto ch) {
-        chain_launch(c, mg::k_mg_post<float, decltype(ch)::value>, grid_for(c, F.n), B, 
-            F.n, F.rows(), F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(),
-            F.y.as<float>(), na);
+        chain_launch(c, mg::k_mg_post<float, decltype(ch)::value>, grid_for(c, F.n), B, F.n, F.rows(),
+                     F.dinv.as<float>(), w, F.b.as<float>(), F.x.as<float>(), F.y.as<float>(), na);
       });
   }
   return 4 * lf + 1;
@@ -1179,7 +1177,6 @@ int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, 
               float* x0, float* t0, const int* na, bool ordered = false,
               const float* beta_q = nullptr) {
   const bool net = mode == 1;
-  cudaStream_t s = c->stream;
   const int B = c->block;
   const float w = (float)c->mg_omega, a = (float)c->mg_alpha;
   const int N = c->N;
@@ -1188,45 +1185,40 @@ int mg_vcycle(solv_gpu_ctx* c, const float* r, TZ* z, int mode, const float* q, 
   MgLevel& L1 = *c->mg[0];
   int k = 0;
   const int ch = c->row_chunk;
-  if (net) {
-    chain_launch(c, mg::k_mg_net<false, float>, grid_resident(c, N), B, N, R0, ge, q, w, r, nullptr, x0, na);
+  const int G = grid_resident(c, N);
+  auto resid = [&]() {
     with_chunk(ch, [&](auto cc) {
-      chain_launch(c, mg::k_mg_resid<decltype(cc)::value>, grid_resident(c, N), B, N, R0, r, x0, t0, na);
+      chain_launch(c, mg::k_mg_resid<decltype(cc)::value>, G, B, N, R0, r, x0, t0, na);
     });
+  };
+  if (net) {
+    chain_launch(c, mg::k_mg_net<false, float>, G, B, N, R0, ge, q, w, r, nullptr, x0, na);
+    resid();
     k += 2;
   } else {
     with_chunk(ch, [&](auto cc) {
-      chain_launch(c, mg::k_mg_pre<decltype(cc)::value>, grid_resident(c, N), B, N, R0, d0, w, r, x0,
-                                                                          t0, na);
+      chain_launch(c, mg::k_mg_pre<decltype(cc)::value>, G, B, N, R0, d0, w, r, x0, t0, na);
     });
     k += 1;
   }
   k += mg_coarse_cycle(c, t0, na, ordered);
-  chain_launch(c, mg::k_mg_prolong, grid_resident(c, N), B, N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0,
-                                                na);
+  chain_launch(c, mg::k_mg_prolong, G, B, N, L1.agg_of.as<int>(), a, L1.y.as<float>(), x0, na);
   k += 1;
-  auto last = [&](auto is_net, const float* dq, const float* in) {
+  auto last = [&](auto kern, const float* dq, const float* in) {
     if constexpr (std::is_same<TZ, float>::value)
-      with_chunk(decltype(is_net)::value ? sg::kRowChunk : ch, [&](auto cc) {
-        chain_launch(c, mg::k_mg_last<decltype(is_net)::value, decltype(cc)::value>,
-                     c->seg.total_blk, B, segmap(c), R0, ge, dq, w, in, x0, z, beta_q,
-                     c->part.as<double>(), c->lanes.as<Lane>());
-      });
+      chain_launch(c, kern, c->seg.total_blk, B, segmap(c), R0, ge, dq, w, in, x0, z, beta_q,
+                   c->part.as<double>(), c->lanes.as<Lane>());
   };
   if (net) {
-    with_chunk(ch, [&](auto cc) {
-      chain_launch(c, mg::k_mg_resid<decltype(cc)::value>, grid_resident(c, N), B, N, R0, r, x0, t0, na);
-    });
-    if (beta_q) last(std::true_type(), q, t0);
-    else chain_launch(c, mg::k_mg_net<true, TZ>, grid_resident(c, N), B, N, R0, ge, q, w, t0, x0, z, na);
+    resid();
+    if (beta_q) last(mg::k_mg_last<true, sg::kRowChunk>, q, t0);
+    else chain_launch(c, mg::k_mg_net<true, TZ>, G, B, N, R0, ge, q, w, t0, x0, z, na);
     k += 2;
   } else {
-    if (beta_q) last(std::false_type(), d0, r);
-    else
-      with_chunk(ch, [&](auto cc) {
-        chain_launch(c, mg::k_mg_post<TZ, decltype(cc)::value>, grid_resident(c, N), B, N, R0, d0, w,
-                     r, x0, z, na);
-      });
+    with_chunk(ch, [&](auto cc) {
+      if (beta_q) last(mg::k_mg_last<false, decltype(cc)::value>, d0, r);
+      else chain_launch(c, mg::k_mg_post<TZ, decltype(cc)::value>, G, B, N, R0, d0, w, r, x0, z, na);
+    });
     k += 1;
   }
   return k;
@@ -1334,8 +1326,8 @@ int coop_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), Args... args) {
   }
   const long long warps = ((long long)c->N + 31) / 32;
   // (a block per system of a batch at least)
-  const long long want = std::max<long long>((warps + sg::kSweepThreads / 32 - 1) / (sg::kSweepThreads / 32),
-                                             c->n_seg);
+  constexpr int per = sg::kSweepThreads / 32;
+  const long long want = std::max<long long>((warps + per - 1) / per, c->n_seg);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)std::max(1LL, std::min<long long>(want, (long long)per_sm * c->n_sm)));
   cfg.blockDim = dim3(sg::kSweepThreads);
@@ -1478,8 +1470,8 @@ void cg_spmv(solv_gpu_ctx* c, const SegMap& sm, WS<T>& w, double* part, Lane* la
   const int G = c->seg.total_blk, B = c->block;
   if constexpr (std::is_same<T, float>::value) {
     with_chunk(c->row_chunk, [&](auto ch) {
-      chain_launch(c, sg::k_cg_spmv<T, V, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q,
-                                                                      part, lanes);
+      chain_launch(c, sg::k_cg_spmv<T, V, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q, part,
+                   lanes);
     });
   } else {
     chain_launch(c, sg::k_cg_spmv<T, V>, G, B, rows<T>(c), sm, w.p, w.q, part, lanes);
@@ -1493,8 +1485,8 @@ void bi_spmv(solv_gpu_ctx* c, const SegMap& sm, const T* z, T* y, const T* wv, d
   const int G = c->seg.total_blk, B = c->block;
   if constexpr (std::is_same<T, float>::value) {
     with_chunk(c->row_chunk, [&](auto ch) {
-      chain_launch(c, sg::k_bi_spmv<T, V, MODE, decltype(ch)::value>, G, B, rows<T>(c), sm, z, y,
-                                                                            wv, part, lanes);
+      chain_launch(c, sg::k_bi_spmv<T, V, MODE, decltype(ch)::value>, G, B, rows<T>(c), sm, z, y, wv,
+                   part, lanes);
     });
   } else {
     chain_launch(c, sg::k_bi_spmv<T, V, MODE>, G, B, rows<T>(c), sm, z, y, wv, part, lanes);
@@ -1513,20 +1505,19 @@ int cg_iteration(solv_gpu_ctx* c, int imat, WS<T>& w) {
   double* part = c->part.as<double>();
   Lane* lanes = c->lanes.as<Lane>();
   const int G = c->seg.total_blk, B = c->block;
-  cudaStream_t st = c->stream;
   if (imat > 0) {
     if (int rc = launch_direct<T, V>(c, imat, w.c, w.cr, w.z, w.r, sm.n_active)) return rc;
     chain_launch(c, sg::k_cg_rz<T, V, false, FLEX>, G, B, sm, w.c, w.r, w.z, part, lanes, w.q);
     chain_launch(c, sg::k_cg_p<T, V, false, FLEX>, G, B, sm, w.c, w.r, w.z, w.p, lanes, part);
     cg_spmv<T, V>(c, sm, w, part, lanes);
     chain_launch(c, sg::k_cg_update<T, V, false, FLEX>, G, B, sm, w.c, w.phi, w.r, w.p, w.q, part,
-                                                        lanes);
+                 lanes);
     c->launches += 4;
   } else {
     chain_launch(c, sg::k_cg_p<T, V, true, FLEX>, G, B, sm, w.c, w.r, w.z, w.p, lanes, part);
     cg_spmv<T, V>(c, sm, w, part, lanes);
     chain_launch(c, sg::k_cg_update<T, V, true, FLEX>, G, B, sm, w.c, w.phi, w.r, w.p, w.q, part,
-                                                       lanes);
+                 lanes);
     c->launches += 3;
   }
   return SOLV_GPU_OK;
@@ -1540,7 +1531,6 @@ int bicg_iteration(solv_gpu_ctx* c, int imat, WS<T>& w) {
   double* part = c->part.as<double>();
   Lane* lanes = c->lanes.as<Lane>();
   const int G = c->seg.total_blk, B = c->block;
-  cudaStream_t st = c->stream;
   // w.q holds u, w.v holds v
   if (imat > 0) {
     chain_launch(c, sg::k_bi_p<T, V, false>, G, B, sm, w.c, w.r, w.p, w.q, w.z, lanes);
@@ -1570,7 +1560,6 @@ void fcg_iteration(solv_gpu_ctx* c, WS<T>& w) {
   double* part = c->part.as<double>();
   Lane* lanes = c->lanes.as<Lane>();
   const int G = c->seg.total_blk, B = c->block;
-  cudaStream_t st = c->stream;
   int nk = 1;
   if constexpr (std::is_same<T, float>::value) {
     if (mg_on(c))  // z = V-cycle(r)
@@ -1580,14 +1569,14 @@ void fcg_iteration(solv_gpu_ctx* c, WS<T>& w) {
   }
   if (!mg_on(c))
     chain_launch(c, gnn::k_gnn_apply<T>, grid_for(c, c->N), B, c->N, rows<float>(c),
-                                                          c->g_ge.as<float>(), c->g_q.as<float>(),
-                                                          w.r, w.z, sm.n_active);  // z = M^-1 r
+                 c->g_ge.as<float>(), c->g_q.as<float>(), w.r, w.z, sm.n_active);  // z = M^-1 r
   c->launches += nk - 1;
   if (!mg_on(c)) chain_launch(c, sg::k_fcg_beta<T>, G, B, sm, w.z, w.q, part, lanes);  // beta
-  chain_launch(c, sg::k_cg_p<T, 1, false>, G, B, sm, w.c, w.r, w.z, w.p, lanes, nullptr);   // p = z + beta p
+  chain_launch(c, sg::k_cg_p<T, 1, false>, G, B, sm, w.c, w.r, w.z, w.p, lanes,
+               nullptr);  // p = z + beta p
   with_chunk(c->row_chunk, [&](auto ch) {
-    chain_launch(c, sg::k_fcg_spmv<T, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q, w.r, part,
-                                                            lanes);
+    chain_launch(c, sg::k_fcg_spmv<T, decltype(ch)::value>, G, B, rows<T>(c), sm, w.p, w.q, w.r,
+                 part, lanes);
   });
   chain_launch(c, sg::k_fcg_update<T>, G, B, sm, w.phi, w.r, w.p, w.q, part, lanes);
   c->launches += 5;
@@ -1940,6 +1929,10 @@ SmallKernel small_kernel(int solver, bool sweeps, int& vectors) {
 // 8192 values also fill the shared memory.  Without a recurrence 4096 (14^3
 // BiCGSTAB 17 against 27 us an iteration), and Jacobi-PCG of one component,
 // which k_pcg_grid spreads over several SMs, 1024.
+// More systems than SMs keep the step kernels, although a block a system would
+// be the faster there too: 149 systems of 300-900 cells, Jacobi-PCG 1.90 ms
+// against 0.48, DIC 2.67 against 1.27; 1000 of 100-400, 1.93 against 1.00 and
+// 2.92 against 2.81.
 constexpr int kSmallValues = 8192;
 constexpr int kSmallValuesNone = 4096;
 constexpr int kSmallValuesJacobi = 1024;
@@ -2198,9 +2191,8 @@ int solve_fp64(solv_gpu_ctx* c, int solver, int imat, double reduc, int n_iter,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CUDA_TRY(c, launch(c, cfg, kern, rows<double>(c), sm.seg_c0, sm.seg_c1,
-                                   (const double*)w.c, w.phi, w.r, w.p, w.q, c->lanes.as<Lane>(),
-                                   c->n_active.as<int>()));
+    CUDA_TRY(c, launch(c, cfg, kern, rows<double>(c), sm.seg_c0, sm.seg_c1, (const double*)w.c, w.phi,
+                       w.r, w.p, w.q, c->lanes.as<Lane>(), c->n_active.as<int>()));
     c->launches++;
   } else if (!grid) {
     rc = iterate<double, V>(c, solver, imat, n_iter, w, gl);
