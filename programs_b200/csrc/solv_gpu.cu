@@ -37,6 +37,7 @@ namespace {
 
 constexpr int kMaxV = 4;
 constexpr int kGateLevels = 8;
+constexpr int kChainCells = 400000;  // bicg_iteration
 
 struct DevBuf {
   void* p = nullptr;
@@ -97,6 +98,7 @@ struct solv_gpu_ctx {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   std::string err;
   cudaError_t launch_err = cudaSuccess;  // a launch refused since launch_status
+  bool chain_ahead = true;               // chains as programmatic dependents
   int fail_launch = 0;                   // launches until one is refused on purpose
   cudaError_t fail_with = cudaSuccess;
   int n_sm = 148;
@@ -1003,7 +1005,7 @@ void chain_launch(solv_gpu_ctx* c, void (*kern)(KArgs...), int grid, int block, 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = c->chain_ahead ? 1 : 0;
   note_launch(c, launch(c, cfg, kern, args...));
 }
 
@@ -1531,6 +1533,18 @@ int bicg_iteration(solv_gpu_ctx* c, int imat, WS<T>& w) {
   double* part = c->part.as<double>();
   Lane* lanes = c->lanes.as<Lane>();
   const int G = c->seg.total_blk, B = c->block;
+  // As programmatic dependents the early exits behind the last iteration (55
+  // kernels after 5 of a graph's 16 iterations) take 0.2 us more each once the
+  // grids fill the SMs with more than one row a thread, while the iterations
+  // gain less and less.  us, dependents / plain: Jacobi, 5 iterations, 70^3
+  // 434 / 442, 80^3 511 / 500, 128^3 1192 / 1182; to 1e-10 1864 / 1940, 2232 /
+  // 2278, 8357 / 8377; DILU, multicolour, 5 iterations 695 / 683, 822 / 807,
+  // 1947 / 1930; to 1e-10 1805 / 1810, 2330 / 2329, 7445 / 7428.
+  struct ChainKeep {  // put back on every way out
+    solv_gpu_ctx* c;
+    ~ChainKeep() { c->chain_ahead = true; }
+  } chain_keep{c};
+  c->chain_ahead = c->N < kChainCells;
   // w.q holds u, w.v holds v
   if (imat > 0) {
     chain_launch(c, sg::k_bi_p<T, V, false>, G, B, sm, w.c, w.r, w.p, w.q, w.z, lanes);
