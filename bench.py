@@ -402,7 +402,7 @@ def time_configs(s, torch, dev):
         B = np.stack([b, uniform(11, A.n_cell), uniform(12, A.n_cell)], axis=1)
         out[f"momentum_96_uvw_bicgstab_dilu_fp32_inner_{order}"] = timed_solve(
             "bicg", 2, 3, B, precision=1)
-    # C1 again with the cluster-persistent fused PCG (the whole loop in one launch)
+    # C1 again under PERSISTENT 1 (the whole loop in one launch: here the resident PCG)
     from programs_b200.solver import OPT_PERSISTENT
     m = Mesh.hex(32, jitter=0.15, seed=0, permute=True)
     A = m.pressure(pin=1)
